@@ -554,17 +554,16 @@ int create_query_state(og_engine *e) {
   e->list_d[1] = e->list_d[0] + e->list_cap[0];
   e->pref_d[1] = e->pref_d[0] + e->list_cap[0] + 1;
   e->tile_d[1] = e->tile_d[0] + e->tile_cap[0];
-  e->lb_tiles = (uint32_t)((e->nwords + kWordsPerCompactTile - 1) / kWordsPerCompactTile + 1);
-  for (int r = 0; r < 2; r++) {
-    RC(dalloc(e, &e->lb[r].status, e->lb_tiles + 1));
-    e->lb[r].ticket = e->lb[r].status + e->lb_tiles;
-    RC(dalloc(e, &e->lb[r].agg_n, e->lb_tiles));
-    RC(dalloc(e, &e->lb[r].agg_e, e->lb_tiles));
-    RC(dalloc(e, &e->lb[r].inc_n, e->lb_tiles));
-    RC(dalloc(e, &e->lb[r].inc_e, e->lb_tiles));
+  // The planner counts 64 B of look-back scratch per 1024 bitmap words and
+  // region pair, i.e. two 16-byte slots per region, and 64 KiB for the small
+  // arrays, of which 2 x 256 slots (8 KiB) are used here.
+  e->lb_tiles = 2 * (uint32_t)((e->nwords + kWordsPerCompactTile - 1) / kWordsPerCompactTile) + 256;
+  for (int r = 0; r < 2; r++) {  // one slot more than tiles: the ticket counter
+    RC(dalloc(e, &e->lb[r].slot, e->lb_tiles + 1));
+    e->lb[r].ticket = (uint32_t *)(e->lb[r].slot + e->lb_tiles);
+    // epochs start at 1: zeroed slots are "empty"
+    CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * (e->lb_tiles + 1), e->s_main));
   }
-  for (int r = 0; r < 2; r++)  // epochs start at 1: zeroed status words are "empty"
-    CK(cudaMemsetAsync(e->lb[r].status, 0, sizeof(uint32_t) * (e->lb_tiles + 1), e->s_main));
   RC(dalloc(e, &e->counts_d, 3));  // Counts[2] + u64 far key[2]
   CK(cudaMemsetAsync(e->counts_d, 0, 3 * sizeof(Counts), e->s_main));
   RC(dalloc(e, &e->err_d, 4));
@@ -819,6 +818,17 @@ struct SplitArgs {
   uint32_t *clear_bits = nullptr;
 };
 
+// Words per compaction tile: the smallest of 128, 256, 512 and 1024 that
+// keeps the range within max_tiles tiles.  Small tiles spread a small graph
+// over the SMs (2^20 vertices are 32 tiles of 1024 words but 256 of 128);
+// beyond what is resident at once (four CTAs per SM) more tiles only add
+// latency.
+uint32_t compact_tile_words(uint32_t words, uint32_t max_tiles) {
+  uint32_t tw = 128;
+  while (tw < kWordsPerCompactTile && (words + tw - 1) / tw > max_tiles) tw *= 2;
+  return tw;
+}
+
 int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint32_t ve,
                    cudaStream_t s, const SplitArgs &sp = SplitArgs()) {
   if (ve <= vb) {  // empty region: no kernel writes its counts
@@ -831,7 +841,8 @@ int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint3
   a.v_end = ve;
   a.w_begin = vb / 32;
   a.w_end = (uint32_t)(((uint64_t)ve + 31) / 32);
-  a.ntiles = (a.w_end - a.w_begin + kWordsPerCompactTile - 1) / kWordsPerCompactTile;
+  a.tile_words = compact_tile_words(a.w_end - a.w_begin, std::min(e->lb_tiles - 1, 4u * (uint32_t)e->sms));
+  a.ntiles = (a.w_end - a.w_begin + a.tile_words - 1) / a.tile_words;
   a.off = e->off_d;
   a.list = e->list_d[r];
   a.pref = e->pref_d[r];
@@ -1098,7 +1109,7 @@ int compact_round(og_engine *e, const uint32_t *cur, og_stats &st, Timing &tm, u
                   const SplitArgs &sp = SplitArgs()) {
   if (++e->epoch >= (1u << 30)) {  // epoch wrap: clear the status words and far keys once
     for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].status, 0, sizeof(uint32_t) * e->lb_tiles, e->s_main));
+      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, e->s_main));
     CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), e->s_main));
     e->epoch = 1;
   }
@@ -1332,7 +1343,7 @@ int run_bfs_dev(og_engine *e, uint32_t src, og_stats &st) {
   }
   if (e->dev_epoch > (1u << 30) - (1u << 20)) {  // epoch wrap: clear the status words once
     for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].status, 0, sizeof(uint32_t) * e->lb_tiles, s));
+      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, s));
     e->dev_epoch = 1u << 29;
   }
   CK(cudaMemsetAsync(e->err_d, 0, 16, s));
@@ -1466,7 +1477,7 @@ int run_min_dev(og_engine *e, int algo, uint32_t src, og_stats &st) {
   }
   if (e->dev_epoch > (1u << 30) - (1u << 20)) {  // epoch wrap: clear the status words once
     for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].status, 0, sizeof(uint32_t) * e->lb_tiles, s));
+      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, s));
     CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), s));
     e->dev_epoch = 1u << 29;
   }
@@ -2026,7 +2037,8 @@ int launch_compact_sb(og_engine *e, int r, uint32_t *bits, uint32_t vb, uint32_t
   a.v_end = ve;
   a.w_begin = vb / 32;
   a.w_end = (uint32_t)(((uint64_t)ve + 31) / 32);
-  a.ntiles = (a.w_end - a.w_begin + kWordsPerCompactTile - 1) / kWordsPerCompactTile;
+  a.tile_words = compact_tile_words(a.w_end - a.w_begin, std::min(e->lb_tiles - 1, 4u * (uint32_t)e->sms));
+  a.ntiles = (a.w_end - a.w_begin + a.tile_words - 1) / a.tile_words;
   a.off = e->off_d;
   a.list = e->list_d[r];
   a.pref = e->pref_d[r];
@@ -2119,7 +2131,7 @@ int sb_round(og_engine *e, og_stats &st, Timing &tm, uint32_t *pending, bool *do
   *done = false;
   if (++e->epoch >= (1u << 30)) {  // epoch wrap: clear the status words and far keys once
     for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].status, 0, sizeof(uint32_t) * e->lb_tiles, e->s_main));
+      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, e->s_main));
     CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), e->s_main));
     e->epoch = 1;
   }
@@ -3149,7 +3161,7 @@ uint32_t compact_tiles(uint32_t v_begin, uint32_t v_end) {
 // (already cleared) and error word.
 void compact_launch(const uint32_t *bits, uint32_t v_begin, uint32_t v_end, const uint64_t *off,
                     uint32_t *list, uint64_t *pref, uint64_t list_cap, uint32_t *tile,
-                    uint64_t tile_cap, Counts *counts, const Lookback &lb, uint32_t *err,
+                    uint64_t tile_cap, Counts *counts, const Lookback &lb, uint32_t max_tiles, uint32_t *err,
                     cudaStream_t s) {
   CompactArgs a{};
   a.bits = bits;
@@ -3157,7 +3169,8 @@ void compact_launch(const uint32_t *bits, uint32_t v_begin, uint32_t v_end, cons
   a.v_end = v_end;
   a.w_begin = v_begin / 32;
   a.w_end = (uint32_t)(((uint64_t)v_end + 31) / 32);
-  a.ntiles = compact_tiles(v_begin, v_end);
+  a.tile_words = compact_tile_words(a.w_end - a.w_begin, max_tiles);
+  a.ntiles = (a.w_end - a.w_begin + a.tile_words - 1) / a.tile_words;
   a.off = off;
   a.list = list;
   a.pref = pref;
@@ -3177,25 +3190,17 @@ void compact_launch(const uint32_t *bits, uint32_t v_begin, uint32_t v_end, cons
   k_compact<<<a.ntiles, kThreads, 0, s>>>(a);
 }
 
-// Look-back scratch of `ntiles` tiles carved out of one allocation:
-// status[ntiles] + ticket, agg_n, inc_n (u32) and agg_e, inc_e (u64).
-uint64_t lookback_bytes(uint32_t ntiles) {
-  const uint64_t n = ntiles;
-  return 4 * (n + 1) + 8 * n + 8 * n + 4 * n + 4 * n + 64;
-}
+// Look-back scratch of `ntiles` tiles: a slot each, then the ticket.
+uint64_t lookback_bytes(uint32_t ntiles) { return sizeof(ulonglong2) * (ntiles + 1ull); }
 
 Lookback lookback_carve(void *base, uint32_t ntiles) {
-  const uint64_t n = ntiles;
-  char *p = (char *)base;
-  Lookback lb;
-  lb.agg_e = (unsigned long long *)p;
-  lb.inc_e = (unsigned long long *)(p + 8 * n);
-  lb.agg_n = (uint32_t *)(p + 16 * n);
-  lb.inc_n = (uint32_t *)(p + 20 * n);
-  lb.status = (uint32_t *)(p + 24 * n);
-  lb.ticket = lb.status + n;
-  return lb;
+  ulonglong2 *p = (ulonglong2 *)base;
+  return Lookback{p, (uint32_t *)(p + ntiles)};
 }
+
+// Tiles a stand-alone compaction may use: those of 1024 words, and up to a few
+// per SM of smaller ones.
+uint32_t compact_max_tiles(uint32_t ntiles1024) { return std::max(ntiles1024, 1024u); }
 
 int compact_args_ok(const uint32_t *bits, uint32_t v_begin, uint32_t v_end, const uint64_t *off,
                     uint32_t *out_list, uint64_t *out_pref, uint64_t list_cap, uint32_t *out_tile,
@@ -3232,7 +3237,7 @@ extern "C" int og_k_compact(const uint32_t *bits, uint32_t v_begin, uint32_t v_e
     CK(cudaStreamSynchronize(s));
     return OG_OK;
   }
-  const uint32_t nt = compact_tiles(v_begin, v_end);
+  const uint32_t nt = compact_max_tiles(compact_tiles(v_begin, v_end));
   void *scratch = nullptr;
   CK(cudaMalloc(&scratch, lookback_bytes(nt) + 256));
   char *err_d = (char *)scratch + lookback_bytes(nt);
@@ -3241,7 +3246,7 @@ extern "C" int og_k_compact(const uint32_t *bits, uint32_t v_begin, uint32_t v_e
   cudaError_t ce = cudaMemsetAsync(scratch, 0, lookback_bytes(nt) + 256, s);
   if (ce == cudaSuccess) {
     compact_launch(bits, v_begin, v_end, off, out_list, out_pref, list_cap, out_tile, tile_cap,
-                   (Counts *)out_counts, lb, (uint32_t *)err_d, s);
+                   (Counts *)out_counts, lb, nt, (uint32_t *)err_d, s);
     ce = cudaGetLastError();
   }
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(&err, err_d, 4, cudaMemcpyDeviceToHost, s);
@@ -3316,10 +3321,11 @@ extern "C" int og_k_compact_noalloc(const uint32_t *bits, uint32_t v_begin, uint
   }
   // the previous call's look-back state and error word must not leak in
   uint32_t *err_d = (uint32_t *)((char *)base + kNoAllocErrOffset);
-  CK(cudaMemsetAsync(base, 0, lookback_bytes(nt), s));
+  const uint32_t mt = compact_max_tiles(nt);
+  CK(cudaMemsetAsync(base, 0, lookback_bytes(mt), s));
   CK(cudaMemsetAsync(err_d, 0, sizeof(uint32_t), s));
   compact_launch(bits, v_begin, v_end, off, out_list, out_pref, list_cap, out_tile, tile_cap,
-                 (Counts *)out_counts, lookback_carve(base, nt), err_d, s);
+                 (Counts *)out_counts, lookback_carve(base, mt), mt, err_d, s);
   CK(cudaGetLastError());
   uint32_t err = 0;
   CK(cudaMemcpyAsync(&err, err_d, sizeof err, cudaMemcpyDeviceToHost, s));

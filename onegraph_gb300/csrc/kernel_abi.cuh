@@ -71,16 +71,12 @@ LbsArgs lbs_for(const uint32_t *list, const uint64_t *pref, const uint32_t *tile
 
 __global__ void k_wait_check(int which, uint32_t spin_limit, uint32_t *scratch, uint32_t *err) {
   if (which == 0) {
-    // tile 1 of a compaction whose tile 0 never publishes (its status word
+    // tile 1 of a compaction whose tile 0 never publishes (its slot
     // stays 0, never this launch's epoch 1)
     if (threadIdx.x >= 32) return;
     Lookback lb;
-    lb.status = scratch;
-    lb.ticket = scratch + 2;
-    lb.agg_n = scratch + 4;
-    lb.inc_n = scratch + 8;
-    lb.agg_e = (unsigned long long *)(scratch + 16);
-    lb.inc_e = (unsigned long long *)(scratch + 24);
+    lb.slot = (ulonglong2 *)scratch;
+    lb.ticket = scratch + 8;
     uint32_t pn;
     uint64_t pe;
     int bad;

@@ -28,8 +28,9 @@ namespace og {
 constexpr int kThreads = 256;
 constexpr uint32_t kTile = 2048;             // LBS edge positions per CTA
 constexpr uint32_t kItems = kTile / kThreads;  // 8
-constexpr uint32_t kCompactWordsPerThread = 4;
-constexpr uint32_t kWordsPerCompactTile = kThreads * kCompactWordsPerThread;  // 32768 vertices
+// largest compaction tile: 1024 bitmap words (32768 vertices); the planner and
+// the bitmaps' padding are sized by it
+constexpr uint32_t kWordsPerCompactTile = 1024;
 
 // device error bits (OR-ed into the engine's error word)
 constexpr uint32_t kErrLookback = 1u;    // look-back wait gave up
@@ -65,12 +66,12 @@ struct Counts {
   uint64_t total;    // sum of their degrees (edge positions)
 };
 
+// Look-back scratch: one 16-byte slot per compaction tile, written and read as
+// a single 128-bit access, so a slot carries its own state, count and degree
+// sum and no fence or second load is needed: x = (n << 32) | (epoch << 2) |
+// state, y = degree sum; state 1 the tile's aggregate, 2 the inclusive prefix.
 struct Lookback {
-  uint32_t *status;  // (epoch << 2) | state; state 1 aggregate, 2 inclusive prefix
-  uint32_t *agg_n;
-  unsigned long long *agg_e;
-  uint32_t *inc_n;
-  unsigned long long *inc_e;
+  ulonglong2 *slot;
   uint32_t *ticket;
 };
 
@@ -78,6 +79,7 @@ struct CompactArgs {
   const uint32_t *bits;  // frontier bitmap
   uint32_t v_begin, v_end;
   uint32_t w_begin, w_end, ntiles;
+  uint32_t tile_words;   // bitmap words per tile: 128, 256, 512 or 1024
   const uint64_t *off;   // CSR offsets (V+1) on the device
   uint32_t *list;
   uint64_t *pref;        // exclusive degree prefix, pref[n] = total
@@ -172,13 +174,30 @@ __device__ __forceinline__ void block_scan_pair(uint32_t cnt, uint64_t sum, uint
   __syncthreads();  // shared arrays are reused by the next call
 }
 
+__device__ __forceinline__ ulonglong2 ld_slot(const ulonglong2 *p) {
+  ulonglong2 r;
+  asm volatile(
+      "{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+      : "=l"(r.x), "=l"(r.y)
+      : "l"(p)
+      : "memory");
+  return r;
+}
+__device__ __forceinline__ void st_slot(ulonglong2 *p, uint32_t epoch, uint32_t state, uint32_t n, uint64_t e) {
+  const unsigned long long x = ((unsigned long long)n << 32) | (epoch << 2) | state;
+  asm volatile(
+      "{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+      "l"(x), "l"((unsigned long long)e)
+      : "memory");
+}
+
 // Warp-wide decoupled look-back of compaction tile `tile` (called by all 32
 // lanes of warp 0): publishes the tile's totals (tot_n, tot_e) and returns in
 // (pn, pe) the exclusive prefix of the tiles before it.  Each pass reads the
-// status of the 32 nearest unaccounted predecessors at once, sums their
+// slots of the 32 nearest unaccounted predecessors at once, sums their
 // aggregates up to the nearest one holding an inclusive prefix, and stops
 // there; tiles before the first count as an inclusive prefix of 0.  Waits
-// are bounded by `spin_limit` polls: a status that never appears sets
+// are bounded by `spin_limit` polls: a slot that never appears sets
 // kErrLookback in *err and bad = 1 (the caller then writes nothing), and the
 // tile still publishes an inclusive prefix so that successors never wait
 // forever.
@@ -191,30 +210,23 @@ __device__ __forceinline__ void lookback_prefix(const Lookback &lb, uint32_t til
   pe = 0;
   bad = 0;
   if (tile == 0) {
-    if (lane == 0) {
-      lb.inc_n[0] = tot_n;
-      lb.inc_e[0] = tot_e;
-      __threadfence();
-      st_release(&lb.status[0], (epoch << 2) | 2u);
-    }
+    if (lane == 0) st_slot(lb.slot, epoch, 2u, tot_n, tot_e);
     return;
   }
-  if (lane == 0) {
-    lb.agg_n[tile] = tot_n;
-    lb.agg_e[tile] = tot_e;
-    __threadfence();
-    st_release(&lb.status[tile], (epoch << 2) | 1u);
-  }
+  if (lane == 0) st_slot(lb.slot + tile, epoch, 1u, tot_n, tot_e);
   for (int p = (int)tile - 1;; p -= 32) {
     const int q = p - lane;  // lane 0: nearest predecessor of the window
-    uint32_t st = 2u;
+    uint32_t st = 2u, vn = 0;
+    uint64_t ve = 0;
     if (q >= 0) {
       uint32_t spins = 0;
       for (;;) {
-        const uint32_t raw = ld_acquire(&lb.status[q]);
-        st = (raw >> 2) == epoch ? (raw & 3u) : 0u;
+        const ulonglong2 v = ld_slot(lb.slot + q);
+        st = ((uint32_t)v.x >> 2) == epoch ? ((uint32_t)v.x & 3u) : 0u;
+        vn = (uint32_t)(v.x >> 32);
+        ve = v.y;
         if (st != 0u || ++spins > spin_limit) break;
-        __nanosleep(64);
+        __nanosleep(32);
       }
     }
     __syncwarp();
@@ -225,123 +237,291 @@ __device__ __forceinline__ void lookback_prefix(const Lookback &lb, uint32_t til
     }
     const unsigned incl = __ballot_sync(0xffffffffu, st == 2u);
     const int k = incl ? __ffs(incl) - 1 : 32;
-    uint32_t vn = 0;
-    uint64_t ve = 0;
-    if (q >= 0 && lane < k) {
-      vn = __ldcg(&lb.agg_n[q]);
-      ve = __ldcg(&lb.agg_e[q]);
-    } else if (q >= 0 && lane == k) {
-      vn = __ldcg(&lb.inc_n[q]);
-      ve = __ldcg(&lb.inc_e[q]);
+    if (q < 0 || lane > k) {
+      vn = 0;
+      ve = 0;
     }
+    vn = __reduce_add_sync(0xffffffffu, vn);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      vn += __shfl_xor_sync(0xffffffffu, vn, o);
-      ve += __shfl_xor_sync(0xffffffffu, ve, o);
-    }
+    for (int o = 16; o; o >>= 1) ve += __shfl_xor_sync(0xffffffffu, ve, o);
     pn += vn;
     pe += ve;
     if (k < 32) break;
   }
-  if (lane == 0) {
-    lb.inc_n[tile] = pn + tot_n;
-    lb.inc_e[tile] = pe + tot_e;
-    __threadfence();
-    st_release(&lb.status[tile], (epoch << 2) | 2u);  // published even when bad
+  if (lane == 0) st_slot(lb.slot + tile, epoch, 2u, pn + tot_n, pe + tot_e);  // published even when bad
+}
+
+// Block-wide exclusive scan of u32 counts; returns the block total.  Callers
+// put a barrier between two calls.
+__device__ __forceinline__ uint32_t block_scan_u32(uint32_t cnt, uint32_t &ex) {
+  __shared__ uint32_t s_w[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t ic = cnt;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t c = __shfl_up_sync(0xffffffffu, ic, d);
+    if (lane >= d) ic += c;
+  }
+  if (lane == 31) s_w[warp] = ic;
+  __syncthreads();
+  uint32_t wp = 0, tot = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; w++) {
+    const uint32_t x = s_w[w];
+    wp += w < warp ? x : 0u;
+    tot += x;
+  }
+  ex = wp + ic - cnt;
+  return tot;
+}
+
+// ------------------------------------------------------------- compaction
+//
+// Frontier compaction of a vertex range: bitmap words -> vertex list in
+// increasing id order, u64 degree prefix and LBS tile map, one pass with a
+// decoupled look-back.  A CTA's tile is tile_words bitmap words.  The set
+// bits are first listed in shared memory, kListPass at a time, and the list
+// entries (not the words) are then spread over the threads, so that a dense
+// frontier costs a thread eight independent vertices per pass instead of a
+// serial walk of 128, and a sparse one keeps one load per lane in flight.
+// Bound: the dependent chain words -> (value ->) offsets -> look-back when the
+// frontier is sparse, the 16 B of offsets and 12 B of list per vertex when it
+// is dense.  With four words walked by each thread (the earlier form) an
+// 8-source SSSP pass over 2^20 vertices spent 0.4 ms per compaction on 32 CTAs;
+// this form took the pass from 7.2 to 2.8 ms and a resident SSSP query of 0.3 M
+// vertices (108 compactions) from 2.4 to 1.95 ms.  64 registers (4 CTAs per SM):
+// left to itself the compiler takes 118, which halves the CTAs in flight and
+// costs 5 % of an SSSP query over 2^24 vertices.  Sel says which vertices are
+// listed:
+//  pre(v)                 v's state
+//  want(pre)              whether its degree matters
+//  settle(v, pre, d, far, clr)  the degree d when v is listed, else 0; far /
+//                         clr: v's bit belongs in the far / cleared words
+//  flush(w, far, clr)     those words, once per bitmap word
+//  finish(tid)            per-thread reductions (all threads, has barriers)
+//  emit(v, pos)           v is list entry pos
+constexpr uint32_t kListPass = 8 * kThreads;
+constexpr uint16_t kDropped = 0xffffu;
+
+struct CompactShared {
+  uint32_t word[kWordsPerCompactTile];   // scanned bits, later the listed ones
+  uint32_t far[kWordsPerCompactTile], clr[kWordsPerCompactTile];
+  uint32_t drop[kWordsPerCompactTile];   // scanned but not listed (several passes)
+  uint16_t wbase[kWordsPerCompactTile];  // set bits before each word
+  uint16_t list[kListPass];              // tile-local vertex of each entry of the pass
+  uint16_t rank[kListPass];              // its list rank within the pass, or kDropped
+  uint64_t pref[kListPass + kThreads + 1];  // its degree, then the exclusive prefix (padded: at())
+  uint32_t tile, excl_n;
+  uint64_t excl_e;
+  int bad;
+  // eight consecutive entries per thread, one pad per eight: no bank conflicts
+  __device__ __forceinline__ static uint32_t at(uint32_t i) { return i + (i >> 3); }
+};
+
+// Set-bit ranks of the tile's words: returns the total, own first rank in ex.
+__device__ __forceinline__ uint32_t compact_ranks(CompactShared &sh, uint32_t wpt, uint32_t w0, uint32_t nw,
+                                                  uint32_t &pc, uint32_t &ex) {
+  pc = 0;
+  for (uint32_t j = 0; j < wpt; j++)
+    if (w0 + j < nw) pc += __popc(sh.word[w0 + j]);
+  const uint32_t N = block_scan_u32(pc, ex);
+  uint32_t r = ex;
+  for (uint32_t j = 0; j < wpt; j++)
+    if (w0 + j < nw) {
+      sh.wbase[w0 + j] = (uint16_t)r;
+      r += __popc(sh.word[w0 + j]);
+    }
+  __syncthreads();
+  return N;
+}
+
+// Lists the set bits of ranks [p0, p0 + kListPass).  Dense words are listed
+// a warp per word, sparse ones by the threads that own them.
+__device__ __forceinline__ void compact_list(CompactShared &sh, uint32_t wpt, uint32_t w0, uint32_t nw, uint32_t N,
+                                             uint32_t pc, uint32_t ex, uint32_t p0) {
+  if (N > 4 * nw) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t w = threadIdx.x >> 5; w < nw; w += kThreads / 32) {
+      const uint32_t r = sh.wbase[w];
+      if (r >= p0 + kListPass || r + 32 <= p0) continue;
+      const uint32_t m = sh.word[w];
+      const uint32_t k = r + __popc(m & ((1u << lane) - 1u)) - p0;
+      if (((m >> lane) & 1u) && k < kListPass) sh.list[k] = (uint16_t)(w * 32 + lane);
+    }
+  } else if (ex < p0 + kListPass && ex + pc > p0) {
+    uint32_t k = ex - p0;
+    for (uint32_t j = 0; j < wpt; j++)
+      if (w0 + j < nw)
+        for (uint32_t m = sh.word[w0 + j]; m; m &= m - 1, k++)
+          if (k < kListPass) sh.list[k] = (uint16_t)((w0 + j) * 32 + __ffs(m) - 1);
+  }
+  __syncthreads();
+}
+
+// Degrees in sh.pref -> ranks and exclusive prefixes; returns the pass totals.
+__device__ __forceinline__ void compact_scan(CompactShared &sh, uint32_t m, uint32_t &tn, uint64_t &te) {
+  const uint32_t i0 = threadIdx.x * 8;
+  uint64_t d[8];
+  uint32_t cnt = 0;
+  uint64_t sum = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < 8; i++) {
+    d[i] = i0 + i < m ? sh.pref[CompactShared::at(i0 + i)] : 0;
+    cnt += d[i] ? 1u : 0u;
+    sum += d[i];
+  }
+  uint32_t exn;
+  uint64_t exe;
+  block_scan_pair(cnt, sum, exn, exe, tn, te);
+#pragma unroll
+  for (uint32_t i = 0; i < 8; i++)
+    if (i0 + i < m) {
+      sh.rank[i0 + i] = d[i] ? (uint16_t)exn : kDropped;
+      sh.pref[CompactShared::at(i0 + i)] = exe;
+      exn += d[i] ? 1u : 0u;
+      exe += d[i];
+      if (i0 + i + 1 == m) sh.pref[CompactShared::at(m)] = exe;
+    }
+  __syncthreads();
+}
+
+// Writes the pass's listed entries at list position base_n, degree base_e.
+template <class Args, class Sel>
+__device__ __forceinline__ void compact_emit(const Args &a, Sel &sel, const CompactShared &sh, uint64_t vbase,
+                                             uint32_t m, uint32_t base_n, uint64_t base_e) {
+  for (uint32_t x = threadIdx.x; x < (m + 31) / 32 * 32; x += kThreads) {
+    const bool on = x < m && sh.rank[x] != kDropped;
+    uint32_t pos = 0;
+    uint64_t t = 0, te = 0;  // tiles that start inside this vertex
+    if (on) {
+      const uint64_t v = vbase + sh.list[x];
+      const uint64_t ep = base_e + sh.pref[CompactShared::at(x)];
+      pos = base_n + sh.rank[x];
+      a.list[pos] = (uint32_t)v;
+      a.pref[pos] = ep;
+      t = (ep + kTile - 1) / kTile;
+      te = (base_e + sh.pref[CompactShared::at(x + 1)] + kTile - 1) / kTile;
+      if (te > a.tile_cap) {
+        atomicOr(a.err, kErrTileMap);
+        te = a.tile_cap;
+      }
+      sel.emit(v, pos);
+    }
+    // a hub's tiles are written by the whole warp
+    const uint32_t big = __ballot_sync(0xffffffffu, te > t + 8);
+    if (te <= t + 8)
+      for (; t < te; t++) a.tile_first[t] = pos;
+    for (uint32_t b = big; b; b &= b - 1) {
+      const int l = __ffs(b) - 1;
+      const uint64_t ts = __shfl_sync(0xffffffffu, t, l), tend = __shfl_sync(0xffffffffu, te, l);
+      const uint32_t p = __shfl_sync(0xffffffffu, pos, l);
+      for (uint64_t q = ts + (threadIdx.x & 31); q < tend; q += 32) a.tile_first[q] = p;
+    }
   }
 }
 
-// Frontier compaction for the vertex range [v_begin, v_end).  Four
-// consecutive bitmap words (128 vertices) per thread, 1024 words per CTA
-// tile, tiles ordered by a ticket so that every predecessor a tile waits for
-// is already running.
-__global__ void __launch_bounds__(kThreads) k_compact(CompactArgs a) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_excl_n;
-  __shared__ uint64_t s_excl_e;
-  __shared__ int s_bad;
-  if (a.run_flag && *a.run_flag == 0u) return;  // every CTA of the launch reads the same flag
-  if (a.epoch_ptr) a.epoch = *a.epoch_ptr;
-  if (a.thr_ptr) a.thr = *a.thr_ptr;
+template <class Args, class Sel>
+__device__ __forceinline__ void compact_tile(const Args &a, Sel &sel, CompactShared &sh) {
   if (threadIdx.x == 0) {
-    s_tile = atomicAdd(a.lb.ticket, 1u);
-    if (s_tile == a.ntiles - 1) *a.lb.ticket = 0u;  // every CTA of this launch has its ticket
+    sh.tile = atomicAdd(a.lb.ticket, 1u);
+    if (sh.tile == a.ntiles - 1) *a.lb.ticket = 0u;  // every CTA of this launch has its ticket
   }
   __syncthreads();
-  const uint32_t tile = s_tile;
-  const uint32_t w0 = a.w_begin + tile * kWordsPerCompactTile + threadIdx.x * kCompactWordsPerThread;
-  // drop vertices without edges: nothing to expand
-  uint32_t keep[kCompactWordsPerThread];
-  uint32_t cnt = 0, tmin = 0xffffffffu;  // smallest waiting value of this thread
-  uint64_t sum = 0;
+  const uint32_t tile = sh.tile;
+  const uint32_t wpt = a.tile_words <= kThreads ? 1u : a.tile_words / kThreads;  // words per thread
+  const uint32_t wt = a.w_begin + tile * a.tile_words;
+  const uint32_t nw = min(a.tile_words, a.w_end - wt);
+  const uint32_t w0 = threadIdx.x * wpt;
+  const uint64_t vbase = (uint64_t)wt * 32;
+  uint32_t wv[kWordsPerCompactTile / kThreads];  // all of a thread's words in flight together
 #pragma unroll
-  for (uint32_t j = 0; j < kCompactWordsPerThread; j++) {
-    const uint32_t w = w0 + j;
-    const uint64_t vbase = (uint64_t)w * 32;
-    uint32_t word = 0;
-    if (w < a.w_end) {
-      word = a.bits[w];
-      if (vbase < a.v_begin) {
-        const uint32_t sh = a.v_begin - (uint32_t)vbase;
-        word = sh >= 32 ? 0 : word & (0xffffffffu << sh);
-      }
-      if (vbase + 32 > a.v_end) {
-        const uint64_t k = a.v_end > vbase ? a.v_end - vbase : 0;
-        word = k >= 32 ? word : word & ((1u << k) - 1u);
-      }
-    }
-    uint32_t kp = 0, far = 0, leave = 0;
-    for (uint32_t m = word; m; m &= m - 1) {
-      const uint32_t b = __ffs(m) - 1;
-      const uint64_t v = vbase + b;
-      if (a.split) {
-        const uint32_t x = __ldcg(a.value + v);
-        if (x >= a.thr) {
-          far |= 1u << b;
-          tmin = min(tmin, x);
-          continue;
-        }
-        leave |= 1u << b;
-      }
-      const uint64_t d = a.off[v + 1] - a.off[v];
-      if (!d) continue;
-      kp |= 1u << b;
-      cnt++;
-      sum += d;
-    }
-    keep[j] = kp;
-    if (far && a.far_bits) atomicOr(a.far_bits + w, far);
-    if (leave && a.clear_bits) atomicAnd(a.clear_bits + w, ~leave);
+  for (uint32_t j = 0; j < kWordsPerCompactTile / kThreads; j++) {
+    const uint32_t l = j * kThreads + threadIdx.x;
+    wv[j] = l < nw ? a.bits[wt + l] : 0u;
   }
-  uint32_t ex_n, tot_n;
-  uint64_t ex_e, tot_e;
-  // smallest waiting value of the CTA: one far-key atomic per CTA
-  __shared__ uint32_t s_wmin[kThreads / 32];
-  if (a.far_key) {
-    const uint32_t wm = __reduce_min_sync(0xffffffffu, tmin);
-    if ((threadIdx.x & 31) == 0) s_wmin[threadIdx.x >> 5] = wm;
-  }
-  block_scan_pair(cnt, sum, ex_n, ex_e, tot_n, tot_e);  // its barriers publish s_wmin
-  if (a.far_key && threadIdx.x == 0) {
-    uint32_t m = 0xffffffffu;
+  uint32_t any = 0;
 #pragma unroll
-    for (int i = 0; i < kThreads / 32; i++) m = min(m, s_wmin[i]);
-    if (m != 0xffffffffu) atomicMax(a.far_key, ((unsigned long long)a.epoch << 32) | (~m & 0xffffffffu));
+  for (uint32_t j = 0; j < kWordsPerCompactTile / kThreads; j++) {
+    const uint32_t l = j * kThreads + threadIdx.x;
+    if (l >= nw) break;
+    uint32_t word = wv[j];
+    const uint64_t vb = vbase + 32ull * l;
+    if (vb < a.v_begin) {
+      const uint32_t s = a.v_begin - (uint32_t)vb;
+      word = s >= 32 ? 0 : word & (0xffffffffu << s);
+    }
+    if (vb + 32 > a.v_end) {
+      const uint64_t k = a.v_end > vb ? a.v_end - vb : 0;
+      word = k >= 32 ? word : word & ((1u << k) - 1u);
+    }
+    sh.word[l] = word;
+    sh.far[l] = 0;
+    sh.clr[l] = 0;
+    sh.drop[l] = 0;
+    any |= word;
+  }
+  uint32_t pc, ex, N = 0;
+  if (__syncthreads_or(any)) N = compact_ranks(sh, wpt, w0, nw, pc, ex);  // most tiles of a sparse frontier are empty
+  uint32_t tot_n = 0;
+  uint64_t tot_e = 0;
+  for (uint32_t p0 = 0; p0 < N; p0 += kListPass) {
+    const uint32_t m = min(kListPass, N - p0);
+    compact_list(sh, wpt, w0, nw, N, pc, ex, p0);
+    // three phases, so that a thread's eight state loads and then its eight
+    // offset pairs are in flight together
+    uint32_t lv[8];
+    typename Sel::Pre pre[8];
+    uint64_t d[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j++) {
+      const uint32_t x = j * kThreads + threadIdx.x;
+      lv[j] = x < m ? sh.list[x] : 0xffffffffu;
+      if (x < m) pre[j] = sel.pre(vbase + lv[j]);
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j++) {
+      d[j] = 0;
+      if (lv[j] != 0xffffffffu && sel.want(pre[j])) d[j] = a.off[vbase + lv[j] + 1] - a.off[vbase + lv[j]];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j++) {
+      if (lv[j] == 0xffffffffu) break;
+      bool far = false, clr = false;
+      const uint32_t l = lv[j];
+      sh.pref[CompactShared::at(j * kThreads + threadIdx.x)] = sel.settle(vbase + l, pre[j], d[j], far, clr);
+      if (far) atomicOr(&sh.far[l >> 5], 1u << (l & 31));
+      if (clr) atomicOr(&sh.clr[l >> 5], 1u << (l & 31));
+    }
+    __syncthreads();
+    uint32_t tn;
+    uint64_t te;
+    compact_scan(sh, m, tn, te);
+    tot_n += tn;
+    tot_e += te;
+    if (N > kListPass) {  // several passes: the listed bits are listed again below
+      for (uint32_t x = threadIdx.x; x < m; x += kThreads)
+        if (sh.rank[x] == kDropped) atomicOr(&sh.drop[sh.list[x] >> 5], 1u << (sh.list[x] & 31));
+      __syncthreads();
+    }
+  }
+  if (N) {
+    for (uint32_t l = threadIdx.x; l < nw; l += kThreads)
+      if (sh.far[l] | sh.clr[l]) sel.flush(wt + l, sh.far[l], sh.clr[l]);
+    sel.finish();
   }
   if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
     uint32_t pn = 0;
     uint64_t pe = 0;
     int bad = 0;
     lookback_prefix(a.lb, tile, a.epoch, tot_n, tot_e, a.err, pn, pe, bad);
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       if (!bad && (uint64_t)pn + tot_n > a.list_cap) {
         atomicOr(a.err, kErrTileMap);
         bad = 1;
       }
-      s_excl_n = pn;
-      s_excl_e = pe;
-      s_bad = bad;
+      sh.excl_n = pn;
+      sh.excl_e = pe;
+      sh.bad = bad;
       if (!bad && tile == a.ntiles - 1) {
         a.counts->n = pn + tot_n;
         a.counts->total = pe + tot_e;
@@ -350,29 +530,82 @@ __global__ void __launch_bounds__(kThreads) k_compact(CompactArgs a) {
     }
   }
   __syncthreads();
-  if (s_bad) return;  // positions unknown: write nothing
-  uint32_t pos = s_excl_n + ex_n;
-  uint64_t ep = s_excl_e + ex_e;
-#pragma unroll
-  for (uint32_t j = 0; j < kCompactWordsPerThread; j++) {
-    const uint64_t vbase = (uint64_t)(w0 + j) * 32;
-    for (uint32_t m = keep[j]; m; m &= m - 1) {
-      const uint32_t b = __ffs(m) - 1;
-      const uint64_t v = vbase + b;
-      const uint64_t d = a.off[v + 1] - a.off[v];
-      a.list[pos] = (uint32_t)v;
-      a.pref[pos] = ep;
-      for (uint64_t t = (ep + kTile - 1) / kTile; t * kTile < ep + d; t++) {
-        if (t >= a.tile_cap) {
-          atomicOr(a.err, kErrTileMap);
-          break;
-        }
-        a.tile_first[t] = pos;
-      }
-      pos++;
-      ep += d;
-    }
+  if (sh.bad || tot_n == 0) return;  // bad: positions unknown, write nothing
+  uint32_t base_n = sh.excl_n;
+  uint64_t base_e = sh.excl_e;
+  if (N <= kListPass) {
+    compact_emit(a, sel, sh, vbase, N, base_n, base_e);
+    return;
   }
+  for (uint32_t l = threadIdx.x; l < nw; l += kThreads) sh.word[l] &= ~sh.drop[l];
+  __syncthreads();
+  compact_ranks(sh, wpt, w0, nw, pc, ex);
+  for (uint32_t p0 = 0; p0 < tot_n; p0 += kListPass) {
+    const uint32_t m = min(kListPass, tot_n - p0);
+    compact_list(sh, wpt, w0, nw, tot_n, pc, ex, p0);
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < m; x += kThreads) {
+      const uint64_t v = vbase + sh.list[x];
+      sh.pref[CompactShared::at(x)] = a.off[v + 1] - a.off[v];
+    }
+    __syncthreads();
+    uint32_t tn;
+    uint64_t te;
+    compact_scan(sh, m, tn, te);
+    compact_emit(a, sel, sh, vbase, m, base_n, base_e);
+    base_n += tn;
+    base_e += te;
+    __syncthreads();  // the next pass rewrites the shared list
+  }
+}
+
+// Smallest of a per-thread value over the CTA (the result is thread 0's).
+__device__ __forceinline__ uint32_t block_min_u32(uint32_t x) {
+  __shared__ uint32_t s_m[kThreads / 32];
+  const uint32_t w = __reduce_min_sync(0xffffffffu, x);
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = w;
+  __syncthreads();
+  uint32_t m = 0xffffffffu;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; i++) m = min(m, s_m[i]);
+  return m;
+}
+
+struct CompactSel {
+  const CompactArgs &a;
+  uint32_t tmin;  // smallest waiting value of this thread
+  using Pre = uint32_t;
+  __device__ __forceinline__ Pre pre(uint64_t v) const { return a.split ? __ldcg(a.value + v) : 0u; }
+  __device__ __forceinline__ bool want(Pre x) const { return !a.split || x < a.thr; }
+  __device__ __forceinline__ uint64_t settle(uint64_t, Pre x, uint64_t d, bool &far, bool &clr) {
+    if (a.split) {
+      far = x >= a.thr;
+      clr = !far;
+      if (far) tmin = min(tmin, x);
+    }
+    return d;
+  }
+  __device__ __forceinline__ void flush(uint32_t w, uint32_t far, uint32_t clr) const {
+    if (far && a.far_bits) atomicOr(a.far_bits + w, far);
+    if (clr && a.clear_bits) atomicAnd(a.clear_bits + w, ~clr);
+  }
+  __device__ __forceinline__ void finish() const {  // one far-key atomic per CTA
+    if (!a.split) return;
+    const uint32_t m = block_min_u32(tmin);
+    if (m != 0xffffffffu && a.far_key)
+      atomicMax(a.far_key, ((unsigned long long)a.epoch << 32) | (~m & 0xffffffffu));
+  }
+  __device__ __forceinline__ void emit(uint64_t, uint32_t) const {}
+};
+
+__global__ void __launch_bounds__(kThreads, 4) k_compact(CompactArgs a) {
+  __shared__ CompactShared sh;
+  if (a.run_flag && *a.run_flag == 0u) return;  // every CTA of the launch reads the same flag
+  if (a.epoch_ptr) a.epoch = *a.epoch_ptr;
+  if (a.thr_ptr) a.thr = *a.thr_ptr;
+  CompactSel sel{a, 0xffffffffu};
+  compact_tile(a, sel, sh);
 }
 
 // ------------------------------------------------------------------ LBS
@@ -635,29 +868,6 @@ template <class T, class = void>
 struct HasProbeVal : std::false_type {};
 template <class T>
 struct HasProbeVal<T, std::void_t<decltype(T::kProbeVal)>> : std::true_type {};
-
-// Block-wide exclusive scan of u32 counts; returns the block total.
-__device__ __forceinline__ uint32_t block_scan_u32(uint32_t cnt, uint32_t &ex) {
-  __shared__ uint32_t s_w[kThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t ic = cnt;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t c = __shfl_up_sync(0xffffffffu, ic, d);
-    if (lane >= d) ic += c;
-  }
-  if (lane == 31) s_w[warp] = ic;
-  __syncthreads();
-  uint32_t wp = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < kThreads / 32; w++) {
-    const uint32_t x = s_w[w];
-    wp += w < warp ? x : 0u;
-    tot += x;
-  }
-  ex = wp + ic - cnt;
-  return tot;
-}
 
 // Builds the local-vertex tables of tile k; returns the local count (0 on
 // error).  Sh is LbsShared<Val, *> or PrShared.  cb[j] is the source cursor

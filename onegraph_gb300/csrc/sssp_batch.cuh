@@ -44,6 +44,7 @@ struct SbCompactArgs {
   uint32_t *wait;        // the waiting set
   uint32_t v_begin, v_end;
   uint32_t w_begin, w_end, ntiles;
+  uint32_t tile_words;
   const uint64_t *off;   // CSR offsets (V+1) on the device
   uint32_t *list;        // listed vertices
   uint64_t *pref;        // exclusive degree prefix, pref[n] = total
@@ -68,9 +69,12 @@ struct SbCompactArgs {
 };
 
 // Near slots of one row: the slots of m whose distance is below thr; the
-// smallest distance among the others goes to fmin.
+// smallest distance among the others goes to fmin.  A pending distance is
+// below 0xFFFFFFFF, so the threshold that never advances (width 0) reads no
+// row at all.
 __device__ __forceinline__ uint32_t sb_split(const uint32_t *row, uint32_t m, uint32_t thr,
                                              uint32_t &fmin) {
+  if (thr == 0xffffffffu) return m;
   uint32_t near = 0;
   for (uint32_t t = m; t; t &= t - 1) {
     const uint32_t s = __ffs(t) - 1;
@@ -81,152 +85,62 @@ __device__ __forceinline__ uint32_t sb_split(const uint32_t *row, uint32_t m, ui
   return near;
 }
 
-// Compaction of one round for the vertex range [v_begin, v_end): the same
-// tiles, ticket order and decoupled look-back as k_compact.  Every vertex of
+// Compaction of one round for the vertex range [v_begin, v_end): the tiles,
+// ticket order and decoupled look-back of k_compact.  Every vertex of
 // the scanned bitmap is classified: its near slots are consumed from pend
 // (listed with their mask when the vertex has edges), its far slots stay
 // pending and the vertex joins the waiting set; a scanned vertex leaves the
 // active set, and leaves the waiting set once nothing of it waits.
-__global__ void __launch_bounds__(kThreads) k_compact_sb(SbCompactArgs a) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_excl_n;
-  __shared__ uint64_t s_excl_e;
-  __shared__ int s_bad;
-  __shared__ uint32_t s_wmin[kThreads / 32], s_seen[kThreads / 32], s_far[kThreads / 32];
-  if (threadIdx.x == 0) {
-    s_tile = atomicAdd(a.lb.ticket, 1u);
-    if (s_tile == a.ntiles - 1) *a.lb.ticket = 0u;
+struct SbSel {
+  const SbCompactArgs &a;
+  uint32_t tmin, seen, farm;  // this thread's smallest waiting distance, pending and waiting slots
+  using Pre = uint32_t;
+  __device__ __forceinline__ Pre pre(uint64_t v) const { return __ldcg(a.pend + v); }
+  __device__ __forceinline__ bool want(Pre) const { return true; }
+  __device__ __forceinline__ uint64_t settle(uint64_t v, Pre pm, uint64_t d, bool &far, bool &clr) {
+    const uint32_t near = sb_split(a.dist + v * a.ks, pm, a.thr, tmin);
+    const uint32_t fm = pm & ~near;
+    seen |= pm;
+    farm |= fm;
+    far = fm && !a.scan_wait;          // joins the waiting set
+    clr = !a.scan_wait || fm == 0;     // classified, or nothing of it waits any more
+    if (near && !d) a.pend[v] = fm;    // no edges: its near slots are final here
+    return near ? d : 0;
   }
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  const uint32_t w0 = a.w_begin + tile * kWordsPerCompactTile + threadIdx.x * kCompactWordsPerThread;
-  uint32_t keep[kCompactWordsPerThread];
-  uint32_t cnt = 0, tmin = 0xffffffffu, seen = 0, farm = 0;
-  uint64_t sum = 0;
-#pragma unroll
-  for (uint32_t j = 0; j < kCompactWordsPerThread; j++) {
-    const uint32_t w = w0 + j;
-    const uint64_t vbase = (uint64_t)w * 32;
-    uint32_t word = 0;
-    if (w < a.w_end) {
-      word = a.bits[w];
-      if (vbase < a.v_begin) {
-        const uint32_t sh = a.v_begin - (uint32_t)vbase;
-        word = sh >= 32 ? 0 : word & (0xffffffffu << sh);
-      }
-      if (vbase + 32 > a.v_end) {
-        const uint64_t k = a.v_end > vbase ? a.v_end - vbase : 0;
-        word = k >= 32 ? word : word & ((1u << k) - 1u);
-      }
-    }
-    uint32_t kp = 0, to_wait = 0, clr = 0;
-    for (uint32_t m = word; m; m &= m - 1) {
-      const uint32_t b = __ffs(m) - 1;
-      const uint64_t v = vbase + b;
-      const uint32_t pm = __ldcg(a.pend + v);
-      uint32_t fmin = 0xffffffffu;
-      const uint32_t near = sb_split(a.dist + v * a.ks, pm, a.thr, fmin);
-      const uint32_t far = pm & ~near;
-      seen |= pm;
-      if (far) {
-        farm |= far;
-        tmin = min(tmin, fmin);
-        if (!a.scan_wait) to_wait |= 1u << b;
-      } else if (a.scan_wait) {
-        clr |= 1u << b;  // nothing of it waits any more
-      }
-      if (!a.scan_wait) clr |= 1u << b;  // classified: leaves the active set
-      if (near) {
-        const uint64_t d = a.off[v + 1] - a.off[v];
-        if (d) {
-          kp |= 1u << b;
-          cnt++;
-          sum += d;
-        } else {
-          a.pend[v] = far;  // no edges: its near slots are final here
-        }
-      }
-    }
-    keep[j] = kp;
-    if (to_wait) atomicOr(a.wait + w, to_wait);
+  __device__ __forceinline__ void flush(uint32_t w, uint32_t far, uint32_t clr) const {
+    if (far) atomicOr(a.wait + w, far);
     if (clr) atomicAnd(a.bits + w, ~clr);
   }
-  {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t wm = __reduce_min_sync(0xffffffffu, tmin);
-    const uint32_t ws = __reduce_or_sync(0xffffffffu, seen);
-    const uint32_t wf = __reduce_or_sync(0xffffffffu, farm);
-    if (lane == 0) {
-      s_wmin[warp] = wm;
-      s_seen[warp] = ws;
-      s_far[warp] = wf;
+  __device__ __forceinline__ void finish() const {
+    __shared__ uint32_t s_seen, s_far;
+    if (threadIdx.x == 0) s_seen = s_far = 0;
+    __syncthreads();
+    const uint32_t ws = __reduce_or_sync(0xffffffffu, seen), wf = __reduce_or_sync(0xffffffffu, farm);
+    if ((threadIdx.x & 31) == 0) {
+      if (ws) atomicOr(&s_seen, ws);
+      if (wf) atomicOr(&s_far, wf);
     }
-  }
-  uint32_t ex_n, tot_n;
-  uint64_t ex_e, tot_e;
-  block_scan_pair(cnt, sum, ex_n, ex_e, tot_n, tot_e);  // its barriers publish the warp results
-  if (threadIdx.x == 0) {
-    uint32_t m = 0xffffffffu, o = 0, f = 0;
-#pragma unroll
-    for (int i = 0; i < kThreads / 32; i++) {
-      m = min(m, s_wmin[i]);
-      o |= s_seen[i];
-      f |= s_far[i];
-    }
-    if (m != 0xffffffffu) atomicMax(a.far_key, ((unsigned long long)a.epoch << 32) | (~m & 0xffffffffu));
-    if (o) atomicOr(a.masks, o);
-    if (f) atomicOr(a.masks + 1, f);
-  }
-  if (threadIdx.x < 32) {
-    uint32_t pn;
-    uint64_t pe;
-    int bad;
-    lookback_prefix(a.lb, tile, a.epoch, tot_n, tot_e, a.err, pn, pe, bad);
+    const uint32_t m = block_min_u32(tmin);  // its barrier publishes the masks
     if (threadIdx.x == 0) {
-      if (!bad && (uint64_t)pn + tot_n > a.list_cap) {
-        atomicOr(a.err, kErrTileMap);
-        bad = 1;
-      }
-      s_excl_n = pn;
-      s_excl_e = pe;
-      s_bad = bad;
-      if (!bad && tile == a.ntiles - 1) {
-        a.counts->n = pn + tot_n;
-        a.counts->total = pe + tot_e;
-        a.pref[pn + tot_n] = pe + tot_e;
-      }
+      if (m != 0xffffffffu) atomicMax(a.far_key, ((unsigned long long)a.epoch << 32) | (~m & 0xffffffffu));
+      if (s_seen) atomicOr(a.masks, s_seen);
+      if (s_far) atomicOr(a.masks + 1, s_far);
     }
   }
-  __syncthreads();
-  if (s_bad) return;  // positions unknown: write nothing (near slots stay pending)
-  uint32_t pos = s_excl_n + ex_n;
-  uint64_t ep = s_excl_e + ex_e;
-#pragma unroll
-  for (uint32_t j = 0; j < kCompactWordsPerThread; j++) {
-    const uint64_t vbase = (uint64_t)(w0 + j) * 32;
-    for (uint32_t m = keep[j]; m; m &= m - 1) {
-      const uint32_t b = __ffs(m) - 1;
-      const uint64_t v = vbase + b;
-      const uint64_t d = a.off[v + 1] - a.off[v];
-      // the same classification as above (nothing changed pend or dist since)
-      const uint32_t pm = __ldcg(a.pend + v);
-      uint32_t fmin = 0xffffffffu;
-      const uint32_t near = sb_split(a.dist + v * a.ks, pm, a.thr, fmin);
-      a.lmask[pos] = near;
-      a.pend[v] = pm & ~near;
-      a.list[pos] = (uint32_t)v;
-      a.pref[pos] = ep;
-      for (uint64_t t = (ep + kTile - 1) / kTile; t * kTile < ep + d; t++) {
-        if (t >= a.tile_cap) {
-          atomicOr(a.err, kErrTileMap);
-          break;
-        }
-        a.tile_first[t] = pos;
-      }
-      pos++;
-      ep += d;
-    }
+  // the same classification as above (nothing changed pend or dist since)
+  __device__ __forceinline__ void emit(uint64_t v, uint32_t pos) const {
+    const uint32_t pm = __ldcg(a.pend + v);
+    uint32_t fmin = 0xffffffffu;
+    const uint32_t near = sb_split(a.dist + v * a.ks, pm, a.thr, fmin);
+    a.lmask[pos] = near;
+    a.pend[v] = pm & ~near;
   }
+};
+
+__global__ void __launch_bounds__(kThreads, 4) k_compact_sb(SbCompactArgs a) {
+  __shared__ CompactShared sh;
+  SbSel sel{a, 0xffffffffu, 0u, 0u};
+  compact_tile(a, sel, sh);
 }
 
 // Relax of the listed vertices' near slots: for an edge (u, v, w) and every
