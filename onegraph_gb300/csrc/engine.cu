@@ -607,7 +607,7 @@ int create_query_state(og_engine *e) {
     RC(dalloc(e, &e->arena, per * (V + 1)));
     if (e->pr_enabled) {
       e->contrib_d = (float *)e->arena;
-      e->sum_d = e->contrib_d + (V + 1);
+      e->sum_d = e->contrib_d + (V + 4) / 4 * 4;  // 16-byte aligned; 8 of at least 24 B per vertex
     }
     if (e->batch_enabled)
       for (int i = 0; i < 3; i++) e->bmask[i] = (unsigned long long *)e->arena + (uint64_t)i * (V + 1);
@@ -706,12 +706,12 @@ int create(og_graph *g, const og_config *cfg, og_engine *e) {
                             cudaFuncAttributePreferredSharedMemoryCarveout, 58));
     CK(cudaFuncSetAttribute(k_lbs<SrcF<true>, MinOp<true>>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
   }
-  // Same for the PageRank pull (29 KB tiles: 4 CTAs per SM at 58 %).  R-MAT 26
-  // directed: 58.5 iterations/s with the CUDA driver's choice, 69.6 at 58 %,
-  // 68.4 at 44 %, 63.2 at 30 %, 34.0 at 86 %.
-  CK(cudaFuncSetAttribute(k_pr_pull<SrcP<false>>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
-  CK(cudaFuncSetAttribute(k_pr_pull_pair<SrcP<false>, SrcP<false>>,
-                          cudaFuncAttributePreferredSharedMemoryCarveout, 58));
+  // The cursor form of the PageRank pull (18 KB of tables a CTA): 58 %.  The
+  // contiguous form (10 KB) runs within 1.5 % of its best at the CUDA driver's
+  // choice (8.4 M vertices, 131 M edges, 49 iterations: 30.9 ms; 30.5 at 30 %,
+  // 37.1 at 20 %, 33.5 at 70 %).
+  CK(cudaFuncSetAttribute(k_pr_pull<false, SrcP<false>>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
+  CK(cudaFuncSetAttribute(k_pr_pull_pair<false, SrcP<false>>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
 
   // host CSR: page-lock so kernels can gather from it over the link
   if (P.dynamic_edges > 0) {
@@ -2270,14 +2270,29 @@ int run_sssp_batch(og_engine *e, const uint32_t *srcs, uint32_t n, uint32_t *out
 
 // ------------------------------------------------------------------ PageRank
 
+// Whether region r's compacted list holds every record of the region, so that
+// list position q is record base + q.
+bool pr_contiguous(const og_engine *e, int r) {
+  return e->counts_h[r].total == (r == 0 ? e->plan.static_edges : e->g->E - e->plan.static_edges);
+}
+
+template <bool kDense>
+int launch_pr_pull(og_engine *e, const LbsArgs &a, SrcP<false> src, const PrArgs &p, cudaStream_t s) {
+  const unsigned grid = lbs_grid(a.pos_begin, a.pos_end);
+  if (grid) {
+    k_pr_pull<kDense><<<grid, kThreads, pr_smem_bytes(kDense, src.bpe), s>>>(a, src, p);
+    e->launches++;
+  }
+  return OG_OK;
+}
+
 int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
-  PrArgs p;
+  PrArgs p{};
   p.contrib = e->contrib_d;
   p.sum = e->sum_d;
   p.V = e->V;
   // static tiles use [0, tile_cap0), dynamic tiles [tile_cap0, ...)
   const uint64_t toff[2] = {0, e->tile_cap[0]};
-  CK(cudaMemsetAsync(e->carry_idx_d, 0xff, 4 * e->pr_tiles, e->s_main));
   CK(cudaEventRecord(e->ev_round, e->s_main));
   CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
   CK(cudaStreamWaitEvent(e->s_gat, e->ev_round, 0));
@@ -2286,39 +2301,50 @@ int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
     q.cont = e->cont_d + toff[r];
     q.carry = e->carry_d + toff[r];
     q.carry_idx = e->carry_idx_d + toff[r];
+    q.base = r ? e->plan.static_edges : 0;
+    q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
     return q;
   };
   auto sfn = [&](const LbsArgs &a) {
-    const unsigned grid = lbs_grid(a.pos_begin, a.pos_end);
-    if (grid) {
-      k_pr_pull<EKU::PSrc><<<grid, kThreads, 0, e->s_main>>>(a, EKU::stat(e), args_for(0));
-      e->launches++;
-    }
-    return (int)OG_OK;
+    return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), args_for(0), e->s_main)
+                               : launch_pr_pull<false>(e, a, EKU::stat(e), args_for(0), e->s_main);
   };
   auto dfn = [&](const LbsArgs &a, auto src, cudaStream_t ds) {
-    const unsigned grid = lbs_grid(a.pos_begin, a.pos_end);
-    if (grid) {
-      k_pr_pull<decltype(src)><<<grid, kThreads, 0, ds>>>(a, src, args_for(1));
-      e->launches++;
+    if constexpr (std::is_same<decltype(src), SrcU>::value) {
+      // a staging buffer: columns from position pos_begin on, as 32-bit records
+      PrArgs q = args_for(1);
+      q.base = 0ull - a.pos_begin;
+      q.nwords = a.edge_bound;
+      return launch_pr_pull<true>(e, a, SrcP<false>{src.col, 32u, 32u, 0u}, q, ds);
+    } else {
+      return pr_contiguous(e, 1) ? launch_pr_pull<true>(e, a, src, args_for(1), ds)
+                                 : launch_pr_pull<false>(e, a, src, args_for(1), ds);
     }
-    return (int)OG_OK;
   };
   auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
     const uint64_t n0 = lbs_grid(a0.pos_begin, a0.pos_end), n1 = lbs_grid(a1.pos_begin, a1.pos_end);
     if (n0 + n1 > 0x7fffffffull) return fail(OG_E_STATE, "pull grid too large");
-    k_pr_pull_pair<decltype(s0), decltype(s1)><<<(unsigned)(n0 + n1), kThreads, 0, ps>>>(
-        a0, s0, args_for(0), a1, s1, args_for(1), n0, n0 + n1);
+    const unsigned n = (unsigned)(n0 + n1);
+    if (pr_contiguous(e, 0) && pr_contiguous(e, 1))
+      k_pr_pull_pair<true><<<n, kThreads, pr_smem_bytes(true, e->bpe), ps>>>(a0, s0, args_for(0), a1, s1, args_for(1),
+                                                                             n0, n);
+    else
+      k_pr_pull_pair<false><<<n, kThreads, pr_smem_bytes(false, e->bpe), ps>>>(a0, s0, args_for(0), a1, s1,
+                                                                               args_for(1), n0, n);
     e->launches++;
     return (int)OG_OK;
   };
   RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn)));
+  PrFixup f[2];
+  uint64_t nt[2];
   for (int r = 0; r < 2; r++) {
     const Counts c = e->counts_h[r];
-    if (!c.n) continue;
-    const uint64_t nt = (c.total + kTile - 1) / kTile;
-    k_pr_fixup<<<(unsigned)((nt + kThreads - 1) / kThreads), kThreads, 0, e->s_main>>>(
-        e->list_d[r], e->pref_d[r], 0, nt, args_for(r));
+    f[r] = PrFixup{e->list_d[r], e->pref_d[r], c.n, args_for(r)};
+    nt[r] = c.n ? (c.total + kTile - 1) / kTile : 0;
+  }
+  if (nt[0] + nt[1]) {
+    k_pr_fixup<<<(unsigned)((nt[0] + nt[1] + kThreads - 1) / kThreads), kThreads, 0, e->s_main>>>(f[0], nt[0], f[1],
+                                                                                              nt[1]);
     e->launches++;
   }
   CK(cudaGetLastError());
