@@ -260,9 +260,7 @@ typedef struct og_stats {
   double ms_gather;          /* device time of the dynamic gather kernels   */
   double ms_relax;           /* device-driven rounds with
                                 OG_PARAM_RELAX_TIMER: time of the (top-down)
-                                relax launches, between stamp kernels
-                                enqueued right before and after each;
-                                otherwise 0                                 */
+                                relax phases; otherwise 0                   */
 } og_stats;
 
 /* initGraphHost + getMaxPartitionSize + initGraphDevice
@@ -471,17 +469,19 @@ int og_engine_clone(og_engine *parent, og_engine **out);
 #define OG_BFS_AUTO 0
 #define OG_BFS_TOP_DOWN 1
 /* OG_PARAM_LEVEL_LOOP: OG_LOOP_AUTO (default) runs the levels / rounds of
- *   og_bfs, og_sssp and label-propagation og_cc from two CUDA graphs replayed
- *   back to back, with every per-round decision taken by kernels (direct mode
- *   or a fully resident graph; staged engines keep the host loop); the host
- *   checks for the end every few rounds.  OG_LOOP_HOST waits for each round's
+ *   og_bfs, og_sssp and label-propagation og_cc on the device, in one
+ *   cooperative kernel that takes every per-round decision itself (BFS: with
+ *   a one-CTA kernel for small frontiers beside it), in direct mode or on a
+ *   fully resident graph of fewer than 2^28 vertices and 2^36 edges; other
+ *   engines keep the host loop.  OG_LOOP_HOST waits for each round's
  *   counts on the host.  Results are identical. */
 #define OG_PARAM_LEVEL_LOOP 4
 #define OG_LOOP_AUTO 0
 #define OG_LOOP_HOST 1
-/* OG_PARAM_RELAX_TIMER: 1 brackets every relax launch of the device-driven
- *   rounds with two one-thread stamp kernels that read the GPU's global timer
- *   (og_stats.ms_relax); 0 (default) leaves them out of the captured rounds. */
+/* OG_PARAM_RELAX_TIMER: 1 sums the time of the (top-down) relax phases of the
+ *   device-driven rounds, read from the GPU's global timer after the grid
+ *   barriers around each (og_stats.ms_relax); 0 (default) does not read it.
+ *   Levels of small BFS frontiers, expanded by one CTA, count as a whole. */
 #define OG_PARAM_RELAX_TIMER 5
 /* OG_PARAM_SSSP_BATCH_DELTA: near/far width of og_sssp_batch, shared by its
  *   sources.  0 (default) expands every improved (vertex, source) pair every

@@ -94,14 +94,17 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, uint32_t *err, u
       st_release((uint32_t *)&bar[1], gen + 1);
     } else {
       uint32_t spins = 0;
-      while (ld_acquire((const uint32_t *)&bar[1]) == gen) {
+      // relaxed polls, then one fence: an acquiring poll drops the SM's L1 each
+      // time, under the CTAs that still work
+      while (ld_relaxed((const uint32_t *)&bar[1]) == gen) {
         if (++spins > spin_limit) {
           atomicOr(err, kErrBarrier);
           ok = 0;
           break;
         }
-        __nanosleep(128);
+        __nanosleep(32);
       }
+      __threadfence();
     }
     s_ok = ok;
   }

@@ -20,9 +20,9 @@
 #include <vector>
 
 #include "batch_persist.cuh"
-#include "bfs_loop.cuh"
 #include "kernels.cuh"
 #include "og_internal.hpp"
+#include "rounds.cuh"
 #include "sssp_batch.cuh"
 
 using namespace og;
@@ -133,21 +133,11 @@ struct og_engine {
   uint32_t *pmisc_h = nullptr;  // host copy of bar_d
   int tuned = -1;               // index into kPersistConfigs chosen by the autotuner
   cudaGraphExec_t graph = nullptr;
-  // device-driven BFS level loop: state, its host mirror, one graph per
-  // frontier parity (captured for the direction mode `bfs_exec_dopt`)
-  BfsLoop *loop_d = nullptr, *loop_h = nullptr;
-  cudaGraphExec_t bfs_exec[2] = {nullptr, nullptr};
-  int bfs_exec_dopt = -1;
-  uint32_t dev_epoch = 1u << 29;  // epochs of device-driven compactions: [2^29, 2^30)
-  uint32_t bfs_levels_hint = 4;   // levels of the last BFS (launched before the first check)
+  // device-driven rounds (rounds.cuh): state and its page-locked host mirror
+  RoundsState *rounds_d = nullptr, *rounds_h = nullptr;
   uint32_t level_loop = 0;        // OG_LOOP_AUTO / OG_LOOP_HOST
   uint32_t relax_timer = 0;       // OG_PARAM_RELAX_TIMER
-  // device-driven SSSP / CC rounds: state, host mirror, round graphs captured
-  // for (algorithm, split) = min_exec_key
-  MinLoop *mloop_d = nullptr, *mloop_h = nullptr;
-  cudaGraphExec_t min_exec[2] = {nullptr, nullptr};
-  int min_exec_key = -1;
-  uint32_t min_rounds_hint[2] = {16, 4};  // SSSP, CC
+  void *out = nullptr;            // the running query's result buffer, until its copy is enqueued
   uint32_t graph_n = 0;
   int graph_cfg = -1;
   int graph_dopt = -1;
@@ -492,12 +482,7 @@ void destroy(og_engine *e) {
   if (e->sb_ck_h) cudaFreeHost(e->sb_ck_h);
   if (e->pmisc_h) cudaFreeHost(e->pmisc_h);
   if (e->graph) cudaGraphExecDestroy(e->graph);
-  for (int p = 0; p < 2; p++)
-    if (e->bfs_exec[p]) cudaGraphExecDestroy(e->bfs_exec[p]);
-  if (e->loop_h) cudaFreeHost(e->loop_h);
-  for (int p = 0; p < 2; p++)
-    if (e->min_exec[p]) cudaGraphExecDestroy(e->min_exec[p]);
-  if (e->mloop_h) cudaFreeHost(e->mloop_h);
+  if (e->rounds_h) cudaFreeHost(e->rounds_h);
   if (e->err_h) cudaFreeHost(e->err_h);
   if (e->l1_h) cudaFreeHost(e->l1_h);
   cudaEvent_t evs[] = {e->ev_round, e->ev_cs, e->ev_cd, e->ev_dyn_done, e->ev_gat[0], e->ev_gat[1],
@@ -570,10 +555,8 @@ int create_query_state(og_engine *e) {
   e->active_d = e->err_d + 1;
   RC(dalloc(e, &e->sum64_d, 3ull * e->sms * 8 + 4));
   CK(cudaMallocHost(&e->counts_h, 3 * sizeof(Counts)));
-  RC(dalloc(e, (char **)&e->loop_d, sizeof(BfsLoop)));
-  CK(cudaMallocHost(&e->loop_h, sizeof(BfsLoop)));
-  RC(dalloc(e, (char **)&e->mloop_d, sizeof(MinLoop)));
-  CK(cudaMallocHost(&e->mloop_h, sizeof(MinLoop)));
+  RC(dalloc(e, (char **)&e->rounds_d, sizeof(RoundsState)));
+  CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState)));
   CK(cudaMallocHost(&e->err_h, 4 * sizeof(uint32_t)));
   CK(cudaMallocHost(&e->l1_h, sizeof(double)));
   if (P.chunk_edges && !(e->cfg.flags & OG_CFG_DIRECT)) {
@@ -699,8 +682,8 @@ int create(og_graph *g, const og_config *cfg, og_engine *e) {
   // choice, 9.85 at 58 %, 6.77 at 86 %, 8.06 at 30 %.
   CK(cudaFuncSetAttribute(k_lbs_pair<SrcP<true>, SrcP<true>, MinOp<true>>,
                           cudaFuncAttributePreferredSharedMemoryCarveout, 58));
-  CK(cudaFuncSetAttribute(k_lbs_pair_dev<SrcP<true>, SrcP<true>, MinOp<true>>,
-                          cudaFuncAttributePreferredSharedMemoryCarveout, 58));
+  CK(cudaFuncSetAttribute(k_min_rounds<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
+  CK(cudaFuncSetAttribute(k_bfs_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared)));
   if (cfg->flags & OG_CFG_REPLACE) {  // the same relax reading fragment slots
     CK(cudaFuncSetAttribute(k_lbs_pair<SrcP<true>, SrcF<true>, MinOp<true>>,
                             cudaFuncAttributePreferredSharedMemoryCarveout, 58));
@@ -808,10 +791,6 @@ int clone(og_engine *parent, og_engine *e) {
 // waiting ones go to far_bits (when not null) and their minimum to the
 // region's Counts::far_min; listed ones are cleared from clear_bits.
 struct SplitArgs {
-  // device-driven loops: epoch read from device memory, launch gated by a flag
-  const uint32_t *epoch_ptr = nullptr;
-  const uint32_t *run_flag = nullptr;
-  const uint32_t *thr_ptr = nullptr;
   bool on = false;
   uint32_t thr = 0;
   uint32_t *far_bits = nullptr;
@@ -859,9 +838,6 @@ int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint3
   a.far_key = (unsigned long long *)(e->counts_d + 2) + r;
   a.clear_bits = sp.clear_bits;
   a.epoch = e->epoch;
-  a.epoch_ptr = sp.epoch_ptr;
-  a.run_flag = sp.run_flag;
-  a.thr_ptr = sp.thr_ptr;
   if (a.ntiles + 1 > e->lb_tiles) return fail(OG_E_STATE, "compaction scratch too small");
   k_compact<<<a.ntiles, kThreads, 0, s>>>(a);
   e->launches++;
@@ -1147,9 +1123,7 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
     e->launches += 2;
   } else if (algo == OG_ALGO_SSSP) {
     if (e->sssp_delta > 0) CK(cudaMemsetAsync(e->bm[2], 0, 4 * e->nwords, s));  // waiting set
-    // far keys: a device-driven query leaves keys of higher epochs, which
-    // atomicMax would keep over this query's
-    CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), s));
+    CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), s));  // far keys of earlier queries
     k_fill_u32<<<g, kThreads, 0, s>>>(e->value_d, V, 0xFFFFFFFFu);  // SSSP GraphMeta.h:377
     k_set_source<<<1, 1, 0, s>>>(e->value_d, src, 1u, cur, nullptr);
     e->launches += 2;
@@ -1271,266 +1245,93 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
   return OG_OK;
 }
 
-// ------------------------------------------------------- device-driven BFS
+// ---------------------------------------------------- device-driven rounds
 
-// Captures one BFS level for the frontier in bm[p] (next in bm[1 - p]).
-int capture_bfs_level(og_engine *e, int p, int dopt, cudaGraphExec_t *out) {
-  cudaStream_t s = e->s_main;
-  uint32_t *cur = e->bm[p], *next = e->bm[1 - p];
-  BfsLoop *L = e->loop_d;
-  cudaGraph_t gr = nullptr;
-  const uint64_t before = e->launches;
-  int per_sm = 0;  // fixed grid of the top-down relax: every CTA resident
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lbs_pair_dev<EKU::PSrc, EKU::PSrc, BfsOp>, kThreads, 0));
-  const unsigned grid = (unsigned)std::max(1, per_sm) * (unsigned)e->sms;
-  CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int rc = OG_OK;
-  auto body = [&]() -> int {
-    SplitArgs sp;
-    sp.epoch_ptr = &L->epoch;
-    sp.run_flag = &L->compact_go;
-    CK(cudaEventRecord(e->ev_round, s));
-    CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-    RC(launch_compact(e, 0, cur, 0, e->Vs, s, sp));
-    RC(launch_compact(e, 1, cur, e->Vs, e->V, e->s_dyn, sp));
-    CK(cudaEventRecord(e->ev_cd, e->s_dyn));
-    CK(cudaStreamWaitEvent(s, e->ev_cd, 0));
-    k_bfs_ctl_mid<<<1, 32, 0, s>>>(L, e->counts_d, dopt);
-    BfsOp op{e->bm[2], next, e->value_d, e->err_d, e->V, 0};
-    if (e->relax_timer) k_stamp<<<1, 1, 0, s>>>(&L->td_go, L->relax_timer, 0);
-    k_lbs_pair_dev<EKU::PSrc, EKU::PSrc, BfsOp><<<grid, kThreads, 0, s>>>(
-        lbs_args(e, 0, 0, 0, true, e->plan.static_edges), EKU::stat(e), lbs_args(e, 1, 0, 0, true, e->g->E),
-        EKU::host(e), op, e->counts_d, &L->td_go, &L->level, &L->tile_next);
-    if (e->relax_timer) k_stamp<<<1, 1, 0, s>>>(&L->td_go, L->relax_timer, 1);
-    k_bfs_bottom_up<EKU::PSrc><<<grid_for(e->V, e->sms), kThreads, 0, s>>>(
-        e->off_d, e->V, e->Vs, EKU::stat(e), EKU::host(e), cur, e->bm[2], next, e->value_d, 0, L->bu,
-        e->err_d, &L->bu_go, &L->level);
-    k_bfs_ctl_end<<<1, 32, 0, s>>>(L, e->V);
-    CK(cudaMemsetAsync(cur, 0, 4 * e->nwords, s));  // the expanded frontier: next level's "next"
-    return OG_OK;
-  };
-  rc = body();
-  const cudaError_t ce = cudaStreamEndCapture(s, &gr);
-  e->launches = before;  // captured, not launched
-  if (rc != OG_OK || ce != cudaSuccess) {
-    if (gr) cudaGraphDestroy(gr);
-    cudaGetLastError();
-    return rc != OG_OK ? rc : fail(OG_E_CUDA, "BFS level capture: %s", cudaGetErrorString(ce));
-  }
-  const cudaError_t ie = cudaGraphInstantiate(out, gr, 0);
-  cudaGraphDestroy(gr);
-  if (ie != cudaSuccess) return fail(OG_E_CUDA, "BFS level graph: %s", cudaGetErrorString(ie));
-  return OG_OK;
+// Whether a query runs in one cooperative kernel (rounds.cuh): direct mode or a
+// fully resident graph (no staging pipeline to drive), and counters that fit
+// its packed list reservations.
+bool rounds_on_device(const og_engine *e) {
+  return e->level_loop == OG_LOOP_AUTO && (e->plan.dynamic_edges == 0 || (e->cfg.flags & OG_CFG_DIRECT)) &&
+         rounds_fit(e->V, e->g->E);
 }
 
-// Single-source BFS with the device-driven level loop (see bfs_loop.cuh):
-// the two level graphs alternate; the host checks the done flag after as many
-// levels as the previous query took, then every two levels.
-int run_bfs_dev(og_engine *e, uint32_t src, og_stats &st) {
-  const uint64_t V = e->V;
+// BFS, SSSP or label-propagation CC as one kernel; the result is copied to the
+// caller's buffer behind it, so that the host waits once.
+int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   cudaStream_t s = e->s_main;
-  const int g = grid_for(V, e->sms);
-  // the captured graphs depend on the direction mode and the relax timer
-  const int dopt = (e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1) | (e->relax_timer ? 2 : 0);
-  if (dopt != e->bfs_exec_dopt) {
-    for (int p = 0; p < 2; p++)
-      if (e->bfs_exec[p]) {
-        cudaGraphExecDestroy(e->bfs_exec[p]);
-        e->bfs_exec[p] = nullptr;
-      }
-    for (int p = 0; p < 2; p++) RC(capture_bfs_level(e, p, dopt & 1, &e->bfs_exec[p]));
-    e->bfs_exec_dopt = dopt;
+  RoundsArgs a{};
+  a.V = e->V;
+  a.Vs = e->Vs;
+  a.E = e->g->E;
+  a.static_edges = e->plan.static_edges;
+  a.nwords = e->nwords;
+  a.off = e->off_d;
+  a.value = e->value_d;
+  for (int i = 0; i < 3; i++) a.bm[i] = e->bm[i];
+  for (int r = 0; r < 2; r++) {
+    a.list[r] = e->list_d[r];
+    a.pref[r] = e->pref_d[r];
+    a.tile[r] = e->tile_d[r];
+    a.list_cap[r] = e->list_cap[r];
+    a.tile_cap[r] = e->tile_cap[r];
   }
-  if (e->dev_epoch > (1u << 30) - (1u << 20)) {  // epoch wrap: clear the status words once
-    for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, s));
-    e->dev_epoch = 1u << 29;
+  a.st = e->rounds_d;
+  a.src = src;
+  a.delta = algo == OG_ALGO_SSSP ? e->sssp_delta : 0;
+  a.split = a.delta ? 1u : 0u;
+  a.dopt = algo == OG_ALGO_BFS && e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1;
+  a.timer = e->relax_timer;
+  SrcP<false> u0 = EKU::stat(e), u1 = EKU::host(e);
+  SrcP<true> w0{e->spk_d, e->bpe, e->bc, e->wmin}, w1{e->hpk_d, e->bpe, e->bc, e->wmin};
+  const bool bfs = algo == OG_ALGO_BFS;
+  const void *kern = bfs                    ? (const void *)k_bfs_rounds
+                     : algo == OG_ALGO_SSSP ? (const void *)k_min_rounds<true>
+                                            : (const void *)k_min_rounds<false>;
+  int occ = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, 0));
+  if (occ < 1) return fail(OG_E_UNSUPPORTED, "rounds kernel does not fit an SM");
+  // all the CTAs that fit at once, or one per edge tile and per 1024 vertices
+  // when the graph has fewer: a barrier over a few CTAs is cheaper
+  const uint64_t work = std::max<uint64_t>(a.E / kTile, a.V / 1024) + 1;
+  const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)occ * e->sms, work);
+  void *args[3] = {&a, &u0, &u1};
+  if (algo == OG_ALGO_SSSP) {
+    args[1] = &w0;
+    args[2] = &w1;
   }
-  CK(cudaMemsetAsync(e->err_d, 0, 16, s));
-  CK(cudaMemsetAsync(e->bm[0], 0, 4 * e->nwords, s));
-  CK(cudaMemsetAsync(e->bm[1], 0, 4 * e->nwords, s));
-  CK(cudaMemsetAsync(e->bm[2], 0, 4 * e->nwords, s));
-  k_fill_u32<<<g, kThreads, 0, s>>>(e->value_d, V, (uint32_t)(V + 1));  // GraphMeta.h:378
-  k_set_source<<<1, 1, 0, s>>>(e->value_d, src, 1u, e->bm[0], e->bm[2]);
-  BfsLoop &h = *e->loop_h;
-  memset(&h, 0, sizeof h);
-  h.level = 1;
-  h.need_compact = 1;
-  h.compact_go = 1;
-  h.epoch = e->dev_epoch;
-  h.unexplored = e->g->E;
-  CK(cudaMemcpyAsync(e->loop_d, &h, sizeof h, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(e->t_d0, s));
-  uint32_t launched = 0, batch = std::max<uint32_t>(2, e->bfs_levels_hint + 1);
-  for (;;) {
-    for (uint32_t i = 0; i < batch; i++, launched++) CK(cudaGraphLaunch(e->bfs_exec[launched & 1], s));
-    CK(cudaMemcpyAsync(&h.done, &e->loop_d->done, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (h.done) break;
-    if (launched > 4 * V + 64) return fail(OG_E_STATE, "BFS did not end after %u levels", launched);
-    batch = 2;
-  }
-  CK(cudaEventRecord(e->ev_dyn_done, s));
-  CK(cudaMemcpyAsync(&h, e->loop_d, sizeof h, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  RC(check_device_error(e));
-  float ms = 0;
-  if (cudaEventElapsedTime(&ms, e->t_d0, e->ev_dyn_done) == cudaSuccess) st.ms_dynamic += ms;
-  st.iterations += (uint32_t)h.iterations;
-  st.frontier_sum += h.frontier_sum;
-  st.edges_static += h.edges_static;
-  st.edges_dynamic += h.edges_dynamic;
-  st.link_bytes += (h.edges_dynamic * e->bpe + 7) / 8;
-  st.chunks += (uint32_t)h.iterations;
-  st.ms_relax += h.relax_timer[1] / 1e6;
-  e->launches += 2 + (7ull + (e->relax_timer ? 2 : 0)) * launched;
-  e->bfs_levels_hint = (uint32_t)h.iterations;
-  e->dev_epoch = h.epoch + 1;
-  e->last_algo = OG_ALGO_BFS;
-  return OG_OK;
-}
-
-// Captures one SSSP / CC round for the frontier in bm[p] (next in bm[1 - p],
-// waiting set in bm[2]); see bfs_loop.cuh.
-template <class K, bool kW>
-int capture_min_round(og_engine *e, int p, bool split, cudaGraphExec_t *out) {
-  cudaStream_t s = e->s_main;
-  uint32_t *cur = e->bm[p], *next = e->bm[1 - p], *waiting = e->bm[2];
-  MinLoop *L = e->mloop_d;
-  const unsigned long long *keys = (const unsigned long long *)(e->counts_d + 2);
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, k_lbs_pair_dev<typename K::PSrc, typename K::PSrc, MinOp<kW>>, kThreads, 0));
-  const unsigned grid = (unsigned)std::max(1, per_sm) * (unsigned)e->sms;
-  cudaGraph_t gr = nullptr;
-  const uint64_t before = e->launches;
-  CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  auto compact_both = [&](const uint32_t *bits, const SplitArgs &sp) -> int {
-    CK(cudaEventRecord(e->ev_round, s));
-    CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-    RC(launch_compact(e, 0, bits, 0, e->Vs, s, sp));
-    RC(launch_compact(e, 1, bits, e->Vs, e->V, e->s_dyn, sp));
-    CK(cudaEventRecord(e->ev_cd, e->s_dyn));
-    CK(cudaStreamWaitEvent(s, e->ev_cd, 0));
-    return OG_OK;
-  };
-  auto body = [&]() -> int {
-    SplitArgs sr;
-    sr.epoch_ptr = &L->epoch;
-    sr.run_flag = &L->round_go;
-    sr.thr_ptr = &L->thr;
-    sr.on = split;
-    sr.far_bits = split ? waiting : nullptr;
-    sr.clear_bits = split ? waiting : nullptr;
-    RC(compact_both(cur, sr));
-    k_min_ctl_a<<<1, 32, 0, s>>>(L, e->counts_d, keys);
-    if (split) {
-      SplitArgs sa = sr;
-      sa.run_flag = &L->adv_go;
-      sa.far_bits = nullptr;
-      RC(compact_both(waiting, sa));
-      k_min_ctl_b<<<1, 32, 0, s>>>(L, e->counts_d, keys);
-    }
-    MinOp<kW> op{e->value_d, next, e->err_d, e->V};
-    if (e->relax_timer) k_stamp<<<1, 1, 0, s>>>(&L->relax_go, L->relax_timer, 0);
-    k_lbs_pair_dev<typename K::PSrc, typename K::PSrc, MinOp<kW>><<<grid, kThreads, 0, s>>>(
-        lbs_args(e, 0, 0, 0, true, e->plan.static_edges), K::stat(e), lbs_args(e, 1, 0, 0, true, e->g->E),
-        K::host(e), op, e->counts_d, &L->relax_go, nullptr, &L->tile_next);
-    if (e->relax_timer) k_stamp<<<1, 1, 0, s>>>(&L->relax_go, L->relax_timer, 1);
-    k_min_ctl_end<<<1, 32, 0, s>>>(L);
-    CK(cudaMemsetAsync(cur, 0, 4 * e->nwords, s));
-    return OG_OK;
-  };
-  const int rc = body();
-  const cudaError_t ce = cudaStreamEndCapture(s, &gr);
-  e->launches = before;  // captured, not launched
-  if (rc != OG_OK || ce != cudaSuccess) {
-    if (gr) cudaGraphDestroy(gr);
-    cudaGetLastError();
-    return rc != OG_OK ? rc : fail(OG_E_CUDA, "round capture: %s", cudaGetErrorString(ce));
-  }
-  const cudaError_t ie = cudaGraphInstantiate(out, gr, 0);
-  cudaGraphDestroy(gr);
-  if (ie != cudaSuccess) return fail(OG_E_CUDA, "round graph: %s", cudaGetErrorString(ie));
-  return OG_OK;
-}
-
-// SSSP (algo OG_ALGO_SSSP) or label-propagation CC with device-driven rounds.
-int run_min_dev(og_engine *e, int algo, uint32_t src, og_stats &st) {
-  const uint64_t V = e->V;
-  cudaStream_t s = e->s_main;
-  const int g = grid_for(V, e->sms);
-  const bool sssp = algo == OG_ALGO_SSSP;
-  const bool split = sssp && e->sssp_delta > 0;
-  const int key = (sssp ? 2 : 0) + (split ? 1 : 0) + (e->relax_timer ? 4 : 0);
-  if (key != e->min_exec_key) {
-    for (int p = 0; p < 2; p++)
-      if (e->min_exec[p]) {
-        cudaGraphExecDestroy(e->min_exec[p]);
-        e->min_exec[p] = nullptr;
-      }
-    for (int p = 0; p < 2; p++)
-      RC((sssp ? capture_min_round<EK<uint8_t>, true>(e, p, split, &e->min_exec[p])
-               : capture_min_round<EKU, false>(e, p, false, &e->min_exec[p])));
-    e->min_exec_key = key;
-  }
-  if (e->dev_epoch > (1u << 30) - (1u << 20)) {  // epoch wrap: clear the status words once
-    for (int r = 0; r < 2; r++)
-      CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * e->lb_tiles, s));
-    CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), s));
-    e->dev_epoch = 1u << 29;
-  }
-  CK(cudaMemsetAsync(e->err_d, 0, 16, s));
-  CK(cudaMemsetAsync(e->bm[0], 0, 4 * e->nwords, s));
-  CK(cudaMemsetAsync(e->bm[1], 0, 4 * e->nwords, s));
-  if (sssp) {
-    if (split) CK(cudaMemsetAsync(e->bm[2], 0, 4 * e->nwords, s));  // waiting set
-    CK(cudaMemsetAsync(e->counts_d + 2, 0, sizeof(Counts), s));    // far keys of earlier queries
-    k_fill_u32<<<g, kThreads, 0, s>>>(e->value_d, V, 0xFFFFFFFFu);  // SSSP GraphMeta.h:377
-    k_set_source<<<1, 1, 0, s>>>(e->value_d, src, 1u, e->bm[0], nullptr);
+  RoundsState &h = *e->rounds_h;
+  if (bfs) {
+    k_bfs_init<<<grid_for(std::max<uint64_t>(a.V, a.nwords), e->sms), kThreads, 0, s>>>(a);
+    e->launches++;
   } else {
-    k_iota_u32<<<g, kThreads, 0, s>>>(e->value_d, V);  // CC GraphMeta.h:341-345
-    k_fill_bits<<<g, kThreads, 0, s>>>(e->bm[0], e->nwords, V);
+    CK(cudaMemsetAsync(e->rounds_d, 0, sizeof(RoundsState), s));
   }
-  MinLoop &h = *e->mloop_h;
-  memset(&h, 0, sizeof h);
-  h.epoch = e->dev_epoch;
-  const uint64_t thr = 1ull + e->sssp_delta;
-  h.thr = thr > 0xffffffffull ? 0xffffffffu : (uint32_t)thr;
-  h.round_go = 1;
-  h.far_min = 0xffffffffu;
-  h.delta = e->sssp_delta;
-  h.split = split ? 1 : 0;
-  CK(cudaMemcpyAsync(e->mloop_d, &h, sizeof h, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(e->t_d0, s));
-  uint32_t &hint = e->min_rounds_hint[sssp ? 0 : 1];
-  uint32_t launched = 0, batch = std::max<uint32_t>(2, hint + 2);
-  for (;;) {
-    for (uint32_t i = 0; i < batch; i++, launched++) CK(cudaGraphLaunch(e->min_exec[launched & 1], s));
-    CK(cudaMemcpyAsync(&h.done, &e->mloop_d->done, 4, cudaMemcpyDeviceToHost, s));
+  for (uint64_t pass = 0;; pass++) {
+    if (bfs) {
+      k_bfs_small<<<1, kSmallThreads, sizeof(SmallShared), s>>>(a, u0, u1);
+      e->launches++;
+    }
+    CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, 0, s));
+    e->launches++;
+    CK(cudaMemcpyAsync(&h, e->rounds_d, sizeof h, cudaMemcpyDeviceToHost, s));
+    // the result goes out behind the first pair, which ends most queries
+    if (e->out) CK(cudaMemcpyAsync(e->out, e->value_d, 4ull * e->V, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (h.done) break;
-    if (launched > 8 * V + 64) return fail(OG_E_STATE, "rounds did not end after %u", launched);
-    batch = 8;
+    if (!bfs || h.done || h.err) break;
+    if (pass > a.V) return fail(OG_E_STATE, "BFS did not end");
   }
-  CK(cudaEventRecord(e->ev_dyn_done, s));
-  CK(cudaMemcpyAsync(&h, e->mloop_d, sizeof h, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
+  e->out = nullptr;
+  if (h.err & kErrBarrier) return fail(OG_E_TIMEOUT, "grid barrier wait gave up");
+  *e->err_h = h.err;
   RC(check_device_error(e));
-  float ms = 0;
-  if (cudaEventElapsedTime(&ms, e->t_d0, e->ev_dyn_done) == cudaSuccess) st.ms_dynamic += ms;
+  st.ms_dynamic += h.ns_total / 1e6;
+  st.ms_relax += h.ns_relax / 1e6;
   st.iterations += (uint32_t)h.iterations;
   st.frontier_sum += h.frontier_sum;
   st.edges_static += h.edges_static;
   st.edges_dynamic += h.edges_dynamic;
   st.link_bytes += (h.edges_dynamic * e->bpe + 7) / 8;
   st.chunks += (uint32_t)h.iterations;
-  st.ms_relax += h.relax_timer[1] / 1e6;
-  e->launches += 2 + ((split ? 11ull : 7ull) + (e->relax_timer ? 2 : 0)) * launched;
-  hint = h.rounds;  // rounds this query needed (the next one is launched that far before its first check)
-  e->dev_epoch = h.epoch + 1;
   e->last_algo = algo;
   return OG_OK;
 }
@@ -2521,9 +2322,11 @@ int query_common(og_engine *e, int algo, og_stats *st_out, void *out,
     e->sb_session = false;
     e->bb_session = false;
     const double t0 = now_ms();
+    e->out = out;
     RC(body(e, st, ctx));
     st.launches = e->launches;
-    if (out) RC(fetch(e, out));
+    if (e->out) RC(fetch(e, out));  // unless the body has copied it
+    e->out = nullptr;
     st.ms_total = now_ms() - t0;
     if (st_out) *st_out = st;
     (void)algo;
@@ -2688,11 +2491,7 @@ extern "C" int og_bfs(og_engine *e, uint32_t src, uint32_t *out_depth, og_stats 
     if (en->frag && en->frag->broken)
       return fail(OG_E_STATE, "the fragment slots were not laid out (a failed OG_PARAM_FRAGMENT_WORDS change)");
     if (en->frag) return run_frontier<EKF<void>>(en, OG_ALGO_BFS, src_, s);
-    // the device-driven loop needs no staging pipeline: direct mode or a
-    // fully resident graph
-    const bool dev = en->level_loop == OG_LOOP_AUTO &&
-                     (en->plan.dynamic_edges == 0 || (en->cfg.flags & OG_CFG_DIRECT));
-    return dev ? run_bfs_dev(en, src_, s) : run_frontier<EKU>(en, OG_ALGO_BFS, src_, s);
+    return rounds_on_device(en) ? run_rounds(en, OG_ALGO_BFS, src_, s) : run_frontier<EKU>(en, OG_ALGO_BFS, src_, s);
   }, &src);
 }
 
@@ -2704,8 +2503,7 @@ extern "C" int og_sssp(og_engine *e, uint32_t src, uint32_t *out_dist, og_stats 
     if (en->frag && en->frag->broken)
       return fail(OG_E_STATE, "the fragment slots were not laid out (a failed OG_PARAM_FRAGMENT_WORDS change)");
     if (en->frag) return run_frontier<EKF<uint8_t>>(en, OG_ALGO_SSSP, src_, s);
-    if (en->level_loop == OG_LOOP_AUTO && (en->plan.dynamic_edges == 0 || (en->cfg.flags & OG_CFG_DIRECT)))
-      return run_min_dev(en, OG_ALGO_SSSP, src_, s);
+    if (rounds_on_device(en)) return run_rounds(en, OG_ALGO_SSSP, src_, s);
     if (en->wbytes == 1) return run_frontier<EK<uint8_t>>(en, OG_ALGO_SSSP, src_, s);
     if (en->wbytes == 2) return run_frontier<EK<uint16_t>>(en, OG_ALGO_SSSP, src_, s);
     return run_frontier<EK<uint32_t>>(en, OG_ALGO_SSSP, src_, s);
@@ -2817,8 +2615,7 @@ extern "C" int og_cc(og_engine *e, uint32_t *out_label, og_stats *st) {
     if (en->frag && en->frag->broken)
       return fail(OG_E_STATE, "the fragment slots were not laid out (a failed OG_PARAM_FRAGMENT_WORDS change)");
     if (en->frag) return run_frontier<EKF<void>>(en, OG_ALGO_CC, 0, s);
-    if (en->level_loop == OG_LOOP_AUTO && (en->plan.dynamic_edges == 0 || (en->cfg.flags & OG_CFG_DIRECT)))
-      return run_min_dev(en, OG_ALGO_CC, 0, s);
+    if (rounds_on_device(en)) return run_rounds(en, OG_ALGO_CC, 0, s);
     return run_frontier<EKU>(en, OG_ALGO_CC, 0, s);
   }, &dummy);
 }

@@ -47,19 +47,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// Launch timer of the device-driven rounds: a one-thread kernel enqueued
-// right before (end = 0) and right after (end = 1) a gated launch, in the
-// same captured stream.  Stream order puts the first stamp before the launch
-// starts and the second after it ends; kt[0] holds the start, kt[1] the
-// accumulated ns.  Rounds whose gate is closed add nothing.
-__global__ void k_stamp(const uint32_t *go, unsigned long long *kt, int end) {
-  if (*go == 0u) return;
-  const unsigned long long t = globaltimer_ns();
-  if (end) kt[1] += t - kt[0];
-  else kt[0] = t;
-}
-
-
 struct Counts {
   uint32_t n;        // compacted vertices
   uint32_t far_min;  // near/far split: smallest value left for later rounds
@@ -108,17 +95,15 @@ struct CompactArgs {
   // the status array needs no clearing between launches.  The CTA that takes
   // the last ticket resets the ticket counter for the next launch.
   uint32_t epoch;
-  // Device-driven loops (launches replayed from a CUDA graph): when not null,
-  // the epoch is read from *epoch_ptr and the launch does nothing while
-  // *run_flag is 0.
-  const uint32_t *epoch_ptr;
-  const uint32_t *run_flag;
-  const uint32_t *thr_ptr;  // when not null, thr is read from *thr_ptr
 };
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
   return cuda::atomic_ref<const uint32_t, cuda::thread_scope_device>(*p).load(
       cuda::memory_order_acquire);
+}
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
+  return cuda::atomic_ref<const uint32_t, cuda::thread_scope_device>(*p).load(
+      cuda::memory_order_relaxed);
 }
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
   cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(*p).store(v, cuda::memory_order_release);
@@ -601,9 +586,6 @@ struct CompactSel {
 
 __global__ void __launch_bounds__(kThreads, 4) k_compact(CompactArgs a) {
   __shared__ CompactShared sh;
-  if (a.run_flag && *a.run_flag == 0u) return;  // every CTA of the launch reads the same flag
-  if (a.epoch_ptr) a.epoch = *a.epoch_ptr;
-  if (a.thr_ptr) a.thr = *a.thr_ptr;
   CompactSel sel{a, 0xffffffffu};
   compact_tile(a, sel, sh);
 }
@@ -1793,12 +1775,7 @@ template <class PS>
 __global__ void __launch_bounds__(kThreads) k_bfs_bottom_up(const uint64_t *off, uint32_t V, uint32_t Vs, PS stat,
                                                             PS host, const uint32_t *cur, uint32_t *visited,
                                                             uint32_t *next, uint32_t *depth, uint32_t newdepth,
-                                                            unsigned long long *cnt, uint32_t *err,
-                                                            const uint32_t *go = nullptr,
-                                                            const uint32_t *level = nullptr) {
-  // device-driven loops: run only when *go, at depth *level + 1
-  if (go && *go == 0u) return;
-  if (level) newdepth = *level + 1;
+                                                            unsigned long long *cnt, uint32_t *err) {
   const uint32_t lane = threadIdx.x & 31;
   unsigned long long nn = 0, nm = 0, nh = 0, ns = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
