@@ -427,6 +427,7 @@ __device__ __forceinline__ void bottom_up_scan(const PersistArgs &a, unsigned lo
                                                uint32_t *next_any) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t)gridDim.x * (BLOCK / 32);
+  const uint32_t cmask = a.ssrc.bc >= 32 ? 0xffffffffu : (1u << a.ssrc.bc) - 1u;
   unsigned long long ns = 0, nd = 0;  // static / dynamic records read
   // a vertex's visited mask and list bounds are fetched one word ahead, so
   // their latency overlaps the scan of the current word
@@ -454,27 +455,33 @@ __device__ __forceinline__ void bottom_up_scan(const PersistArgs &a, unsigned lo
       const unsigned long long need = ~vis & sel;
       if (need) {
         const uint64_t lim = min(e1, e0 + kBuLaneRecords);
-        for (uint64_t e = e0; e < lim && found != need; e += kBuStep) {
-          uint32_t u[kBuStep];
+        // a list lies in one region; its records come four to a load or two
+        const bool st = e0 < a.static_edges;
+        const SrcP<false> &src = st ? a.ssrc : a.hsrc;
+        if (e0 < lim && (lim > (st ? a.static_edges : a.E) || !src.words)) {
+          atomicOr(a.err, kErrEdgeIndex);
+        } else {
+          for (uint64_t e = e0; e < lim && found != need; e += kBuStep) {
+            uint32_t u[kBuStep];
+            const uint32_t left = (uint32_t)min((uint64_t)kBuStep, lim - e);
+            if (src.bpe <= 32) {  // uniform
 #pragma unroll
-          for (int j = 0; j < kBuStep; j++) {
-            const uint64_t i = e + j;
-            u[j] = 0xffffffffu;
-            if (i >= lim) continue;
-            if (i < a.static_edges) {
-              u[j] = a.ssrc.load(i);
-              ns++;
-            } else if (i < a.E && a.hsrc.words) {
-              u[j] = a.hsrc.load(i);
-              nd++;
+              for (int j = 0; j < kBuStep; j += 4)
+                records4(src.words, (e + j) * src.bpe, (int)left > j ? min(left - j, 4u) : 0u, src.bpe, cmask, u + j);
             } else {
-              atomicOr(a.err, kErrEdgeIndex);
-            }
-          }
 #pragma unroll
-          for (int j = 0; j < kBuStep; j++) {
-            if (u[j] < a.V) found |= __ldcg(cur + u[j]) & need;
-            else if (u[j] != 0xffffffffu) atomicOr(a.err, kErrVertex);
+              for (int j = 0; j < kBuStep; j++) u[j] = j < (int)left ? src.load(e + j) : 0u;
+            }
+            if (st) ns += left;
+            else nd += left;
+            unsigned long long m[kBuStep];
+#pragma unroll
+            for (int j = 0; j < kBuStep; j++) m[j] = j < (int)left && u[j] < a.V ? __ldcg(cur + u[j]) : 0ull;
+#pragma unroll
+            for (int j = 0; j < kBuStep; j++) {
+              found |= m[j] & need;
+              if (j < (int)left && u[j] >= a.V) atomicOr(a.err, kErrVertex);
+            }
           }
         }
         defer = found != need && lim < e1;

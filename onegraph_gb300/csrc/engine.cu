@@ -721,7 +721,7 @@ int create(og_graph *g, const og_config *cfg, og_engine *e) {
   // resident graph state shared with clones
   const uint64_t V = g->V;
   RC(dalloc(e, &e->off_d, V + 1));
-  if (P.static_edges) RC(dalloc(e, &e->spk_d, g->packed_words_for(P.static_edges)));
+  if (P.static_edges) RC(dalloc(e, &e->spk_d, g->packed_words_for(P.static_edges) + 4));  // records4
   if (e->pr_enabled) RC(dalloc(e, &e->outdeg_d, V + 1));
   e->resident_bytes = e->dbytes;
   if (e->frag) RC(frag_layout(e, frag_default_shift(g->packed_words)));

@@ -690,6 +690,50 @@ struct SrcP {
   }
 };
 
+// The columns of up to four consecutive records from bit `b` of the stream on
+// (bpe <= 32), for lanes that each read a list of their own: such reads cost
+// the L1 one tag lookup a lane and load, so the records come as one or two
+// aligned 16-byte loads instead of eight words, and are shifted out of a
+// 128-bit window.  `n` (0 to 4) records are wanted; the second load is made
+// only if they reach into it, and what lies beyond them is not used.  The
+// arrays are readable to a 16-byte boundary.  Measured: level 4 of a resident
+// 2^20-vertex R-MAT (1.8 M records) 16 -> 14 us, a 64-source batch over 2^23
+// vertices 12.9 -> 11.0 ms.
+__device__ __forceinline__ void records4(const uint32_t *words, uint64_t b, uint32_t n, uint32_t bpe, uint32_t mask,
+                                         uint32_t u[4]) {
+  const uint4 *q = reinterpret_cast<const uint4 *>(words) + (b >> 7);
+  const uint32_t r = (uint32_t)b & 127u;
+  uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+  if (n) lo = q[0];
+  if (r + n * bpe > 128u && n) hi = q[1];
+  // window of four words from word r / 32 on, then from bit r % 32 on
+  const bool s1 = r & 32u, s2 = r & 64u;
+  uint32_t w[6] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y}, x[5];
+  const uint32_t w6 = hi.z, w7 = hi.w;
+  if (s2) {
+    w[0] = w[2];
+    w[1] = w[3];
+    w[2] = w[4];
+    w[3] = w[5];
+    w[4] = w6;
+    w[5] = w7;
+  }
+#pragma unroll
+  for (int i = 0; i < 5; i++) x[i] = s1 ? w[i + 1] : w[i];
+  const uint32_t sh = r & 31u;
+#pragma unroll
+  for (int i = 0; i < 4; i++) x[i] = __funnelshift_r(x[i], x[i + 1], sh);
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    u[j] = x[0] & mask;
+    // shift the window by bpe (funnel shifts clamp at 32)
+    x[0] = __funnelshift_rc(x[0], x[1], bpe);
+    x[1] = __funnelshift_rc(x[1], x[2], bpe);
+    x[2] = __funnelshift_rc(x[2], x[3], bpe);
+    x[3] = __funnelshift_rc(x[3], 0u, bpe);
+  }
+}
+
 // Dynamic-region records with fragment slots (the static-region replacement
 // the reference declares as bfs_kernelStaticSwap / recordFragmentVisit,
 // BFS/oneGraph_BFS/gpu_kernels.h:46-66,153-176): the page-locked record
@@ -840,9 +884,13 @@ struct HasProbeVal<T, std::void_t<decltype(T::kProbeVal)>> : std::true_type {};
 // reads src.at(cb[map[x]], x).  Every local vertex's edge indices in the tile
 // are checked against edge_bound here, once per vertex; a tile with one out
 // of bounds sets kErrEdgeIndex and relaxes nothing.
-template <bool kNeedVal, class Src, class Op, class Sh>
+//
+// kPart: only positions [lo, hi) of the tile are read, and only the vertices
+// that have some are looked up.
+template <bool kNeedVal, bool kPart = false, class Src, class Op, class Sh>
 __device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, const Op &op, Sh &sh,
-                                              uint64_t k, uint64_t pos0, uint32_t &i0_out) {
+                                              uint64_t k, uint64_t pos0, uint32_t &i0_out, uint32_t lo = 0,
+                                              uint32_t hi = kTile) {
   __shared__ uint32_t s_bad;
   const uint64_t ntiles_total = (a.total + kTile - 1) / kTile;
   const uint32_t i0 = a.tile_first[k];
@@ -867,6 +915,10 @@ __device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, 
     const uint64_t p = a.pref[i], pn = a.pref[i + 1];
     const uint32_t r = p > pos0 ? (uint32_t)min(p - pos0, (uint64_t)kTile) : 0u;
     sh.rs[j] = r;
+    // head flag.  Compacted lists hold no zero-degree vertex, so for j >= 1
+    // the starts are distinct and strictly increasing (rs[0] = 0).
+    if (j >= 1 && r < kTile) sh.map[r] = (unsigned short)1;
+    if (kPart && (r >= hi || pn <= pos0 + lo)) continue;
     const uint64_t e0 = (a.off ? a.off[v] - p : (0ull - a.stage_base)) + pos0;  // edge index of position 0
     if constexpr (HasCurRange<Src>::value) {
       uint64_t cb = src.cur(e0);
@@ -891,9 +943,6 @@ __device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, 
     }
     if constexpr (HasListVal<Op>::value) sh.val[j] = op.list_val(v, a.list + i);
     else if constexpr (kNeedVal) sh.val[j] = op.src_val(v);
-    // head flag.  Compacted lists hold no zero-degree vertex, so for j >= 1
-    // the starts are distinct and strictly increasing (rs[0] = 0).
-    if (j >= 1 && r < kTile) sh.map[r] = (unsigned short)1;
   }
   if (bad) {
     s_bad = 1;
@@ -926,23 +975,27 @@ __device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, 
 template <class Op>
 using LbsSh = LbsShared<typename Op::Val, Op::kNeedVal || HasListVal<Op>::value>;
 
-// One LBS tile (kTile positions starting at tile k of the list) of a CTA.
-template <class Src, class Op>
+// One LBS tile (kTile positions starting at tile k of the list) of a CTA; with
+// kPart, part `part` of `parts` (1, 2, 4 or 8) equal ones.
+template <bool kPart = false, class Src, class Op>
 __device__ __forceinline__ void lbs_tile(const LbsArgs &a, const Src &src, const Op &op, LbsSh<Op> &sh,
-                                         uint64_t k) {
+                                         uint64_t k, uint32_t part = 0, uint32_t parts = 1) {
   const uint64_t pos0 = k * kTile;
   if (pos0 >= a.pos_end) return;
-  const uint32_t tlen = (uint32_t)(min(pos0 + kTile, a.pos_end) - pos0);
+  const uint32_t lo = kPart ? part * (kTile / parts) : 0u;
+  const uint32_t tlen = min((uint32_t)min((uint64_t)kTile, a.pos_end - pos0), kPart ? lo + kTile / parts : kTile);
+  if (kPart && lo >= tlen) return;  // uniform
   uint32_t i0;
-  const uint32_t nl = lbs_setup<Op::kNeedVal>(a, src, op, sh, k, pos0, i0);
+  const uint32_t nl = lbs_setup<Op::kNeedVal, kPart>(a, src, op, sh, k, pos0, i0, lo, tlen);
   if (nl == 0) return;
   // All eight loads are issued before the first relax, so each thread keeps
   // eight edge reads in flight (the host-link gather is latency bound).
+  const uint32_t x0 = lo + threadIdx.x;
   typename Src::Item ev[kItems];
   uint32_t lv[kItems];
 #pragma unroll
   for (int it = 0; it < (int)kItems; it++) {
-    const uint32_t x = it * kThreads + threadIdx.x;
+    const uint32_t x = it * kThreads + x0;
     lv[it] = 0;
     if (x < tlen) {
       const uint32_t l = sh.map[x];
@@ -958,15 +1011,15 @@ __device__ __forceinline__ void lbs_tile(const LbsArgs &a, const Src &src, const
   typename Op::Probe pr[kItems];
 #pragma unroll
   for (int it = 0; it < (int)kItems; it++)
-    if (it * kThreads + threadIdx.x < tlen) {
+    if (it * kThreads + x0 < tlen) {
       if constexpr (HasProbeVal<Op>::value) pr[it] = op.probe_v(ev[it], sh.val[lv[it]]);
       else pr[it] = op.probe(ev[it]);
     }
 #pragma unroll
   for (int it = 0; it < (int)kItems; it++) {
-    if (it * kThreads + threadIdx.x < tlen)
+    if (it * kThreads + x0 < tlen)
       op.relax(ev[it], Op::kNeedVal ? sh.val[lv[it]] : typename Op::Val{},
-               pos0 + it * kThreads + threadIdx.x, pr[it]);
+               pos0 + it * kThreads + x0, pr[it]);
   }
 }
 
@@ -1771,66 +1824,130 @@ __global__ void k_depth_expand(const uint8_t *b, uint64_t n, uint32_t unreached,
 // (one bitmap word), so each word of next / visited has a single writer.
 // cnt[0] += vertices reached, cnt[1] += their degrees, cnt[2] += records read
 // from the host copy, cnt[3] += records read from the static region.
+//
+// Large levels are bound by the L1's tag lookups (every lane reads a list of its
+// own), small ones by the chain visited word -> offsets -> records -> frontier
+// words.  So records come through records4, frontier words two at a time, the
+// next word's visited bits are fetched ahead, and the last two unfinished
+// vertices of a word are scanned by the whole warp, 32 records a step (a lane
+// alone on a list of 40 records kept a level waiting for 10 us).  The counts of
+// records read are those of four-record steps in either form.
 template <class PS>
-__global__ void __launch_bounds__(kThreads) k_bfs_bottom_up(const uint64_t *off, uint32_t V, uint32_t Vs, PS stat,
-                                                            PS host, const uint32_t *cur, uint32_t *visited,
-                                                            uint32_t *next, uint32_t *depth, uint32_t newdepth,
-                                                            unsigned long long *cnt, uint32_t *err) {
+__device__ __forceinline__ void bottom_up_words(const uint64_t *off, uint32_t V, uint32_t Vs, const PS &stat,
+                                                const PS &host, const uint32_t *cur, uint32_t *visited,
+                                                uint32_t *next, uint32_t *depth, uint32_t newdepth,
+                                                unsigned long long *cnt, uint32_t *err) {
+  __shared__ unsigned long long s_cnt[4];
+  if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
   const uint32_t lane = threadIdx.x & 31;
-  unsigned long long nn = 0, nm = 0, nh = 0, ns = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < V; base += stride) {
-    const uint64_t v = base + lane;
-    const uint32_t w = (uint32_t)(base >> 5);
-    const uint32_t vis = __ldcg(visited + w);
-    bool found = false;
-    uint64_t d = 0;
+  uint32_t nn = 0;
+  unsigned long long nm = 0, nh = 0, ns = 0;
+  const uint64_t words = ((uint64_t)V + 31) / 32, nw = (uint64_t)gridDim.x * (kThreads / 32);
+  // consecutive words go to different CTAs
+  uint64_t w = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  uint32_t vis_next = w < words ? visited[w] : 0u;
+  const uint32_t cmask = stat.bc >= 32 ? 0xffffffffu : (1u << stat.bc) - 1u;
+  for (; w < words; w += nw) {
+    const uint32_t vis = vis_next;
+    if (w + nw < words) vis_next = visited[w + nw];
+    const uint64_t v = w * 32 + lane;
+    const bool st = v < Vs;
+    uint64_t e = 0, e1 = 0;  // this lane's unread records
     if (v < V && !((vis >> lane) & 1u)) {
-      const uint64_t o = off[v], e1 = off[v + 1];
-      d = e1 - o;
-      const bool st = v < Vs;
-      const PS &src = st ? stat : host;
-      for (uint64_t e = o; e < e1 && !found; e += 4) {
+      e = off[v];
+      e1 = off[v + 1];
+    }
+    const uint64_t deg = e1 - e;
+    bool found = false;
+    for (uint32_t open = __ballot_sync(0xffffffffu, e < e1); open; open = __ballot_sync(0xffffffffu, e < e1)) {
+      if (__popc(open) > 2) {
+        const uint32_t left = (uint32_t)min((uint64_t)4, e1 - e);
         uint32_t u[4];
+        const uint32_t *base = st ? stat.words : host.words;
+        if (stat.bpe <= 32) {  // uniform
+          records4(base, e * stat.bpe, left, stat.bpe, cmask, u);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 4; j++) u[j] = e + j < e1 ? src.load(e + j) : 0xffffffffu;
-        const uint64_t got = (e1 - e < 4) ? e1 - e : 4;
-        if (st) ns += got;
-        else nh += got;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (u[j] < V) {
-            if ((__ldcg(cur + (u[j] >> 5)) >> (u[j] & 31)) & 1u) found = true;
-          } else if (u[j] != 0xffffffffu) {
-            atomicOr(err, kErrVertex);
+          for (uint32_t j = 0; j < 4; j++) {
+            const uint64_t b = (e + j) * stat.bpe;
+            u[j] = j < left ? stat.decode(base + (b >> 5), (uint32_t)b & 31u) : 0u;
           }
+        }
+        // two frontier words at a time: most vertices of a large level are
+        // found by their first records
+        bool hit = false;
+#pragma unroll
+        for (uint32_t h = 0; h < 4; h += 2) {
+          uint32_t f[2] = {0u, 0u};
+#pragma unroll
+          for (uint32_t j = 0; j < 2; j++)
+            if (h + j < left && !hit) {
+              if (u[h + j] < V) f[j] = (cur[u[h + j] >> 5] >> (u[h + j] & 31)) & 1u;
+              else atomicOr(err, kErrVertex);
+            }
+          hit |= (f[0] | f[1]) != 0u;
+        }
+        if (st) ns += left;
+        else nh += left;
+        found |= hit;
+        e = hit ? e1 : e + left;
+      } else {
+        const int l = __ffs(open) - 1;
+        const uint64_t eb = __shfl_sync(0xffffffffu, e, l), ee = __shfl_sync(0xffffffffu, e1, l);
+        const uint32_t left = (uint32_t)min((uint64_t)32, ee - eb);
+        bool hit = false;
+        if (lane < left) {
+          const uint64_t b = (eb + lane) * stat.bpe;
+          const uint32_t u =
+              stat.decode((w * 32 + l < Vs ? stat.words : host.words) + (b >> 5), (uint32_t)b & 31u);
+          if (u < V) hit = (cur[u >> 5] >> (u & 31)) & 1u;
+          else atomicOr(err, kErrVertex);
+        }
+        const uint32_t hb = __ballot_sync(0xffffffffu, hit);
+        if ((int)lane == l) {
+          const uint32_t got = hb ? min(left, ((uint32_t)(__ffs(hb) - 1) / 4 + 1) * 4) : left;
+          if (st) ns += got;
+          else nh += got;
+          found |= hb != 0u;
+          e = hb ? e1 : e + left;
         }
       }
     }
     const uint32_t ball = __ballot_sync(0xffffffffu, found);
-    if (lane == 0 && ball) {
+    if (lane == 0) {
       next[w] = ball;
-      visited[w] = vis | ball;
+      if (ball) visited[w] = vis | ball;
     }
     if (found) {
       depth[v] = newdepth;
       nn++;
-      nm += d;
+      nm += deg;
     }
   }
-  nn = __reduce_add_sync(0xffffffffu, (uint32_t)nn);
+  nn = __reduce_add_sync(0xffffffffu, nn);
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     nm += __shfl_xor_sync(0xffffffffu, nm, o);
     nh += __shfl_xor_sync(0xffffffffu, nh, o);
     ns += __shfl_xor_sync(0xffffffffu, ns, o);
   }
-  if (lane == 0) {
-    if (nn) atomicAdd(cnt, nn);
-    if (nm) atomicAdd(cnt + 1, nm);
-    if (nh) atomicAdd(cnt + 2, nh);
-    if (ns) atomicAdd(cnt + 3, ns);
+  if (lane == 0) {  // one global atomic per CTA and counter
+    if (nn) atomicAdd(&s_cnt[0], (unsigned long long)nn);
+    if (nm) atomicAdd(&s_cnt[1], nm);
+    if (nh) atomicAdd(&s_cnt[2], nh);
+    if (ns) atomicAdd(&s_cnt[3], ns);
   }
+  __syncthreads();
+  if (threadIdx.x < 4 && s_cnt[threadIdx.x]) atomicAdd(cnt + threadIdx.x, s_cnt[threadIdx.x]);
+}
+
+template <class PS>
+__global__ void __launch_bounds__(kThreads) k_bfs_bottom_up(const uint64_t *off, uint32_t V, uint32_t Vs, PS stat,
+                                                            PS host, const uint32_t *cur, uint32_t *visited,
+                                                            uint32_t *next, uint32_t *depth, uint32_t newdepth,
+                                                            unsigned long long *cnt, uint32_t *err) {
+  bottom_up_words(off, V, Vs, stat, host, cur, visited, next, depth, newdepth, cnt, err);
 }
 
 // ------------------------------------------------------------ union-find CC
