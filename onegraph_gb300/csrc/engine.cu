@@ -2513,7 +2513,7 @@ extern "C" int og_sssp(og_engine *e, uint32_t src, uint32_t *out_dist, og_stats 
 // ------------------------------------------------------------ union-find CC
 //
 // Symmetric graphs only (the result equals label propagation's there): two
-// sampling passes over every vertex's first two edges, compression, the giant
+// sampling passes over every vertex's first two edges (read once), compression, the giant
 // component picked from 1024 sampled roots, then one edge-balanced pass over
 // the edges of the vertices outside it (both regions, interleaved), and a
 // final compression.  parent[] lives in value_d and ends as the labels.
@@ -2527,17 +2527,16 @@ int run_cc_uf(og_engine *e, og_stats &st) {
   constexpr uint32_t kRoots = 1024;
   CK(cudaMemsetAsync(e->err_d, 0, 16, s));
   CK(cudaMemsetAsync(reads, 0, 16, s));
-  k_iota_u32<<<g, kThreads, 0, s>>>(par, V);
-  e->launches++;
   cudaEvent_t t0 = e->t_d0, t1 = e->ev_dyn_done;
   CK(cudaEventRecord(t0, s));
-  for (uint32_t r = 0; r < 2; r++) {
-    k_uf_sample<EKU::PSrc><<<g, kThreads, 0, s>>>(e->off_d, V, e->plan.static_edges, EKU::stat(e),
-                                                  EKU::host(e), r, par, reads, e->err_d);
-    k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
-    e->launches += 2;
-    st.iterations++;
-  }
+  uint2 *pend = (uint2 *)e->pref_d[0];  // V + 2 entries of 8 bytes, not in use before the compaction
+  k_uf_init<EKU::PSrc><<<g, kThreads, 0, s>>>(e->off_d, V, e->plan.static_edges, EKU::stat(e), EKU::host(e), par, pend,
+                                              reads, e->err_d);
+  k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
+  k_uf_link<<<g, kThreads, 0, s>>>(pend, V, par, e->err_d);
+  k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
+  e->launches += 4;
+  st.iterations += 2;
   k_uf_roots<<<(kRoots + kThreads - 1) / kThreads, kThreads, 0, s>>>(par, V, kRoots, roots_d);
   e->launches++;
   CK(cudaEventRecord(t1, s));
@@ -2594,7 +2593,11 @@ int run_cc_uf(og_engine *e, og_stats &st) {
     RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
     CK(cudaStreamWaitEvent(e->s_main, e->ev_cd, 0));
   }
-  k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
+  if (n) {  // nothing was linked since the last compression otherwise
+    k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
+    e->launches++;
+  }
+  k_uf_flatten<<<g, kThreads, 0, s>>>(par, V, e->err_d);
   e->launches++;
   CK(cudaStreamSynchronize(s));
   collect_timing(e, tm, &st);

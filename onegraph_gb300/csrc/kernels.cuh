@@ -1962,15 +1962,21 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bottom_up(const uint64_t *off,
 // Walks follow strictly decreasing ids, so they end within V steps; a broken
 // invariant sets kErrVertex instead of looping.
 
+// Parents are read through L1.  The giant component's root is read by every
+// walk, and from the L2 those reads of one line run one after another (linking
+// 8.4 M vertices: 0.95 ms so, 0.27 ms through L1; a compression 125 and 33 us);
+// a stale
+// parent is an older ancestor, so a walk only ends too early, at a vertex that
+// is no root any more, and the compare-and-swap on it returns the newer one.
 __device__ __forceinline__ uint32_t uf_find(uint32_t *par, uint32_t x, uint32_t V, uint32_t *err) {
   for (uint32_t steps = 0; steps <= V; steps++) {
-    const uint32_t p = __ldcg(par + x);
+    const uint32_t p = __ldca(par + x);
     if (p == x) return x;
     if (p > x) {
       atomicOr(err, kErrVertex);
       return x;
     }
-    const uint32_t gp = __ldcg(par + p);
+    const uint32_t gp = __ldca(par + p);
     if (gp < p) __stcg(par + x, gp);  // path halving: gp is an ancestor of x
     x = gp;
   }
@@ -1980,40 +1986,62 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *par, uint32_t x, uint32_t 
 
 __device__ __forceinline__ void uf_link(uint32_t *par, uint32_t a, uint32_t b, uint32_t V, uint32_t *err) {
   for (uint32_t tries = 0; tries <= V; tries++) {
-    const uint32_t ra = uf_find(par, a, V, err), rb = uf_find(par, b, V, err);
-    if (ra == rb) return;
-    const uint32_t hi = max(ra, rb), lo = min(ra, rb);
-    if (atomicCAS(par + hi, hi, lo) == hi) return;
-    a = ra;  // hi gained a parent meanwhile: retry from the two roots
-    b = rb;
+    a = uf_find(par, a, V, err);
+    b = uf_find(par, b, V, err);
+    if (a == b) return;
+    const uint32_t hi = max(a, b), lo = min(a, b);
+    const uint32_t old = atomicCAS(par + hi, hi, lo);
+    if (old == hi) return;
+    a = old;  // hi had a parent already: go on from it
+    b = lo;
   }
   atomicOr(err, kErrVertex);
 }
 
-// Sampling pass r: link every vertex of degree > r with its r-th neighbour
-// (edge off[v] + r, from the static region or from the host copy).
+// First sampling pass: reads every vertex's first two records (one or two
+// 16-byte loads, where the passes used to fetch the same link sector twice) and
+// hooks v under its first neighbour when that is smaller: parents are smaller
+// than their vertices from the start, so a plain store does it, where linking
+// all first edges by compare-and-swap spent 0.8 ms of retries on 2^23
+// vertices.  What is left of the two edges (a larger first neighbour, the
+// second one) goes to pend for k_uf_link.
 template <class PS>
-__global__ void __launch_bounds__(kThreads) k_uf_sample(const uint64_t *off, uint32_t V, uint64_t static_edges,
-                                                        PS stat, PS host, uint32_t r, uint32_t *par,
-                                                        unsigned long long *reads, uint32_t *err) {
+__global__ void __launch_bounds__(kThreads) k_uf_init(const uint64_t *off, uint32_t V, uint64_t static_edges, PS stat,
+                                                      PS host, uint32_t *par, uint2 *pend, unsigned long long *reads,
+                                                      uint32_t *err) {
+  const uint32_t cmask = stat.bc >= 32 ? 0xffffffffu : (1u << stat.bc) - 1u;
   uint32_t nh = 0, ns = 0;  // records read from the host copy / the static region
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t o = off[v];
-    if (off[v + 1] - o <= r) continue;
-    const uint64_t idx = o + r;
-    uint32_t u;
-    if (idx < static_edges) {
-      u = stat.load(idx);
-      ns++;
-    } else {
-      u = host.load(idx);
-      nh++;
+    const uint32_t n = (uint32_t)min((uint64_t)2, off[v + 1] - o);
+    const bool st = o < static_edges;
+    const uint32_t *base = st ? stat.words : host.words;
+    uint32_t u[4] = {0u, 0u, 0u, 0u};
+    if (n) {
+      if (stat.bpe <= 32) {  // uniform
+        records4(base, o * stat.bpe, n, stat.bpe, cmask, u);
+      } else {
+        for (uint32_t j = 0; j < n; j++) {
+          const uint64_t b = (o + j) * stat.bpe;
+          u[j] = stat.decode(base + (b >> 5), (uint32_t)b & 31u);
+        }
+      }
     }
-    if (u >= V) {
+    if (st) ns += n;
+    else nh += n;
+    uint32_t p = (uint32_t)v;
+    uint2 rest = make_uint2(0xffffffffu, 0xffffffffu);
+    if ((n > 0 && u[0] >= V) || (n > 1 && u[1] >= V)) {
       atomicOr(err, kErrVertex);
-      continue;
+    } else {
+      if (n > 0) {
+        if (u[0] < p) p = u[0];
+        else rest.x = u[0];
+      }
+      if (n > 1) rest.y = u[1];
     }
-    uf_link(par, (uint32_t)v, u, V, err);
+    par[v] = p;
+    pend[v] = rest;
   }
   nh = __reduce_add_sync(0xffffffffu, nh);
   ns = __reduce_add_sync(0xffffffffu, ns);
@@ -2023,10 +2051,74 @@ __global__ void __launch_bounds__(kThreads) k_uf_sample(const uint64_t *off, uin
   }
 }
 
-// parent[v] = root of v for every vertex.
+// The sampled edges that k_uf_init left over.  On a graph with a giant component
+// most of them join the same few roots at the same time, and compare-and-swaps
+// on one address run one after another in the L2: the lanes of a warp that want
+// to hook the same root send one (8.4 M vertices: 1.1 ms with a swap per lane).
+__global__ void __launch_bounds__(kThreads) k_uf_link(const uint2 *pend, uint32_t V, uint32_t *par, uint32_t *err) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < V; base += stride) {
+    const uint64_t v = base + lane;
+    const uint2 r = v < V ? pend[v] : make_uint2(0xffffffffu, 0xffffffffu);
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+      uint32_t x = (uint32_t)v, y = k ? r.y : r.x;
+      bool todo = y != 0xffffffffu;
+      for (uint32_t tries = 0; __any_sync(0xffffffffu, todo); tries++) {
+        if (tries > V) {  // a broken forest: report, never hang
+          if (todo) atomicOr(err, kErrVertex);
+          break;
+        }
+        if (todo) {
+          x = uf_find(par, x, V, err);
+          y = uf_find(par, y, V, err);
+          todo = x != y;
+        }
+        __syncwarp();
+        const uint32_t hi = max(x, y), lo = min(x, y);
+        const uint32_t same = __match_any_sync(0xffffffffu, todo ? hi : 0xffffffffu);
+        uint32_t old = hi;
+        const int first = __ffs(same) - 1;
+        const bool mine = todo && (int)lane == first;
+        if (mine) old = atomicCAS(par + hi, hi, lo);
+        if (mine && old == hi) todo = false;
+        old = __shfl_sync(0xffffffffu, mine && old == hi ? lo : old, first);  // hi's parent now
+        if (todo) {
+          x = old;
+          y = lo;
+        }
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// parent[v] = root of v for every vertex, up to the walks that halve a path
+// through v at the same moment: such a walk may put an ancestor it read
+// earlier back after v's own store.  Long chains become short ones.
 __global__ void __launch_bounds__(kThreads) k_uf_compress(uint32_t *par, uint32_t V, uint32_t *err) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
     __stcg(par + v, uf_find(par, (uint32_t)v, V, err));
+}
+
+// The labels, after k_uf_compress: walks that store nothing but their own
+// vertex's root, so every vertex ends with it.
+__global__ void __launch_bounds__(kThreads) k_uf_flatten(uint32_t *par, uint32_t V, uint32_t *err) {
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t p0 = __ldca(par + v);
+    uint32_t x = p0;
+    for (uint32_t steps = 0;; steps++) {
+      const uint32_t p = __ldca(par + x);
+      if (p == x) break;
+      if (p > x || steps > V) {
+        atomicOr(err, kErrVertex);
+        break;
+      }
+      x = p;
+    }
+    if (x != p0) __stcg(par + v, x);
+  }
 }
 
 // Roots of k pseudo-random vertices (after compression), for the host to
@@ -2042,17 +2134,17 @@ __global__ void k_uf_roots(const uint32_t *par, uint32_t V, uint32_t k, uint32_t
 }
 
 // Frontier of the final pass: vertices of degree > 2 (their first two edges
-// are already linked) outside component c.  One thread per bitmap word.
+// are already linked) outside component c.  A lane per vertex, a warp per
+// bitmap word.
 __global__ void __launch_bounds__(kThreads) k_uf_mark(const uint64_t *off, const uint32_t *par, uint32_t V,
                                                       uint32_t c, uint32_t *bits, uint64_t nwords) {
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t word = 0;
-    for (uint32_t b = 0; b < 32; b++) {
-      const uint64_t v = w * 32 + b;
-      if (v >= V) break;
-      if (off[v + 1] - off[v] > 2 && __ldcg(par + v) != c) word |= 1u << b;
-    }
-    bits[w] = word;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nw = (uint64_t)gridDim.x * (kThreads / 32);
+  for (uint64_t w = (blockIdx.x * (uint64_t)kThreads + threadIdx.x) >> 5; w < nwords; w += nw) {
+    const uint64_t v = w * 32 + lane;
+    const bool on = v < V && par[v] != c && off[v + 1] - off[v] > 2;
+    const uint32_t word = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) bits[w] = word;
   }
 }
 
