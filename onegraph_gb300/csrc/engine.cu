@@ -114,7 +114,9 @@ struct og_engine {
   // PageRank state
   float *contrib_d = nullptr, *sum_d = nullptr, *cont_d = nullptr, *carry_d = nullptr;
   uint32_t *outdeg_d = nullptr, *carry_idx_d = nullptr;
-  double *part_d = nullptr, *l1_d = nullptr, *l1_h = nullptr;
+  double *part_d = nullptr;
+  PrLoop *prl_d = nullptr, *prl_h = nullptr;  // L1 iterations: state and its page-locked mirror
+  uint32_t pr_hint = 8;  // iterations the last run took (launched before its first check)
   uint32_t part_n = 0;
   uint64_t pr_tiles = 0;
 
@@ -484,7 +486,7 @@ void destroy(og_engine *e) {
   if (e->graph) cudaGraphExecDestroy(e->graph);
   if (e->rounds_h) cudaFreeHost(e->rounds_h);
   if (e->err_h) cudaFreeHost(e->err_h);
-  if (e->l1_h) cudaFreeHost(e->l1_h);
+  if (e->prl_h) cudaFreeHost(e->prl_h);
   cudaEvent_t evs[] = {e->ev_round, e->ev_cs, e->ev_cd, e->ev_dyn_done, e->ev_gat[0], e->ev_gat[1],
                        e->ev_rel[0], e->ev_rel[1], e->t_s0, e->t_s1, e->t_d0};
   for (auto ev : evs)
@@ -558,7 +560,7 @@ int create_query_state(og_engine *e) {
   RC(dalloc(e, (char **)&e->rounds_d, sizeof(RoundsState)));
   CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState)));
   CK(cudaMallocHost(&e->err_h, 4 * sizeof(uint32_t)));
-  CK(cudaMallocHost(&e->l1_h, sizeof(double)));
+  CK(cudaMallocHost(&e->prl_h, sizeof(PrLoop)));
   if (P.chunk_edges && !(e->cfg.flags & OG_CFG_DIRECT)) {
     for (int b = 0; b < 2; b++) {
       RC(dalloc(e, &e->stage_col[b], P.chunk_edges));
@@ -579,7 +581,7 @@ int create_query_state(og_engine *e) {
     RC(dalloc(e, &e->carry_idx_d, e->pr_tiles));
     e->part_n = (uint32_t)e->sms * 8;
     RC(dalloc(e, &e->part_d, e->part_n));
-    RC(dalloc(e, &e->l1_d, 1));
+    RC(dalloc(e, &e->prl_d, 1));
   }
   if (arena) {
     // one arena for the batched BFS masks (24 B per vertex), the
@@ -2087,60 +2089,43 @@ int launch_pr_pull(og_engine *e, const LbsArgs &a, SrcP<false> src, const PrArgs
   return OG_OK;
 }
 
-int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
-  PrArgs p{};
-  p.contrib = e->contrib_d;
-  p.sum = e->sum_d;
-  p.V = e->V;
-  // static tiles use [0, tile_cap0), dynamic tiles [tile_cap0, ...)
-  const uint64_t toff[2] = {0, e->tile_cap[0]};
-  CK(cudaEventRecord(e->ev_round, e->s_main));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-  CK(cudaStreamWaitEvent(e->s_gat, e->ev_round, 0));
-  auto args_for = [&](int r) {
-    PrArgs q = p;
-    q.cont = e->cont_d + toff[r];
-    q.carry = e->carry_d + toff[r];
-    q.carry_idx = e->carry_idx_d + toff[r];
-    q.base = r ? e->plan.static_edges : 0;
-    q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
-    return q;
-  };
-  auto sfn = [&](const LbsArgs &a) {
-    return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), args_for(0), e->s_main)
-                               : launch_pr_pull<false>(e, a, EKU::stat(e), args_for(0), e->s_main);
-  };
-  auto dfn = [&](const LbsArgs &a, auto src, cudaStream_t ds) {
-    if constexpr (std::is_same<decltype(src), SrcU>::value) {
-      // a staging buffer: columns from position pos_begin on, as 32-bit records
-      PrArgs q = args_for(1);
-      q.base = 0ull - a.pos_begin;
-      q.nwords = a.edge_bound;
-      return launch_pr_pull<true>(e, a, SrcP<false>{src.col, 32u, 32u, 0u}, q, ds);
-    } else {
-      return pr_contiguous(e, 1) ? launch_pr_pull<true>(e, a, src, args_for(1), ds)
-                                 : launch_pr_pull<false>(e, a, src, args_for(1), ds);
-    }
-  };
-  auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
-    const uint64_t n0 = lbs_grid(a0.pos_begin, a0.pos_end), n1 = lbs_grid(a1.pos_begin, a1.pos_end);
-    if (n0 + n1 > 0x7fffffffull) return fail(OG_E_STATE, "pull grid too large");
-    const unsigned n = (unsigned)(n0 + n1);
-    if (pr_contiguous(e, 0) && pr_contiguous(e, 1))
-      k_pr_pull_pair<true><<<n, kThreads, pr_smem_bytes(true, e->bpe), ps>>>(a0, s0, args_for(0), a1, s1, args_for(1),
-                                                                             n0, n);
-    else
-      k_pr_pull_pair<false><<<n, kThreads, pr_smem_bytes(false, e->bpe), ps>>>(a0, s0, args_for(0), a1, s1,
-                                                                               args_for(1), n0, n);
-    e->launches++;
-    return (int)OG_OK;
-  };
-  RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn)));
+// Arguments of region r's pull; done: see PrArgs.
+PrArgs pr_args(const og_engine *e, int r, const uint32_t *done) {
+  PrArgs q{};
+  const uint64_t toff = r ? e->tile_cap[0] : 0;  // the dynamic region's tiles follow the static ones
+  q.contrib = e->contrib_d;
+  q.sum = e->sum_d;
+  q.V = e->V;
+  q.cont = e->cont_d + toff;
+  q.carry = e->carry_d + toff;
+  q.carry_idx = e->carry_idx_d + toff;
+  q.base = r ? e->plan.static_edges : 0;
+  q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
+  q.done = done;
+  return q;
+}
+
+int launch_pr_pull_pair(og_engine *e, const LbsArgs &a0, SrcP<false> s0, const LbsArgs &a1, SrcP<false> s1,
+                        const uint32_t *done, cudaStream_t ps) {
+  const uint64_t n0 = lbs_grid(a0.pos_begin, a0.pos_end), n1 = lbs_grid(a1.pos_begin, a1.pos_end);
+  if (n0 + n1 > 0x7fffffffull) return fail(OG_E_STATE, "pull grid too large");
+  const unsigned n = (unsigned)(n0 + n1);
+  if (pr_contiguous(e, 0) && pr_contiguous(e, 1))
+    k_pr_pull_pair<true><<<n, kThreads, pr_smem_bytes(true, e->bpe), ps>>>(a0, s0, pr_args(e, 0, done), a1, s1,
+                                                                           pr_args(e, 1, done), n0, n);
+  else
+    k_pr_pull_pair<false><<<n, kThreads, pr_smem_bytes(false, e->bpe), ps>>>(a0, s0, pr_args(e, 0, done), a1, s1,
+                                                                             pr_args(e, 1, done), n0, n);
+  e->launches++;
+  return OG_OK;
+}
+
+int launch_pr_fixup(og_engine *e, const uint32_t *done) {
   PrFixup f[2];
   uint64_t nt[2];
   for (int r = 0; r < 2; r++) {
     const Counts c = e->counts_h[r];
-    f[r] = PrFixup{e->list_d[r], e->pref_d[r], c.n, args_for(r)};
+    f[r] = PrFixup{e->list_d[r], e->pref_d[r], c.n, pr_args(e, r, done)};
     nt[r] = c.n ? (c.total + kTile - 1) / kTile : 0;
   }
   if (nt[0] + nt[1]) {
@@ -2150,6 +2135,33 @@ int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
   }
   CK(cudaGetLastError());
   return OG_OK;
+}
+
+int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
+  CK(cudaEventRecord(e->ev_round, e->s_main));
+  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
+  CK(cudaStreamWaitEvent(e->s_gat, e->ev_round, 0));
+  auto sfn = [&](const LbsArgs &a) {
+    return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main)
+                               : launch_pr_pull<false>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main);
+  };
+  auto dfn = [&](const LbsArgs &a, auto src, cudaStream_t ds) {
+    if constexpr (std::is_same<decltype(src), SrcU>::value) {
+      // a staging buffer: columns from position pos_begin on, as 32-bit records
+      PrArgs q = pr_args(e, 1, nullptr);
+      q.base = 0ull - a.pos_begin;
+      q.nwords = a.edge_bound;
+      return launch_pr_pull<true>(e, a, SrcP<false>{src.col, 32u, 32u, 0u}, q, ds);
+    } else {
+      return pr_contiguous(e, 1) ? launch_pr_pull<true>(e, a, src, pr_args(e, 1, nullptr), ds)
+                                 : launch_pr_pull<false>(e, a, src, pr_args(e, 1, nullptr), ds);
+    }
+  };
+  auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
+    return launch_pr_pull_pair(e, a0, s0, a1, s1, nullptr, ps);
+  };
+  RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn)));
+  return launch_pr_fixup(e, nullptr);
 }
 
 int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
@@ -2188,12 +2200,34 @@ int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
   return OG_OK;
 }
 
+// The update of every rank and the end of the iteration (k_pr_finish).
+int launch_pr_update(og_engine *e, float teleport, float damping, double tol, const uint32_t *done) {
+  k_pr_update_l1<<<e->part_n, kThreads, 0, e->s_main>>>(e->V, (float *)e->value_d, e->contrib_d, e->sum_d,
+                                                        e->outdeg_d, teleport, damping, e->part_d, done);
+  k_pr_finish<<<1, kThreads, 0, e->s_main>>>(e->part_d, e->part_n, e->prl_d, tol);
+  e->launches += 2;
+  return OG_OK;
+}
+
+// Reads the iterations' state back and waits.
+int pr_check(og_engine *e, og_stats &st) {
+  cudaStream_t s = e->s_main;
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(e->prl_h, e->prl_d, sizeof(PrLoop), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  RC(check_device_error(e));
+  st.residual = e->prl_h->residual;
+  return OG_OK;
+}
+
 int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &st) {
   const uint64_t V = e->V;
   uint32_t *cur = e->bm[0];
   cudaStream_t s = e->s_main;
   const int g = grid_for(V, e->sms);
   CK(cudaMemsetAsync(e->err_d, 0, 16, s));
+  CK(cudaMemsetAsync(e->prl_d, 0, sizeof(PrLoop), s));
   k_pr_init<<<g, kThreads, 0, s>>>(V, (float *)e->value_d, e->contrib_d, e->sum_d, e->outdeg_d,
                                    (float)(1.0 / (double)V));
   e->launches++;
@@ -2204,23 +2238,63 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
   uint64_t n = 0;
   RC(compact_round(e, cur, st, tm, &n));  // every vertex with in-edges, once
   const float teleport = (float)((1.0 - (double)damping) / (double)V);
+  const Counts c0 = e->counts_h[0], c1 = e->counts_h[1];
+  if (c1.n == 0 || (e->cfg.flags & OG_CFG_DIRECT)) {
+    // Nothing to stage: iterations are launched ahead of the host's check, as
+    // many as the last run took, then four at a time; those after the end
+    // only read the done flag.  (A wait per iteration cost 25-35 us of each,
+    // all of an iteration on a small graph.)
+    const uint32_t *done = &e->prl_d->done;
+    const LbsArgs a0 = lbs_args(e, 0, 0, c0.total, true, e->plan.static_edges);
+    const LbsArgs a1 = lbs_args(e, 1, 0, c1.total, true, e->g->E);
+    CK(cudaStreamWaitEvent(s, e->ev_cd, 0));  // the dynamic region's list
+    uint32_t launched = 0, batch = std::max<uint32_t>(1, e->pr_hint);
+    while (launched < (uint32_t)max_iter) {
+      batch = std::min<uint32_t>(batch, (uint32_t)max_iter - launched);
+      const uint32_t before = launched ? e->prl_h->iters : 0;
+      for (uint32_t i = 0; i < batch; i++, launched++) {
+        // the pulls of a run are alike: the first of a batch is timed
+        if (i == 0) CK(cudaEventRecord(e->t_d0, s));
+        if (c0.n && c1.n) {
+          RC(launch_pr_pull_pair(e, a0, EKU::stat(e), a1, EKU::host(e), done, s));
+        } else if (c0.n || c1.n) {
+          const int r = c0.n ? 0 : 1;
+          RC((pr_contiguous(e, r)
+                  ? launch_pr_pull<true>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)
+                  : launch_pr_pull<false>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)));
+        }
+        if (i == 0) CK(cudaEventRecord(e->ev_dyn_done, s));
+        RC(launch_pr_fixup(e, done));
+        RC(launch_pr_update(e, teleport, damping, tol, done));
+      }
+      RC(pr_check(e, st));
+      float ms = 0;
+      if (cudaEventElapsedTime(&ms, e->t_d0, e->ev_dyn_done) == cudaSuccess)
+        (c1.n ? st.ms_dynamic : st.ms_static) += ms * (e->prl_h->iters - before);
+      if (e->prl_h->done) break;
+      batch = 4;
+    }
+    const uint64_t its = e->prl_h->iters;
+    e->pr_hint = (uint32_t)its;
+    st.iterations += (uint32_t)its;
+    st.frontier_sum += n * its;
+    st.static_vertices += c0.n * its;
+    st.edges_static += c0.total * its;
+    st.edges_dynamic += c1.total * its;
+    st.link_bytes += (c1.total * e->bpe + 7) / 8 * its;
+    if (c1.n) st.chunks += (uint32_t)its;
+    e->last_algo = OG_ALGO_PR;
+    return OG_OK;
+  }
   for (int it = 0; it < max_iter; it++) {
     st.iterations++;
     st.frontier_sum += n;
     st.static_vertices += e->counts_h[0].n;
     RC(pr_sums(e, st, tm));
-    k_pr_update_l1<<<e->part_n, kThreads, 0, s>>>(V, (float *)e->value_d, e->contrib_d, e->sum_d,
-                                                  e->outdeg_d, teleport, damping, e->part_d);
-    e->launches++;
-    k_reduce_f64<<<1, kThreads, 0, s>>>(e->part_d, e->part_n, e->l1_d);
-    e->launches++;
-    CK(cudaMemcpyAsync(e->l1_h, e->l1_d, sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    RC(check_device_error(e));
+    RC(launch_pr_update(e, teleport, damping, tol, nullptr));
+    RC(pr_check(e, st));
     collect_timing(e, tm, &st);
-    st.residual = *e->l1_h;
-    if (*e->l1_h < tol) break;
+    if (e->prl_h->done) break;
   }
   e->last_algo = OG_ALGO_PR;
   return OG_OK;
@@ -2233,6 +2307,7 @@ int run_pr_l1_push(og_engine *e, float damping, double tol, int max_iter, og_sta
   cudaStream_t s = e->s_main;
   const int g = grid_for(V, e->sms);
   CK(cudaMemsetAsync(e->err_d, 0, 16, s));
+  CK(cudaMemsetAsync(e->prl_d, 0, sizeof(PrLoop), s));
   k_pr_init<<<g, kThreads, 0, s>>>(V, (float *)e->value_d, e->contrib_d, e->sum_d, e->outdeg_d,
                                    (float)(1.0 / (double)V));
   e->launches++;
@@ -2267,18 +2342,10 @@ int run_pr_l1_push(og_engine *e, float damping, double tol, int max_iter, og_sta
     st.static_vertices += e->counts_h[0].n;
     CK(cudaMemsetAsync(e->sum_d, 0, 4 * V, s));
     RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
-    k_pr_update_l1<<<e->part_n, kThreads, 0, s>>>(V, (float *)e->value_d, e->contrib_d, e->sum_d,
-                                                  e->outdeg_d, teleport, damping, e->part_d);
-    e->launches++;
-    k_reduce_f64<<<1, kThreads, 0, s>>>(e->part_d, e->part_n, e->l1_d);
-    e->launches++;
-    CK(cudaMemcpyAsync(e->l1_h, e->l1_d, sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    RC(check_device_error(e));
+    RC(launch_pr_update(e, teleport, damping, tol, nullptr));
+    RC(pr_check(e, st));
     collect_timing(e, tm, &st);
-    st.residual = *e->l1_h;
-    if (*e->l1_h < tol) break;
+    if (e->prl_h->done) break;
   }
   e->last_algo = OG_ALGO_PR;
   return OG_OK;

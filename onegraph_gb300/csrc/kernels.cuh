@@ -1348,6 +1348,8 @@ struct PrArgs {
   // a staging buffer): position q is record base + q of the record stream,
   // which holds nwords words
   uint64_t base, nwords;
+  // iterations launched ahead: when not null, nothing is done once *done is set
+  const uint32_t *done;
 };
 
 // Pull sum sum[v] = sum over in-edges (u -> v) of contrib[u]
@@ -1385,7 +1387,7 @@ __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const 
   __shared__ float s_wv[kThreads / 32];
   __shared__ uint32_t s_wc[kThreads / 32];
   const uint64_t pos0 = k * kTile;
-  if (pos0 >= a.pos_end) return;
+  if (pos0 >= a.pos_end || (p.done && *p.done)) return;
   const uint64_t pend = min(pos0 + kTile, a.pos_end);
   const uint32_t tlen = (uint32_t)(pend - pos0), tid = threadIdx.x, x0 = tid * kItems;
   // the tile's words, from the 16-byte boundary at or before its first record
@@ -1595,7 +1597,7 @@ struct PrFixup {
 };
 __global__ void k_pr_fixup(PrFixup f0, uint64_t n0, PrFixup f1, uint64_t n1) {
   const uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (x >= n0 + n1) return;
+  if (x >= n0 + n1 || (f0.p.done && *f0.p.done)) return;
   const bool r0 = x < n0;
   const uint64_t k = r0 ? x : x - n0;
   const PrFixup &f = r0 ? f0 : f1;
@@ -1643,20 +1645,37 @@ __global__ void __launch_bounds__(kThreads) k_pr_update_delta(
   if (threadIdx.x == 0 && s_cnt) atomicAdd(active, s_cnt);
 }
 
+// State of L1 iterations that are launched ahead of the host's checks.
+struct PrLoop {
+  double residual;  // of the last iteration
+  uint32_t done;    // it was below the tolerance
+  uint32_t iters;
+};
+
 // Normalised update p' = teleport + damping*sum for every vertex, with the L1
 // delta accumulated in FP64: per-thread, then a fixed-shape block tree, one
 // partial per block (the grid size is fixed, so the order never changes).
-// Bound by HBM (20 B a vertex): four vertices per thread and load.  All four
-// arrays are 16-byte aligned (their own allocations, or padded in the arena).
+// Bound by FP64 (few units on this part): 8.4 M vertices took 69 us with two
+// conversions, a subtraction and an addition each.  new - old is first taken in
+// FP32 together with its rounding error (Knuth's two-sum); where a warp's
+// errors are all zero, as in most iterations but the first, the FP32
+// difference is exact and costs one conversion and one addition, with the
+// same bits.  Four vertices per thread and load; all four arrays are 16-byte
+// aligned (their own allocations, or padded in the arena).
 __global__ void __launch_bounds__(kThreads) k_pr_update_l1(uint64_t V, float *rank, float *contrib,
                                                            const float *sum, const uint32_t *outdeg,
                                                            float teleport, float damping,
-                                                           double *part) {
+                                                           double *part, const uint32_t *done) {
   __shared__ double s_d[kThreads];
+  if (done && *done) return;
   double acc = 0.0;
-  auto one = [&](float s, uint32_t od, float &r, float &c) {
+  // one vertex's update; d = new - old in FP32, err its rounding error
+  auto one = [&](float s, uint32_t od, float &r, float &c, float &old, float &d, float &err) {
     const float nvv = teleport + damping * s;
-    acc += fabs((double)nvv - (double)r);
+    old = r;
+    d = __fsub_rn(nvv, r);
+    const float t = __fsub_rn(d, nvv);
+    err = __fsub_rn(__fsub_rn(nvv, __fsub_rn(d, t)), __fadd_rn(r, t));
     r = nvv;
     c = od ? nvv / (float)od : 0.f;
   };
@@ -1665,16 +1684,29 @@ __global__ void __launch_bounds__(kThreads) k_pr_update_l1(uint64_t V, float *ra
     const float4 s = reinterpret_cast<const float4 *>(sum)[q];
     const uint4 od = reinterpret_cast<const uint4 *>(outdeg)[q];
     float4 r = reinterpret_cast<float4 *>(rank)[q], c;
-    one(s.x, od.x, r.x, c.x);
-    one(s.y, od.y, r.y, c.y);
-    one(s.z, od.z, r.z, c.z);
-    one(s.w, od.w, r.w, c.w);
+    float old[4], d[4], err[4];
+    one(s.x, od.x, r.x, c.x, old[0], d[0], err[0]);
+    one(s.y, od.y, r.y, c.y, old[1], d[1], err[1]);
+    one(s.z, od.z, r.z, c.z, old[2], d[2], err[2]);
+    one(s.w, od.w, r.w, c.w, old[3], d[3], err[3]);
     reinterpret_cast<float4 *>(rank)[q] = r;
     reinterpret_cast<float4 *>(contrib)[q] = c;
+    const bool exact = err[0] == 0.f && err[1] == 0.f && err[2] == 0.f && err[3] == 0.f;
+    if (__all_sync(__activemask(), exact)) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc += (double)fabsf(d[i]);
+    } else {
+      acc += fabs((double)r.x - (double)old[0]);
+      acc += fabs((double)r.y - (double)old[1]);
+      acc += fabs((double)r.z - (double)old[2]);
+      acc += fabs((double)r.w - (double)old[3]);
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x < V - 4 * V4) {
     const uint64_t v = 4 * V4 + threadIdx.x;
-    one(sum[v], outdeg[v], rank[v], contrib[v]);
+    float old, d, err;
+    one(sum[v], outdeg[v], rank[v], contrib[v], old, d, err);
+    acc += fabs((double)rank[v] - (double)old);
   }
   s_d[threadIdx.x] = acc;
   __syncthreads();
@@ -1685,8 +1717,10 @@ __global__ void __launch_bounds__(kThreads) k_pr_update_l1(uint64_t V, float *ra
   if (threadIdx.x == 0) part[blockIdx.x] = s_d[0];
 }
 
-__global__ void k_reduce_f64(const double *part, uint32_t n, double *out) {
+// Sum of the partials, and the end of the iteration.
+__global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double tol) {
   __shared__ double s_d[kThreads];
+  if (loop->done) return;
   double acc = 0.0;
   for (uint32_t i = threadIdx.x; i < n; i += kThreads) acc += part[i];
   s_d[threadIdx.x] = acc;
@@ -1695,7 +1729,11 @@ __global__ void k_reduce_f64(const double *part, uint32_t n, double *out) {
     if ((int)threadIdx.x < s) s_d[threadIdx.x] += s_d[threadIdx.x + s];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = s_d[0];
+  if (threadIdx.x == 0) {
+    loop->residual = s_d[0];
+    loop->iters++;
+    if (s_d[0] < tol) loop->done = 1;
+  }
 }
 
 __global__ void k_pr_init(uint64_t V, float *rank, float *contrib, float *sum, const uint32_t *outdeg,
