@@ -3026,7 +3026,7 @@ extern "C" int og_result_checksum(og_engine *e, int algo, uint64_t *out) {
     const uint32_t nb = (uint32_t)e->sms * 8;
     unsigned long long *fin = e->sum64_d + 3ull * nb;
     k_checksum<<<nb, kThreads, 0, e->s_main>>>(e->value_d, e->V, mode, unreached, e->sum64_d);
-    k_checksum_final<<<1, 32, 0, e->s_main>>>(e->sum64_d, nb, mode, fin);
+    k_checksum_final<<<1, kThreads, 0, e->s_main>>>(e->sum64_d, nb, mode, fin);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(e->counts_h, fin, 16, cudaMemcpyDeviceToHost, e->s_main));
     CK(cudaStreamSynchronize(e->s_main));

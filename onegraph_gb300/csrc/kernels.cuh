@@ -1801,18 +1801,39 @@ __global__ void __launch_bounds__(kThreads) k_checksum(const uint32_t *val, uint
   }
 }
 
-__global__ void k_checksum_final(const unsigned long long *part, uint32_t n, int mode,
-                                 unsigned long long *out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Sums the partials of the blocks.  The integer sums are exact in
+// any order; the FP64 sum is added in block order by one thread, as it defines
+// the checksum's bits, but out of shared memory (one dependent global load per
+// block took 120 us).
+constexpr uint32_t kChecksumBatch = 1024;
+__global__ void __launch_bounds__(kThreads) k_checksum_final(const unsigned long long *part, uint32_t n, int mode,
+                                                             unsigned long long *out) {
+  __shared__ unsigned long long s_c, s_s;
+  __shared__ double s_d[kChecksumBatch];
+  if (threadIdx.x == 0) s_c = s_s = 0;
+  __syncthreads();
   unsigned long long c = 0, sum = 0;
-  double d = 0.0;
-  for (uint32_t i = 0; i < n; i++) {
+  for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
     c += part[3 * i];
     sum += part[3 * i + 1];
-    d += __longlong_as_double(part[3 * i + 2]);
   }
-  out[0] = c;
-  out[1] = mode == 2 ? (unsigned long long)__double_as_longlong(d) : sum;
+  atomicAdd(&s_c, c);
+  atomicAdd(&s_s, sum);
+  double d = 0.0;
+  if (mode == 2)
+    for (uint32_t i0 = 0; i0 < n; i0 += kChecksumBatch) {
+      const uint32_t m = min(kChecksumBatch, n - i0);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < m; i += kThreads) s_d[i] = __longlong_as_double(part[3 * (i0 + i) + 2]);
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (uint32_t i = 0; i < m; i++) d += s_d[i];
+    }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out[0] = s_c;
+    out[1] = mode == 2 ? (unsigned long long)__double_as_longlong(d) : s_s;
+  }
 }
 
 // ------------------------------------------------------------------ fills
