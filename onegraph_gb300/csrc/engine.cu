@@ -966,6 +966,30 @@ int launch_relax(og_engine *e, const RoundOps &ro, const LbsArgs &a, Src src, ui
   return OG_OK;
 }
 
+// One staged step (k_stage_step): gathers chunk `g` into buffer gbuf and relaxes
+// chunk `r` out of the other one; either may be absent (pos_begin == pos_end).
+template <class K>
+int launch_stage_step(og_engine *e, const RoundOps &ro, const LbsArgs &g, int gbuf, const LbsArgs &r, uint32_t *next,
+                      cudaStream_t s) {
+  const unsigned ng = lbs_grid(g.pos_begin, g.pos_end), nr = lbs_grid(r.pos_begin, r.pos_end);
+  const auto src = K::stage(e, gbuf ^ 1);
+  const auto dst = K::stage_dst(e, gbuf);
+  if constexpr (std::is_same<typename K::Src, SrcU>::value) {
+    if (ro.algo == OG_ALGO_BFS) {
+      BfsOp op{e->bm[2], next, e->value_d, e->err_d, e->V, ro.level + 1};
+      k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
+    } else {
+      MinOp<false> op{e->value_d, next, e->err_d, e->V};
+      k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
+    }
+  } else {
+    MinOp<true> op{e->value_d, next, e->err_d, e->V};
+    k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
+  }
+  e->launches++;
+  return OG_OK;
+}
+
 template <class K>
 int launch_gather(og_engine *e, const LbsArgs &a, int buf, cudaStream_t s) {
   constexpr uint64_t T = (uint64_t)kGatherMult * kTile;
@@ -1007,6 +1031,7 @@ void collect_timing(og_engine *e, Timing &t, og_stats *st) {
 }
 
 struct NoPair {};
+struct NoStage {};
 
 // One round's region work given the compaction counts (already on the host).
 // `static_fn(a)` / `dyn_fn(a, src, stream)` launch the per-region kernel;
@@ -1014,9 +1039,11 @@ struct NoPair {};
 // as one interleaved kernel (direct mode with both regions non-empty): the
 // static tiles then overlap the link-bound dynamic ones instead of taking the
 // SMs first.  Its time is counted as dynamic-region time.
-template <class K, class StaticFn, class DynFn, class PairFn = NoPair>
+// `stage_fn(g, gbuf, r)`, when given, launches a staged step: gather of chunk g
+// into buffer gbuf beside the relax of chunk r (empty: none) out of the other.
+template <class K, class StaticFn, class DynFn, class PairFn = NoPair, class StageFn = NoStage>
 int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynFn dyn_fn,
-                PairFn pair_fn = PairFn()) {
+                PairFn pair_fn = PairFn(), StageFn stage_fn = StageFn()) {
   const Counts cs = e->counts_h[0], cd = e->counts_h[1];
   if constexpr (!std::is_same<PairFn, NoPair>::value) {
     if (cs.n && cd.n && (e->cfg.flags & OG_CFG_DIRECT)) {
@@ -1047,6 +1074,18 @@ int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynF
     } else if constexpr (!K::kFrag) {
       const uint64_t C = e->plan.chunk_edges;
       const uint64_t nch = (cd.total + C - 1) / C;
+      if constexpr (!std::is_same<StageFn, NoStage>::value) {
+        cudaEvent_t g0, g1;
+        RC(gather_events(e, tm.pend_g, &g0, &g1));
+        CK(cudaEventRecord(g0, e->s_dyn));
+        for (uint64_t c = 0; c <= nch; c++) {
+          const uint64_t gb = std::min(c * C, cd.total), ge = std::min(gb + C, cd.total);
+          const uint64_t rb = c ? (c - 1) * C : 0, re = c ? std::min(rb + C, cd.total) : 0;
+          RC(stage_fn(lbs_args(e, 1, gb, ge, true, e->g->E), (int)(c & 1), lbs_args(e, 1, rb, re, false, C)));
+          if (c + 1 == nch) CK(cudaEventRecord(g1, e->s_dyn));  // the last step that gathers
+        }
+        tm.pend_g++;
+      } else
       for (uint64_t c = 0; c < nch; c++) {
         const int buf = (int)(c & 1);
         const uint64_t b = c * C, en = std::min(b + C, cd.total);
@@ -1232,7 +1271,11 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
     auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
       return launch_relax_pair(e, ro, a0, s0, a1, s1, next, ps);
     };
-    RC((run_regions<K>(e, st, tm, sfn, dfn, pfn)));
+    auto gfn = [&](const LbsArgs &ga, int gbuf, const LbsArgs &ra) {
+      if constexpr (K::kFrag) return (int)OG_OK;  // direct mode only
+      else return launch_stage_step<K>(e, ro, ga, gbuf, ra, next, e->s_dyn);
+    };
+    RC((run_regions<K>(e, st, tm, sfn, dfn, pfn, gfn)));
     if constexpr (K::kFrag) e->frag->since += e->counts_h[1].total;
     CK(cudaStreamWaitEvent(e->s_main, e->ev_cd, 0));
     CK(cudaMemsetAsync(cur, 0, 4 * e->nwords, e->s_main));
@@ -2140,27 +2183,31 @@ int launch_pr_fixup(og_engine *e, const uint32_t *done) {
 int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
   CK(cudaEventRecord(e->ev_round, e->s_main));
   CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-  CK(cudaStreamWaitEvent(e->s_gat, e->ev_round, 0));
   auto sfn = [&](const LbsArgs &a) {
     return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main)
                                : launch_pr_pull<false>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main);
   };
   auto dfn = [&](const LbsArgs &a, auto src, cudaStream_t ds) {
-    if constexpr (std::is_same<decltype(src), SrcU>::value) {
-      // a staging buffer: columns from position pos_begin on, as 32-bit records
-      PrArgs q = pr_args(e, 1, nullptr);
-      q.base = 0ull - a.pos_begin;
-      q.nwords = a.edge_bound;
-      return launch_pr_pull<true>(e, a, SrcP<false>{src.col, 32u, 32u, 0u}, q, ds);
-    } else {
+    if constexpr (std::is_same<decltype(src), SrcU>::value) return (int)OG_OK;  // staged: gfn
+    else
       return pr_contiguous(e, 1) ? launch_pr_pull<true>(e, a, src, pr_args(e, 1, nullptr), ds)
                                  : launch_pr_pull<false>(e, a, src, pr_args(e, 1, nullptr), ds);
-    }
+  };
+  auto gfn = [&](const LbsArgs &g, int gbuf, const LbsArgs &r) {
+    const unsigned ng = lbs_grid(g.pos_begin, g.pos_end), nr = lbs_grid(r.pos_begin, r.pos_end);
+    // a staging buffer: columns from position pos_begin on, as 32-bit records
+    PrArgs q = pr_args(e, 1, nullptr);
+    q.base = 0ull - r.pos_begin;
+    q.nwords = r.edge_bound;
+    k_stage_step_pr<<<ng + nr, kThreads, pr_smem_bytes(true, 32), e->s_dyn>>>(
+        g, EKU::host(e), EKU::stage_dst(e, gbuf), ng, r, SrcP<false>{e->stage_col[gbuf ^ 1], 32u, 32u, 0u}, q);
+    e->launches++;
+    return (int)OG_OK;
   };
   auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
     return launch_pr_pull_pair(e, a0, s0, a1, s1, nullptr, ps);
   };
-  RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn)));
+  RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn, gfn)));
   return launch_pr_fixup(e, nullptr);
 }
 

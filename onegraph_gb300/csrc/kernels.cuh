@@ -1064,6 +1064,44 @@ __global__ void __launch_bounds__(kThreads) k_lbs_pair(LbsArgs a0, Src0 s0, LbsA
   else lbs_tile(a1, s1, op, sh, a1.pos_begin / kTile + pt.t);
 }
 
+// The dynamic-region gather as an edge op: positions of a chunk go to a staging
+// buffer whose entry 0 is position `base`.
+template <class Dst>
+struct GatherOp {
+  using Val = uint32_t;
+  static constexpr bool kNeedVal = false;
+  Dst stage;
+  uint64_t base;
+  __device__ uint32_t src_val(uint32_t) const { return 0; }
+  using Probe = uint32_t;
+  template <class Edge>
+  __device__ __forceinline__ Probe probe(Edge) const {
+    return 0u;
+  }
+  template <class Edge>
+  __device__ __forceinline__ void relax(Edge e, uint32_t, uint64_t pos, Probe) const {
+    stage.store(pos - base, e);
+  }
+};
+
+// One step of a staged round: the first ng CTAs gather chunk c (list g) while
+// the others relax chunk c - 1 (list r) out of the other staging buffer.  With
+// two streams and an event in each direction per chunk the same work took a
+// dozen host calls a chunk, 40 us of them; now launch order is the only
+// synchronisation.
+template <class PSrc, class Dst, class Src, class Op>
+__global__ void __launch_bounds__(kThreads, 5) k_stage_step(LbsArgs g, PSrc ps, Dst dst, uint32_t ng, LbsArgs r,
+                                                            Src src, Op op) {
+  __shared__ union {
+    LbsSh<GatherOp<Dst>> gather;
+    LbsSh<Op> relax;
+  } sh;
+  if (blockIdx.x < ng)
+    lbs_tile(g, ps, GatherOp<Dst>{dst, g.pos_begin}, sh.gather, g.pos_begin / kTile + blockIdx.x);
+  else
+    lbs_tile(r, src, op, sh.relax, r.pos_begin / kTile + blockIdx.x - ng);
+}
+
 template <int MULT>
 constexpr size_t gather_smem_bytes() {
   return 8 * (MULT * kTile + 1) + 4 * (MULT * kTile + 2) + 2 * (MULT * kTile);
@@ -1573,6 +1611,17 @@ __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const 
 template <bool kDense, class Src>
 __global__ void __launch_bounds__(kThreads, 6) k_pr_pull(LbsArgs a, Src src, PrArgs p) {
   pr_tile<kDense>(a, src, p, a.pos_begin / kTile + blockIdx.x);
+}
+
+// The staged step of a PageRank round (see k_stage_step).
+template <class PSrc, class Dst, class Src>
+__global__ void __launch_bounds__(kThreads, 6) k_stage_step_pr(LbsArgs g, PSrc ps, Dst dst, uint32_t ng, LbsArgs r,
+                                                               Src src, PrArgs p) {
+  __shared__ LbsSh<GatherOp<Dst>> sh;
+  if (blockIdx.x < ng)
+    lbs_tile(g, ps, GatherOp<Dst>{dst, g.pos_begin}, sh, g.pos_begin / kTile + blockIdx.x);
+  else
+    pr_tile<true>(r, src, p, r.pos_begin / kTile + blockIdx.x - ng);
 }
 
 // Both regions' pull sums in one launch, static and dynamic tiles interleaved
