@@ -684,7 +684,6 @@ int create(og_graph *g, const og_config *cfg, og_engine *e) {
   // choice, 9.85 at 58 %, 6.77 at 86 %, 8.06 at 30 %.
   CK(cudaFuncSetAttribute(k_lbs_pair<SrcP<true>, SrcP<true>, MinOp<true>>,
                           cudaFuncAttributePreferredSharedMemoryCarveout, 58));
-  CK(cudaFuncSetAttribute(k_min_rounds<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
   CK(cudaFuncSetAttribute(k_bfs_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShared)));
   if (cfg->flags & OG_CFG_REPLACE) {  // the same relax reading fragment slots
     CK(cudaFuncSetAttribute(k_lbs_pair<SrcP<true>, SrcF<true>, MinOp<true>>,

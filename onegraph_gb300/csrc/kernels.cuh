@@ -842,13 +842,17 @@ struct DstW {
   }
 };
 
-// Per-tile tables.  kVal = false (BFS reads no source value) drops the value
-// table, 8 KB of shared memory per CTA that L1 gets instead.
+// Per-tile tables.  Most tiles hold far fewer vertices than positions, so the
+// cursor and value tables have kLocal entries, and a tile with more vertices
+// is worked off in parts of kThreads positions (which hold at most kThreads
+// vertices each, plus one).  With tables for 2048 vertices a CTA took 37 KB of shared
+// memory: four CTAs per SM and little L1.  kVal = false (BFS reads no source
+// value) drops the value table.
+constexpr uint32_t kLocal = 512;
 template <class Val, bool kVal = true>
 struct LbsShared {
-  uint32_t rs[kTile + 2];      // tile-relative start of each local vertex
-  unsigned long long cb[kTile + 1];  // source cursor of tile position 0 for the vertex
-  Val val[kVal ? kTile + 1 : 1];     // source value of each local vertex
+  unsigned long long cb[kLocal];  // source cursor of tile position 0 for the vertex
+  Val val[kVal ? kLocal : 1];     // source value of each local vertex
   alignas(16) unsigned short map[kTile];  // tile position -> local vertex
 };
 
@@ -878,75 +882,60 @@ struct HasProbeVal : std::false_type {};
 template <class T>
 struct HasProbeVal<T, std::void_t<decltype(T::kProbeVal)>> : std::true_type {};
 
-// Builds the local-vertex tables of tile k; returns the local count (0 on
-// error).  Sh is LbsShared<Val, *> or PrShared.  cb[j] is the source cursor
-// (Src::cur) of tile position 0 for local vertex j, so position x of the tile
-// reads src.at(cb[map[x]], x).  Every local vertex's edge indices in the tile
-// are checked against edge_bound here, once per vertex; a tile with one out
-// of bounds sets kErrEdgeIndex and relaxes nothing.
-//
-// kPart: only positions [lo, hi) of the tile are read, and only the vertices
-// that have some are looked up.
-template <bool kNeedVal, bool kPart = false, class Src, class Op, class Sh>
-__device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, const Op &op, Sh &sh,
-                                              uint64_t k, uint64_t pos0, uint32_t &i0_out, uint32_t lo = 0,
-                                              uint32_t hi = kTile) {
+// Runs `body(lo, hi, j0)` over positions [plo, phi) of tile k: once, or in parts
+// of kThreads positions when the tile holds more than kLocal vertices.  In
+// the body, position x belongs to table entry map[x] - j0, and src.at(cb[entry],
+// x) is its record (cb holds the source cursor, Src::cur, of tile position
+// 0).  Every vertex's edge indices in the range are checked against edge_bound
+// when its entry is made; one out of bounds sets kErrEdgeIndex and the range is
+// skipped.  Sh is LbsShared<Val, *>.
+template <bool kNeedVal, class Src, class Op, class Sh, class Body>
+__device__ __forceinline__ void lbs_run(const LbsArgs &a, const Src &src, const Op &op, Sh &sh, uint64_t k,
+                                        uint32_t plo, uint32_t phi, Body body) {
   __shared__ uint32_t s_bad;
+  const uint64_t pos0 = k * kTile;
   const uint64_t ntiles_total = (a.total + kTile - 1) / kTile;
   const uint32_t i0 = a.tile_first[k];
   const uint32_t i1 = (k + 1 < ntiles_total) ? a.tile_first[k + 1] : a.n - 1;
-  i0_out = i0;
   if (i1 < i0 || i1 - i0 > kTile || i1 >= a.n) {
     if (threadIdx.x == 0) atomicOr(a.err, kErrTileMap);
-    return 0;
+    return;
   }
-  const uint64_t pend = min(pos0 + kTile, a.pos_end);
   const uint32_t nl = i1 - i0 + 1;
+  const bool parts = nl > kLocal;  // uniform
   if (threadIdx.x == 0) s_bad = 0;
   // zero the position map: 2048 u16 = one 16-byte store per thread
   static_assert(kTile * sizeof(unsigned short) == kThreads * sizeof(uint4), "map zeroing");
   reinterpret_cast<uint4 *>(sh.map)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  bool bad = false;
+  // table entry x of local vertex j (list prefix p, start r), whose positions in [lo, hi) are used
+  auto entry = [&](uint32_t x, uint32_t j, uint64_t p, uint32_t r, uint32_t lo, uint32_t hi) {
+    const uint32_t i = i0 + j;
+    const uint64_t pn = a.pref[i + 1];
+    if (r >= hi || pn <= pos0 + lo) return;  // no position here
+    const uint32_t v = a.list[i];
+    const uint64_t e0 = (a.off ? a.off[v] - p : (0ull - a.stage_base)) + pos0;  // edge index of position 0
+    const uint64_t first = e0 + max(r, lo), last = e0 + (min(pn, pos0 + hi) - pos0) - 1;
+    uint64_t cb = src.cur(e0);
+    if (pn < p || last < first || last >= a.edge_bound) {
+      s_bad = 1;
+      atomicOr(a.err, kErrEdgeIndex);
+    } else if constexpr (HasCurRange<Src>::value) {
+      cb = src.cur_range(e0, first, last);
+      if constexpr (HasNote<Src>::value) src.note(first, (uint32_t)(last - first + 1));
+    }
+    sh.cb[x] = cb;
+    if constexpr (HasListVal<Op>::value) sh.val[x] = op.list_val(v, a.list + i);
+    else if constexpr (kNeedVal) sh.val[x] = op.src_val(v);
+  };
 #pragma unroll 1
   for (uint32_t j = threadIdx.x; j < nl; j += kThreads) {
-    const uint32_t i = i0 + j;
-    const uint32_t v = a.list[i];
-    const uint64_t p = a.pref[i], pn = a.pref[i + 1];
+    const uint64_t p = a.pref[i0 + j];
     const uint32_t r = p > pos0 ? (uint32_t)min(p - pos0, (uint64_t)kTile) : 0u;
-    sh.rs[j] = r;
     // head flag.  Compacted lists hold no zero-degree vertex, so for j >= 1
-    // the starts are distinct and strictly increasing (rs[0] = 0).
+    // the starts are distinct and strictly increasing (the first is 0).
     if (j >= 1 && r < kTile) sh.map[r] = (unsigned short)1;
-    if (kPart && (r >= hi || pn <= pos0 + lo)) continue;
-    const uint64_t e0 = (a.off ? a.off[v] - p : (0ull - a.stage_base)) + pos0;  // edge index of position 0
-    if constexpr (HasCurRange<Src>::value) {
-      uint64_t cb = src.cur(e0);
-      const uint64_t q1 = min(pn, pend);  // end of the vertex's positions in this tile
-      if (q1 > pos0 + r) {
-        const uint64_t first = e0 + r, last = e0 + (q1 - pos0) - 1;
-        if (pn < p || last < first || last >= a.edge_bound) {
-          bad = true;
-        } else {
-          cb = src.cur_range(e0, first, last);
-          if constexpr (HasNote<Src>::value) src.note(first, (uint32_t)(last - first + 1));
-        }
-      }
-      sh.cb[j] = cb;
-    } else {
-      sh.cb[j] = src.cur(e0);
-      const uint64_t q1 = min(pn, pend);  // end of the vertex's positions in this tile
-      if (q1 > pos0 + r) {
-        const uint64_t first = e0 + r, last = e0 + (q1 - pos0) - 1;
-        if (pn < p || last < first || last >= a.edge_bound) bad = true;
-      }
-    }
-    if constexpr (HasListVal<Op>::value) sh.val[j] = op.list_val(v, a.list + i);
-    else if constexpr (kNeedVal) sh.val[j] = op.src_val(v);
-  }
-  if (bad) {
-    s_bad = 1;
-    atomicOr(a.err, kErrEdgeIndex);
+    if (!parts) entry(j, j, p, r, plo, phi);
   }
   __syncthreads();
   // inclusive scan of the head flags (blocked: thread t owns positions 8t..8t+7)
@@ -968,63 +957,79 @@ __device__ __forceinline__ uint32_t lbs_setup(const LbsArgs &a, const Src &src, 
     reinterpret_cast<uint4 *>(sh.map)[threadIdx.x] = m;
   }
   __syncthreads();
-  return s_bad ? 0u : nl;
+  const uint32_t step = parts ? kThreads : kTile;
+#pragma unroll 1
+  for (uint32_t lo = plo; lo < phi; lo += step) {
+    const uint32_t hi = min(lo + step, phi);
+    uint32_t j0 = 0;
+    if (parts) {
+      j0 = sh.map[lo];
+      const uint32_t j1 = sh.map[hi - 1];
+      if (lo != plo) __syncthreads();  // the part before has been read
+      for (uint32_t j = j0 + threadIdx.x; j <= j1; j += kThreads) {
+        const uint64_t p = a.pref[i0 + j];
+        entry(j - j0, j, p, p > pos0 ? (uint32_t)min(p - pos0, (uint64_t)kTile) : 0u, lo, hi);
+      }
+      __syncthreads();
+    }
+    if (s_bad) return;  // uniform: written before a barrier, or a part later by nobody
+    body(lo, hi, j0);
+  }
 }
 
 // Shared tables of an LBS relax tile for Op.
 template <class Op>
 using LbsSh = LbsShared<typename Op::Val, Op::kNeedVal || HasListVal<Op>::value>;
 
-// One LBS tile (kTile positions starting at tile k of the list) of a CTA; with
-// kPart, part `part` of `parts` (1, 2, 4 or 8) equal ones.
-template <bool kPart = false, class Src, class Op>
+// One LBS tile (kTile positions starting at tile k of the list) of a CTA, or
+// part `part` of `parts` (1, 2, 4 or 8) equal ones.
+template <class Src, class Op>
 __device__ __forceinline__ void lbs_tile(const LbsArgs &a, const Src &src, const Op &op, LbsSh<Op> &sh,
                                          uint64_t k, uint32_t part = 0, uint32_t parts = 1) {
   const uint64_t pos0 = k * kTile;
   if (pos0 >= a.pos_end) return;
-  const uint32_t lo = kPart ? part * (kTile / parts) : 0u;
-  const uint32_t tlen = min((uint32_t)min((uint64_t)kTile, a.pos_end - pos0), kPart ? lo + kTile / parts : kTile);
-  if (kPart && lo >= tlen) return;  // uniform
-  uint32_t i0;
-  const uint32_t nl = lbs_setup<Op::kNeedVal, kPart>(a, src, op, sh, k, pos0, i0, lo, tlen);
-  if (nl == 0) return;
-  // All eight loads are issued before the first relax, so each thread keeps
-  // eight edge reads in flight (the host-link gather is latency bound).
-  const uint32_t x0 = lo + threadIdx.x;
-  typename Src::Item ev[kItems];
-  uint32_t lv[kItems];
+  const uint32_t plo = part * (kTile / parts);
+  const uint32_t phi = min((uint32_t)min((uint64_t)kTile, a.pos_end - pos0), plo + kTile / parts);
+  if (plo >= phi) return;  // uniform
+  lbs_run<Op::kNeedVal>(a, src, op, sh, k, plo, phi, [&](uint32_t lo, uint32_t hi, uint32_t j0) {
+    // All eight loads are issued before the first relax, so each thread keeps
+    // eight edge reads in flight (the host-link gather is latency bound).
+    const uint32_t x0 = lo + threadIdx.x;
+    typename Src::Item ev[kItems];
+    uint32_t lv[kItems];
 #pragma unroll
-  for (int it = 0; it < (int)kItems; it++) {
-    const uint32_t x = it * kThreads + x0;
-    lv[it] = 0;
-    if (x < tlen) {
-      const uint32_t l = sh.map[x];
-      lv[it] = l;
-      ev[it] = src.at(sh.cb[l], x);
+    for (int it = 0; it < (int)kItems; it++) {
+      const uint32_t x = it * kThreads + x0;
+      lv[it] = 0;
+      if (x < hi) {
+        const uint32_t l = sh.map[x] - j0;
+        lv[it] = l;
+        ev[it] = src.at(sh.cb[l], x);
+      }
     }
-  }
-  // Probe phase: every target's current state is read before the first
-  // atomic, so the eight random reads of a thread overlap (in program order
-  // the compiler may not lift a load above an earlier atomic).  A probe is
-  // only a filter: relax() acts through atomics, so a stale probe costs an
-  // extra atomic, never a wrong result.
-  typename Op::Probe pr[kItems];
+    // Probe phase: every target's current state is read before the first
+    // atomic, so the eight random reads of a thread overlap (in program order
+    // the compiler may not lift a load above an earlier atomic).  A probe is
+    // only a filter: relax() acts through atomics, so a stale probe costs an
+    // extra atomic, never a wrong result.
+    typename Op::Probe pr[kItems];
 #pragma unroll
-  for (int it = 0; it < (int)kItems; it++)
-    if (it * kThreads + x0 < tlen) {
-      if constexpr (HasProbeVal<Op>::value) pr[it] = op.probe_v(ev[it], sh.val[lv[it]]);
-      else pr[it] = op.probe(ev[it]);
+    for (int it = 0; it < (int)kItems; it++)
+      if (it * kThreads + x0 < hi) {
+        if constexpr (HasProbeVal<Op>::value) pr[it] = op.probe_v(ev[it], sh.val[lv[it]]);
+        else pr[it] = op.probe(ev[it]);
+      }
+#pragma unroll
+    for (int it = 0; it < (int)kItems; it++) {
+      if (it * kThreads + x0 < hi)
+        op.relax(ev[it], Op::kNeedVal ? sh.val[lv[it]] : typename Op::Val{},
+                 pos0 + it * kThreads + x0, pr[it]);
     }
-#pragma unroll
-  for (int it = 0; it < (int)kItems; it++) {
-    if (it * kThreads + x0 < tlen)
-      op.relax(ev[it], Op::kNeedVal ? sh.val[lv[it]] : typename Op::Val{},
-               pos0 + it * kThreads + x0, pr[it]);
-  }
+  });
 }
 
 template <class Src, class Op>
-__global__ void __launch_bounds__(kThreads) k_lbs(LbsArgs a, Src src, Op op) {
+__global__ void __launch_bounds__(kThreads, 5) k_lbs(LbsArgs a, Src src, Op op) {
   __shared__ LbsSh<Op> sh;
   lbs_tile(a, src, op, sh, a.pos_begin / kTile + blockIdx.x);
 }
@@ -1056,7 +1061,7 @@ __device__ __forceinline__ PairTile pair_split_cta(uint64_t n0, uint64_t n) {
 }
 
 template <class Src0, class Src1, class Op>
-__global__ void __launch_bounds__(kThreads) k_lbs_pair(LbsArgs a0, Src0 s0, LbsArgs a1, Src1 s1, Op op,
+__global__ void __launch_bounds__(kThreads, 5) k_lbs_pair(LbsArgs a0, Src0 s0, LbsArgs a1, Src1 s1, Op op,
                                                        uint64_t n0, uint64_t n) {
   __shared__ LbsSh<Op> sh;
   const PairTile pt = pair_split_cta(n0, n);

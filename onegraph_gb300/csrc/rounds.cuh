@@ -319,8 +319,9 @@ struct RelaxShared {
 // (resident SSSP of 0.3 M vertices: 1.05 -> 0.87 ms with parts).  The next ticket (and its region
 // split, by thread 0) is fetched while the current tile runs.
 template <class Src, class Op>
-__device__ __forceinline__ void relax_lists(const RoundsArgs &a, RelaxShared<Src> &rs, LbsSh<Op> &sh, const Op &op,
-                                            RoundSlot *slot) {
+__device__ __noinline__ Op relax_lists(RelaxShared<Src> &rs, LbsSh<Op> &sh, Op op, RoundSlot *slot) {
+  __builtin_assume(__isShared(&rs));  // shared, not generic, accesses
+  __builtin_assume(__isShared(&sh));
   if (threadIdx.x == 0) {
     for (int r = 0; r < 2; r++) {
       const unsigned long long x = slot->app[r];
@@ -348,9 +349,10 @@ __device__ __forceinline__ void relax_lists(const RoundsArgs &a, RelaxShared<Src
       rs.b[k ^ 1] = nb;
       if (nb < n) rs.pt[k ^ 1] = pair_split(nb / parts, n0, n0 + n1);
     }
-    lbs_tile<true>(rs.a[pt.r], rs.s[pt.r], op, sh, pt.t, b % parts, parts);
+    lbs_tile(rs.a[pt.r], rs.s[pt.r], op, sh, pt.t, b % parts, parts);
     __syncthreads();  // the tile tables are rebuilt and the next ticket is read after this
   }
+  return op;
 }
 
 template <class Src>
@@ -401,8 +403,12 @@ struct MinRoundOp : MinOp<kWeighted> {
 // propagation.  A round whose relax lowered nothing below the threshold is
 // followed by one scan of frontier and waiting set together at the advanced
 // threshold (the host loop scans the frontier, then the waiting set).
+// CTAs per SM, measured: three for label propagation and BFS (85 registers,
+// 23 M directed edges 641 us against 748 at four; resident BFS of 2^20 vertices
+// 173 against 182), four for SSSP, whose host-link rounds want more reads in
+// flight (2^24 vertices 12.5 ms against 12.9 at three and 12.7 at five).
 template <bool kWeighted>
-__global__ void __launch_bounds__(kThreads, 4) k_min_rounds(const __grid_constant__ RoundsArgs a,
+__global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(const __grid_constant__ RoundsArgs a,
                                                                            const __grid_constant__ SrcP<kWeighted> s0,
                                                                            const __grid_constant__ SrcP<kWeighted> s1) {
   using Op = MinRoundOp<kWeighted>;
@@ -470,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_min_rounds(const __grid_constan
     op.far_cand = 0xffffffffu;
     unsigned long long tr = 0;
     if (lead && a.timer) tr = globaltimer_ns();
-    relax_lists(a, rs, sh.lbs, op, slot);
+    op = relax_lists(rs, sh.lbs, op, slot);
     if (a.split) {
       const int near = __syncthreads_or(op.near);
       const uint32_t fc = block_min_u32(op.far_cand);
@@ -737,7 +743,7 @@ __device__ __noinline__ void bfs_bottom_up_level(const RoundsArgs &a, const SrcP
   bottom_up_words(a.off, a.V, a.Vs, stat, host, cur, a.bm[2], next, a.value, newdepth, slot->bu, &a.st->err);
 }
 
-__global__ void __launch_bounds__(kThreads, 4) k_bfs_rounds(const __grid_constant__ RoundsArgs a,
+__global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constant__ RoundsArgs a,
                                                             const __grid_constant__ SrcP<false> s0,
                                                             const __grid_constant__ SrcP<false> s1) {
   __shared__ union {
@@ -792,7 +798,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_bfs_rounds(const __grid_constan
         BfsOp op{a.bm[2], next, a.value, &st->err, a.V, level + 1};
         unsigned long long tr = 0;
         if (lead && a.timer) tr = globaltimer_ns();
-        relax_lists(a, rs, sh.lbs, op, slot);
+        relax_lists(rs, sh.lbs, op, slot);
         if (!rounds_sync(st, target)) return;
         if (lead && a.timer) st->ns_relax += globaltimer_ns() - tr;
       }

@@ -30,14 +30,13 @@
 namespace og {
 
 constexpr uint32_t kSbMaxSources = 32;
-// CTAs per SM of the relax (at most 64 registers at 256 threads) and
-// positions in flight per thread, chosen with -Xptxas -v (no spills) and by
-// measurement on R-MAT 23 and 27: 5 CTAs per SM at 48 registers ran 30-40 %
-// slower, and a 58 % shared-memory carve-out (3 CTAs per SM, more L1) 5-8 %
-// slower, than 4 CTAs per SM with the CUDA driver's carve-out.
-constexpr int kSbMinBlocks = 4;
+// CTAs per SM of the relax and positions in flight per thread: latency-bound
+// (long-scoreboard stalls, 22-26 % issue), so many CTAs with one position each.
+// 8-source pass over 2^20 vertices, ms: 8 CTAs x 1 position 2.29, 6 x 2 2.37,
+// 5 x 2 2.42, 4 x 3 2.61 (2.68 with 45 KB of tables a CTA instead of 12).
+constexpr int kSbMinBlocks = 8;
 template <int KS>
-constexpr int sb_positions_in_flight() { return 3; }
+constexpr int sb_positions_in_flight() { return 1; }
 
 struct SbCompactArgs {
   uint32_t *bits;        // bitmap scanned this round: the active set, or the waiting set
@@ -230,10 +229,8 @@ __device__ __forceinline__ void sb_tile(const LbsArgs &a, const Src &src, const 
   const uint64_t pos0 = k * kTile;
   if (pos0 >= a.pos_end) return;
   const uint32_t tlen = (uint32_t)(min(pos0 + kTile, a.pos_end) - pos0);
-  uint32_t i0;
-  const uint32_t nl = lbs_setup<true>(a, src, op, sh, k, pos0, i0);
-  if (nl == 0) return;
-  for (uint32_t base = 0; base < tlen; base += U * kThreads) {
+  lbs_run<true>(a, src, op, sh, k, 0u, tlen, [&](uint32_t lo, uint32_t hi, uint32_t j0) {
+  for (uint32_t base = lo; base < hi; base += U * kThreads) {
     typename Src::Item ev[U];
     uint2 val[U];
     uint32_t okm = 0;
@@ -241,8 +238,8 @@ __device__ __forceinline__ void sb_tile(const LbsArgs &a, const Src &src, const 
     for (int j = 0; j < U; j++) {
       const uint32_t x = base + j * kThreads + threadIdx.x;
       val[j] = make_uint2(0u, 0u);
-      if (x < tlen) {
-        const uint32_t l = sh.map[x];
+      if (x < hi) {
+        const uint32_t l = sh.map[x] - j0;
         val[j] = sh.val[l];
         ev[j] = src.at(sh.cb[l], x);
         okm |= 1u << j;
@@ -262,13 +259,13 @@ __device__ __forceinline__ void sb_tile(const LbsArgs &a, const Src &src, const 
     constexpr uint32_t cmask = (1u << C) - 1u;
 #pragma unroll
     for (int c = 0; c < KS / C; c++) {
-      uint4 lo[U], hi[U];
+      uint4 r0[U], r1[U];
 #pragma unroll
       for (int j = 0; j < U; j++) {
         if (((okm >> j) & 1u) && ((val[j].x >> (C * c)) & cmask)) {
           const uint4 *r = (const uint4 *)(op.dist + (uint64_t)edge_dst(ev[j]) * KS + C * c);
-          lo[j] = __ldcg(r);
-          if constexpr (C == 8) hi[j] = __ldcg(r + 1);
+          r0[j] = __ldcg(r);
+          if constexpr (C == 8) r1[j] = __ldcg(r + 1);
         }
       }
 #pragma unroll
@@ -279,12 +276,12 @@ __device__ __forceinline__ void sb_tile(const LbsArgs &a, const Src &src, const 
         const uint32_t w = edge_w(ev[j]);
         const uint32_t *ru = op.dist + (uint64_t)val[j].y * KS + C * c;
         uint32_t *rv = op.dist + (uint64_t)v * KS + C * c;
-        uint32_t d[8] = {lo[j].x, lo[j].y, lo[j].z, lo[j].w, 0u, 0u, 0u, 0u};
+        uint32_t d[8] = {r0[j].x, r0[j].y, r0[j].z, r0[j].w, 0u, 0u, 0u, 0u};
         if constexpr (C == 8) {
-          d[4] = hi[j].x;
-          d[5] = hi[j].y;
-          d[6] = hi[j].z;
-          d[7] = hi[j].w;
+          d[4] = r1[j].x;
+          d[5] = r1[j].y;
+          d[6] = r1[j].z;
+          d[7] = r1[j].w;
         }
 #pragma unroll
         for (int t = 0; t < C; t++) {
@@ -310,6 +307,7 @@ __device__ __forceinline__ void sb_tile(const LbsArgs &a, const Src &src, const 
       }
     }
   }
+  });
 }
 
 template <class Src, int KS>
