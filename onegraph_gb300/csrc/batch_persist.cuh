@@ -546,7 +546,7 @@ __device__ __forceinline__ uint32_t word_counts(uint32_t x, uint32_t present) {
 // newly reached vertices are counted per source (hist), and for the sources
 // in `msum_sel` their degrees are summed (the next level's direction
 // choice); the consumed frontier is cleared.
-constexpr int kTallyWords = 4;
+constexpr int kTallyWords = 2;
 template <int BLOCK, class SH>
 __device__ __forceinline__ void level_tally(const PersistArgs &a, SH &sh, unsigned long long bu,
                                             unsigned long long msum_sel, unsigned long long all_src,
@@ -613,13 +613,29 @@ __device__ __forceinline__ void level_tally(const PersistArgs &a, SH &sh, unsign
           }
         }
       }
-      if (a.depth)
-        for (unsigned long long b = x; b; b &= b - 1)
-          a.depth[(uint64_t)(__ffsll((long long)b) - 1) * a.V + (g + j) * 32 + lane] = level + 1;
-      if (a.depth8)
-        for (unsigned long long b = x; b; b &= b - 1)
-          a.depth8[(uint64_t)(__ffsll((long long)b) - 1) * a.V + (g + j) * 32 + lane] =
-              (uint8_t)min(level + 1, 255u);
+      // depths, one source of the word after another: the lanes' stores are
+      // consecutive (each lane walking its own bits scattered 64 sources x 32
+      // vertices of byte stores: 2.6 ms of a 64-source batch over 2^23
+      // vertices, 1.1 ms so)
+      if (a.depth8) {
+        uint8_t *row = a.depth8 + (g + j) * 32 + lane;
+        const uint8_t dl = (uint8_t)min(level + 1, 255u);
+        const uint32_t xl = (uint32_t)x, xh = (uint32_t)(x >> 32);
+        for (uint32_t m = plo; m; m &= m - 1) {
+          const uint32_t src = __ffs(m) - 1;
+          if ((xl >> src) & 1u) row[(uint64_t)src * a.V] = dl;
+        }
+        row += 32ull * a.V;
+        for (uint32_t m = phi; m; m &= m - 1) {
+          const uint32_t src = __ffs(m) - 1;
+          if ((xh >> src) & 1u) row[(uint64_t)src * a.V] = dl;
+        }
+      } else if (a.depth) {
+        for (unsigned long long m = ((unsigned long long)phi << 32) | plo; m; m &= m - 1) {
+          const uint32_t src = __ffsll((long long)m) - 1;
+          if ((x >> src) & 1ull) a.depth[(uint64_t)src * a.V + (g + j) * 32 + lane] = level + 1;
+        }
+      }
     }
 #pragma unroll
     for (int j = 0; j < kTallyWords; j++) {
