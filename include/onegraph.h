@@ -257,9 +257,9 @@ typedef struct og_stats {
   double ms_compact;         /* device time of frontier compaction          */
   double residual;           /* PR: last L1 delta; otherwise 0              */
   uint64_t launches;         /* kernels launched for the query              */
-  double ms_gather;          /* staged mode: device time of the steps that gather
-                                a chunk (each relaxes the one before beside
-                                it; batched queries: of the gathers alone)  */
+  double ms_gather;          /* staged mode: device time of the rounds' one
+                                launch, which gathers and relaxes (batched
+                                queries: of the gathers alone)              */
   double ms_relax;           /* device-driven rounds with
                                 OG_PARAM_RELAX_TIMER: time of the (top-down)
                                 relax phases; otherwise 0                   */

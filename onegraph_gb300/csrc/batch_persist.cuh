@@ -31,7 +31,6 @@
 
 namespace og {
 
-constexpr uint32_t kErrBarrier = 16u;   // a grid barrier wait gave up
 constexpr uint32_t kErrLevels = 32u;    // more levels than the histogram holds
 constexpr uint32_t kMaxBatchLevels = 1024;
 

@@ -137,6 +137,7 @@ struct og_engine {
   cudaGraphExec_t graph = nullptr;
   // device-driven rounds (rounds.cuh): state and its page-locked host mirror
   RoundsState *rounds_d = nullptr, *rounds_h = nullptr;
+  uint32_t *ring_d = nullptr;  // staged rounds: ticket, then (kRingPad words on) the slot states
   uint32_t level_loop = 0;        // OG_LOOP_AUTO / OG_LOOP_HOST
   uint32_t relax_timer = 0;       // OG_PARAM_RELAX_TIMER
   void *out = nullptr;            // the running query's result buffer, until its copy is enqueued
@@ -566,6 +567,7 @@ int create_query_state(og_engine *e) {
       RC(dalloc(e, &e->stage_col[b], P.chunk_edges));
       if (e->wbytes) RC(dalloc(e, (char **)&e->stage_w[b], P.chunk_edges * e->wbytes));
     }
+    RC(dalloc(e, &e->ring_d, kRingPad + kRingSlots));  // 8 KiB of the planner's 64 for small arrays
   }
   // PageRank's contributions and sums live in the batch arena when the
   // engine has one (a context runs one computation at a time)
@@ -868,6 +870,7 @@ int check_device_error(og_engine *e) {
   const uint32_t err = *e->err_h;
   if (!err) return OG_OK;
   if (err & kErrLookback) return fail(OG_E_TIMEOUT, "frontier compaction look-back wait gave up");
+  if (err & kErrBarrier) return fail(OG_E_TIMEOUT, "staged round: a slot wait gave up");
   return fail(OG_E_DEVICE, "kernel reported an out-of-range index (flags 0x%x)", err);
 }
 
@@ -965,25 +968,33 @@ int launch_relax(og_engine *e, const RoundOps &ro, const LbsArgs &a, Src src, ui
   return OG_OK;
 }
 
-// One staged step (k_stage_step): gathers chunk `g` into buffer gbuf and relaxes
-// chunk `r` out of the other one; either may be absent (pos_begin == pos_end).
+// The ring of a staged round (k_stage_round) over both staging buffers, cleared
+// on `s`.
+int stage_ring(og_engine *e, StageRing *g, cudaStream_t s) {
+  const uint64_t half = e->plan.chunk_edges / kTile;
+  g->state = e->ring_d + kRingPad;
+  g->ticket = e->ring_d;
+  g->slots = (uint32_t)std::min<uint64_t>(2 * half, kRingSlots);
+  g->half = (uint32_t)std::min<uint64_t>(half, kRingSlots);
+  CK(cudaMemsetAsync(e->ring_d, 0, 4ull * (kRingPad + g->slots), s));
+  return OG_OK;
+}
+
+// A staged round of the dynamic list `a`.
 template <class K>
-int launch_stage_step(og_engine *e, const RoundOps &ro, const LbsArgs &g, int gbuf, const LbsArgs &r, uint32_t *next,
-                      cudaStream_t s) {
-  const unsigned ng = lbs_grid(g.pos_begin, g.pos_end), nr = lbs_grid(r.pos_begin, r.pos_end);
-  const auto src = K::stage(e, gbuf ^ 1);
-  const auto dst = K::stage_dst(e, gbuf);
+int launch_stage_round(og_engine *e, const RoundOps &ro, const LbsArgs &a, uint32_t *next, cudaStream_t s) {
+  StageRing ring;
+  RC(stage_ring(e, &ring, s));
+  const unsigned grid = 2 * lbs_grid(0, a.total);
+  auto launch = [&](auto op) {
+    k_stage_round<<<grid, kThreads, 0, s>>>(a, K::host(e), K::stage_dst(e, 0), K::stage_dst(e, 1), K::stage(e, 0),
+                                            K::stage(e, 1), e->plan.chunk_edges, op, ring);
+  };
   if constexpr (std::is_same<typename K::Src, SrcU>::value) {
-    if (ro.algo == OG_ALGO_BFS) {
-      BfsOp op{e->bm[2], next, e->value_d, e->err_d, e->V, ro.level + 1};
-      k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
-    } else {
-      MinOp<false> op{e->value_d, next, e->err_d, e->V};
-      k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
-    }
+    if (ro.algo == OG_ALGO_BFS) launch(BfsOp{e->bm[2], next, e->value_d, e->err_d, e->V, ro.level + 1});
+    else launch(MinOp<false>{e->value_d, next, e->err_d, e->V});
   } else {
-    MinOp<true> op{e->value_d, next, e->err_d, e->V};
-    k_stage_step<<<ng + nr, kThreads, 0, s>>>(g, K::host(e), dst, ng, r, src, op);
+    launch(MinOp<true>{e->value_d, next, e->err_d, e->V});
   }
   e->launches++;
   return OG_OK;
@@ -1038,8 +1049,7 @@ struct NoStage {};
 // as one interleaved kernel (direct mode with both regions non-empty): the
 // static tiles then overlap the link-bound dynamic ones instead of taking the
 // SMs first.  Its time is counted as dynamic-region time.
-// `stage_fn(g, gbuf, r)`, when given, launches a staged step: gather of chunk g
-// into buffer gbuf beside the relax of chunk r (empty: none) out of the other.
+// `stage_fn(a)`, when given, launches a staged round of the dynamic list a.
 template <class K, class StaticFn, class DynFn, class PairFn = NoPair, class StageFn = NoStage>
 int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynFn dyn_fn,
                 PairFn pair_fn = PairFn(), StageFn stage_fn = StageFn()) {
@@ -1077,12 +1087,8 @@ int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynF
         cudaEvent_t g0, g1;
         RC(gather_events(e, tm.pend_g, &g0, &g1));
         CK(cudaEventRecord(g0, e->s_dyn));
-        for (uint64_t c = 0; c <= nch; c++) {
-          const uint64_t gb = std::min(c * C, cd.total), ge = std::min(gb + C, cd.total);
-          const uint64_t rb = c ? (c - 1) * C : 0, re = c ? std::min(rb + C, cd.total) : 0;
-          RC(stage_fn(lbs_args(e, 1, gb, ge, true, e->g->E), (int)(c & 1), lbs_args(e, 1, rb, re, false, C)));
-          if (c + 1 == nch) CK(cudaEventRecord(g1, e->s_dyn));  // the last step that gathers
-        }
+        RC(stage_fn(lbs_args(e, 1, 0, cd.total, true, e->g->E)));
+        CK(cudaEventRecord(g1, e->s_dyn));
         tm.pend_g++;
       } else
       for (uint64_t c = 0; c < nch; c++) {
@@ -1270,9 +1276,9 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
     auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
       return launch_relax_pair(e, ro, a0, s0, a1, s1, next, ps);
     };
-    auto gfn = [&](const LbsArgs &ga, int gbuf, const LbsArgs &ra) {
+    auto gfn = [&](const LbsArgs &a) {
       if constexpr (K::kFrag) return (int)OG_OK;  // direct mode only
-      else return launch_stage_step<K>(e, ro, ga, gbuf, ra, next, e->s_dyn);
+      else return launch_stage_round<K>(e, ro, a, next, e->s_dyn);
     };
     RC((run_regions<K>(e, st, tm, sfn, dfn, pfn, gfn)));
     if constexpr (K::kFrag) e->frag->since += e->counts_h[1].total;
@@ -2198,14 +2204,13 @@ int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
       return pr_contiguous(e, 1) ? launch_pr_pull<true>(e, a, src, pr_args(e, 1, nullptr), ds)
                                  : launch_pr_pull<false>(e, a, src, pr_args(e, 1, nullptr), ds);
   };
-  auto gfn = [&](const LbsArgs &g, int gbuf, const LbsArgs &r) {
-    const unsigned ng = lbs_grid(g.pos_begin, g.pos_end), nr = lbs_grid(r.pos_begin, r.pos_end);
-    // a staging buffer: columns from position pos_begin on, as 32-bit records
-    PrArgs q = pr_args(e, 1, nullptr);
-    q.base = 0ull - r.pos_begin;
-    q.nwords = r.edge_bound;
-    k_stage_step_pr<<<ng + nr, kThreads, pr_smem_bytes(true, 32), e->s_dyn>>>(
-        g, EKU::host(e), EKU::stage_dst(e, gbuf), ng, r, SrcP<false>{e->stage_col[gbuf ^ 1], 32u, 32u, 0u}, q);
+  auto gfn = [&](const LbsArgs &a) {
+    StageRing ring;
+    RC(stage_ring(e, &ring, e->s_dyn));
+    auto buf = [&](int b) { return SrcP<false>{e->stage_col[b], 32u, 32u, 0u}; };
+    k_stage_round_pr<<<2 * lbs_grid(0, a.total), kThreads, pr_smem_bytes(true, 32), e->s_dyn>>>(
+        a, EKU::host(e), EKU::stage_dst(e, 0), EKU::stage_dst(e, 1), buf(0), buf(1), e->plan.chunk_edges,
+        pr_args(e, 1, nullptr), ring);
     e->launches++;
     return (int)OG_OK;
   };

@@ -39,6 +39,7 @@ constexpr uint32_t kErrVertex = 4u;      // column >= V
 constexpr uint32_t kErrTileMap = 8u;     // LBS tile map inconsistent
 
 constexpr uint32_t kSpinLimit = 1u << 24;
+constexpr uint32_t kErrBarrier = 16u;  // a bounded wait within a launch gave up
 
 // Nanosecond global timer (the same clock on every SM).
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -881,6 +882,10 @@ template <class T, class = void>
 struct HasProbeVal : std::false_type {};
 template <class T>
 struct HasProbeVal<T, std::void_t<decltype(T::kProbeVal)>> : std::true_type {};
+template <class T, class = void>
+struct HasCommit : std::false_type {};
+template <class T>
+struct HasCommit<T, std::void_t<decltype(&T::commit)>> : std::true_type {};
 
 // Runs `body(lo, hi, j0)` over positions [plo, phi) of tile k: once, or in parts
 // of kThreads positions when the tile holds more than kLocal vertices.  In
@@ -1007,6 +1012,8 @@ __device__ __forceinline__ void lbs_tile(const LbsArgs &a, const Src &src, const
         ev[it] = src.at(sh.cb[l], x);
       }
     }
+    if constexpr (HasCommit<Op>::value)
+      if (!op.commit()) return;
     // Probe phase: every target's current state is read before the first
     // atomic, so the eight random reads of a thread overlap (in program order
     // the compiler may not lift a load above an earlier atomic).  A probe is
@@ -1069,14 +1076,99 @@ __global__ void __launch_bounds__(kThreads, 5) k_lbs_pair(LbsArgs a0, Src0 s0, L
   else lbs_tile(a1, s1, op, sh, a1.pos_begin / kTile + pt.t);
 }
 
-// The dynamic-region gather as an edge op: positions of a chunk go to a staging
-// buffer whose entry 0 is position `base`.
+// A staged round in one launch.  The two staging buffers are a ring of tile
+// slots: position tile t is gathered into slot t % slots and relaxed out of it,
+// one CTA per step.  state[slot] counts the slot's steps: use u of a slot is
+// gathered when it reads 2u and relaxed when it reads 2u + 1.  CTAs take their
+// step from a ticket: first `lead` gathers, then gather t + lead and relax t in
+// turn, so a step waits only for steps with earlier tickets, which running
+// CTAs hold; the whole grid need not be resident.  With lead = slots / 2 both
+// waits are `slots` steps back and rarely last (5/8 to 7/8 of slots measured the same).
+// One launch per chunk (gather of chunk c beside the relax of c - 1) was bound
+// by a wave's latency per chunk and the gap between launches: 15 + 3 us for
+// 1.65 MB that the link moves in 8; delta PageRank of 777777 vertices took 4.24
+// ms so and takes 3.31 now (a round of 18.4 MB: 127 us, of them 87 link), BFS
+// of 2^20 vertices with chunks of 55296 edges 1.95 (8.5 with two streams and an
+// event each way per chunk).  A grid of 2 to 6 CTAs per SM that loop over the
+// tickets was slower (4.19 to 3.41 ms).
+constexpr uint32_t kRingSlots = 2048;  // most slots in use: 4 M positions, more than are ever in flight
+constexpr uint32_t kRingPad = 32;      // words before them: the ticket's cache line
+struct StageRing {
+  uint32_t *state, *ticket;  // zeroed before the launch
+  uint32_t slots, half;      // half: slots of buffer 0
+};
+struct StageStep {
+  uint64_t tile, base;  // base: position minus buffer entry (mod 2^64)
+  uint32_t slot, want;  // want: the state this step waits for; odd: relax
+  uint32_t buf, ready;
+};
+// This CTA's step, from the next ticket.
+__device__ __forceinline__ void stage_take(const StageRing &g, uint64_t ntiles, StageStep &step) {
+  if (threadIdx.x == 0) {
+    const uint64_t i = atomicAdd(g.ticket, 1u), lead = min((uint64_t)(g.slots / 2), ntiles);
+    const uint64_t j = i - lead, pairs = ntiles - lead;  // j: valid for i >= lead
+    StageStep x;
+    bool relax = false;
+    if (i < lead) {
+      x.tile = i;
+    } else if (j < 2 * pairs) {
+      relax = j & 1u;
+      x.tile = (j >> 1) + (relax ? 0 : lead);
+    } else {
+      relax = true;
+      x.tile = j - pairs;
+    }
+    const uint32_t use = (uint32_t)x.tile / g.slots;
+    x.slot = (uint32_t)x.tile - use * g.slots;
+    x.want = 2 * use + relax;
+    x.buf = x.slot >= g.half;
+    x.base = (x.tile - (x.slot - x.buf * g.half)) * kTile;
+    x.ready = 0;
+    step = x;
+  }
+  __syncthreads();
+}
+// Thread 0: waits for the step's slot, a bounded number of polls (an expired
+// wait sets kErrBarrier, which ends the waits of the others).  The polls are
+// relaxed and one fence follows: it also drops lines of the slot's earlier
+// use from L1.
+__device__ __forceinline__ void stage_wait(const StageRing &g, StageStep &x, uint32_t *err) {
+  for (uint32_t spins = 0; ld_relaxed(g.state + x.slot) != x.want;) {
+    if (++spins > kSpinLimit || ((spins & 255u) == 0 && (ld_relaxed(err) & kErrBarrier))) {
+      atomicOr(err, kErrBarrier);
+      return;
+    }
+    __nanosleep(spins < 256 ? 20 : 200);
+  }
+  __threadfence();
+  x.ready = 1;
+}
+// All threads: waits for the slot; false: gave up.
+__device__ __forceinline__ bool stage_ready(const StageRing &g, StageStep &x, uint32_t *err) {
+  if (threadIdx.x == 0 && !x.ready) stage_wait(g, x, err);
+  __syncthreads();
+  return x.ready != 0;
+}
+__device__ __forceinline__ void stage_post(const StageRing &g, StageStep &x, uint32_t *err) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (!x.ready) stage_wait(g, x, err);  // a gather that stopped before its stores
+  if (x.ready) st_release(g.state + x.slot, x.want + 1);
+}
+
+// The gather of a staged round as an edge op: position pos goes to entry
+// pos - base of a staging buffer.  The slot is waited for after the link reads
+// have been issued, so a step holds it for its stores alone.
 template <class Dst>
 struct GatherOp {
   using Val = uint32_t;
   static constexpr bool kNeedVal = false;
   Dst stage;
   uint64_t base;
+  const StageRing *ring;
+  StageStep *step;  // shared memory
+  uint32_t *err;
+  __device__ __forceinline__ bool commit() const { return stage_ready(*ring, *step, err); }
   __device__ uint32_t src_val(uint32_t) const { return 0; }
   using Probe = uint32_t;
   template <class Edge>
@@ -1089,22 +1181,27 @@ struct GatherOp {
   }
 };
 
-// One step of a staged round: the first ng CTAs gather chunk c (list g) while
-// the others relax chunk c - 1 (list r) out of the other staging buffer.  With
-// two streams and an event in each direction per chunk the same work took a
-// dozen host calls a chunk, 40 us of them; now launch order is the only
-// synchronisation.
 template <class PSrc, class Dst, class Src, class Op>
-__global__ void __launch_bounds__(kThreads, 5) k_stage_step(LbsArgs g, PSrc ps, Dst dst, uint32_t ng, LbsArgs r,
-                                                            Src src, Op op) {
+__global__ void __launch_bounds__(kThreads, 5) k_stage_round(const __grid_constant__ LbsArgs a, PSrc ps, Dst d0, Dst d1,
+                                                             Src s0, Src s1, uint64_t cap, Op op,
+                                                             const __grid_constant__ StageRing ring) {
   __shared__ union {
     LbsSh<GatherOp<Dst>> gather;
     LbsSh<Op> relax;
   } sh;
-  if (blockIdx.x < ng)
-    lbs_tile(g, ps, GatherOp<Dst>{dst, g.pos_begin}, sh.gather, g.pos_begin / kTile + blockIdx.x);
-  else
-    lbs_tile(r, src, op, sh.relax, r.pos_begin / kTile + blockIdx.x - ng);
+  __shared__ StageStep x;
+  stage_take(ring, (a.total + kTile - 1) / kTile, x);
+  if (x.want & 1u) {
+    if (!stage_ready(ring, x, a.err)) return;
+    LbsArgs r = a;  // positions of a staging buffer instead of CSR offsets
+    r.off = nullptr;
+    r.stage_base = x.base;
+    r.edge_bound = cap;
+    lbs_tile(r, x.buf ? s1 : s0, op, sh.relax, x.tile);
+  } else {
+    lbs_tile(a, ps, GatherOp<Dst>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh.gather, x.tile);
+  }
+  stage_post(ring, x, a.err);
 }
 
 template <int MULT>
@@ -1618,15 +1715,28 @@ __global__ void __launch_bounds__(kThreads, 6) k_pr_pull(LbsArgs a, Src src, PrA
   pr_tile<kDense>(a, src, p, a.pos_begin / kTile + blockIdx.x);
 }
 
-// The staged step of a PageRank round (see k_stage_step).
+// A staged PageRank round (see k_stage_round): the buffers hold columns as
+// 32-bit records.
 template <class PSrc, class Dst, class Src>
-__global__ void __launch_bounds__(kThreads, 6) k_stage_step_pr(LbsArgs g, PSrc ps, Dst dst, uint32_t ng, LbsArgs r,
-                                                               Src src, PrArgs p) {
+__global__ void __launch_bounds__(kThreads, 6) k_stage_round_pr(const __grid_constant__ LbsArgs a, PSrc ps, Dst d0,
+                                                                Dst d1, Src s0, Src s1, uint64_t cap,
+                                                                const __grid_constant__ PrArgs p,
+                                                                const __grid_constant__ StageRing ring) {
   __shared__ LbsSh<GatherOp<Dst>> sh;
-  if (blockIdx.x < ng)
-    lbs_tile(g, ps, GatherOp<Dst>{dst, g.pos_begin}, sh, g.pos_begin / kTile + blockIdx.x);
-  else
-    pr_tile<true>(r, src, p, r.pos_begin / kTile + blockIdx.x - ng);
+  __shared__ StageStep x;
+  stage_take(ring, (a.total + kTile - 1) / kTile, x);
+  if (x.want & 1u) {
+    if (!stage_ready(ring, x, a.err)) return;
+    LbsArgs r = a;
+    PrArgs q = p;
+    r.edge_bound = cap;
+    q.base = 0ull - x.base;
+    q.nwords = cap;
+    pr_tile<true>(r, x.buf ? s1 : s0, q, x.tile);
+  } else {
+    lbs_tile(a, ps, GatherOp<Dst>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh, x.tile);
+  }
+  stage_post(ring, x, a.err);
 }
 
 // Both regions' pull sums in one launch, static and dynamic tiles interleaved
