@@ -1143,7 +1143,7 @@ int compact_round(og_engine *e, const uint32_t *cur, og_stats &st, Timing &tm, u
   CK(cudaEventRecord(e->ev_cd, e->s_dyn));
   CK(cudaStreamWaitEvent(e->s_dyn, e->ev_cs, 0));
   CK(cudaMemcpyAsync(e->counts_h, e->counts_d, 3 * sizeof(Counts), cudaMemcpyDeviceToHost, e->s_dyn));
-  CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, e->s_dyn));
+  CK(cudaMemcpyAsync(e->err_h, e->err_d, 8, cudaMemcpyDeviceToHost, e->s_dyn));  // and active_d
   CK(cudaStreamSynchronize(e->s_dyn));
   collect_timing(e, tm, &st);
   float ms;
@@ -2233,9 +2233,13 @@ int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
   e->launches += 2;
   CK(cudaGetLastError());
   Timing tm;
-  for (int round = 0; max_rounds <= 0 || round < max_rounds; round++) {
-    uint64_t n = 0;
-    RC(compact_round(e, cur, st, tm, &n));
+  // The compaction of the next round is enqueued behind the update, and one wait
+  // a round reads its counts and whether anything is active; a wait after
+  // the update as well left the device idle twice a round (777777 vertices
+  // staged, 17 rounds: 3.33 ms; 3.09 now).
+  uint64_t n = 0;
+  RC(compact_round(e, cur, st, tm, &n));
+  for (int round = 1;; round++) {
     st.iterations++;
     st.frontier_sum += n;
     st.static_vertices += e->counts_h[0].n;
@@ -2245,10 +2249,14 @@ int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
         cur, next, e->nwords, (float *)e->value_d, e->contrib_d, e->sum_d, e->outdeg_d, thresh,
         e->active_d);
     e->launches++;
-    CK(cudaMemcpyAsync(e->err_h, e->err_d, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    RC(check_device_error(e));
+    if (round == max_rounds) {
+      CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      RC(check_device_error(e));
+      break;
+    }
     std::swap(cur, next);
+    RC(compact_round(e, cur, st, tm, &n));
     if (e->err_h[1] == 0) break;
   }
   CK(cudaStreamSynchronize(s));
