@@ -71,6 +71,9 @@ struct FragState {
   og_fragment_stats st{};
 };
 
+// Counts-sized (16-byte) parts of an engine's control block (og_engine::counts_d).
+constexpr uint32_t kControlCounts = 5;
+
 struct og_engine {
   og_graph *g = nullptr;
   og_config cfg{};
@@ -83,7 +86,7 @@ struct og_engine {
   uint64_t nwords = 0;
 
   cudaStream_t s_main = nullptr, s_dyn = nullptr, s_gat = nullptr;
-  cudaEvent_t ev_round = nullptr, ev_cs = nullptr, ev_cd = nullptr, ev_dyn_done = nullptr;
+  cudaEvent_t ev_round = nullptr, ev_cd = nullptr, ev_dyn_done = nullptr;
   cudaEvent_t ev_gat[2] = {nullptr, nullptr}, ev_rel[2] = {nullptr, nullptr};
   cudaEvent_t t_s0 = nullptr, t_s1 = nullptr, t_d0 = nullptr;
   std::vector<cudaEvent_t> t_gat;  // start/end pairs around each gather launch
@@ -106,6 +109,8 @@ struct og_engine {
   Lookback lb[2]{};
   uint32_t lb_tiles = 0;
   // counts of the two regions followed by their two far keys (u64), one D2H
+  // What the host reads after a compaction, in one copy: Counts[2], u64 far
+  // key[2], 4 error words (err_d, active_d), 4 mask words (sb_masks).
   Counts *counts_d = nullptr, *counts_h = nullptr;
   uint32_t epoch = 0;  // look-back epoch of the last compaction launch
   uint32_t *err_d = nullptr, *err_h = nullptr;
@@ -486,9 +491,8 @@ void destroy(og_engine *e) {
   if (e->pmisc_h) cudaFreeHost(e->pmisc_h);
   if (e->graph) cudaGraphExecDestroy(e->graph);
   if (e->rounds_h) cudaFreeHost(e->rounds_h);
-  if (e->err_h) cudaFreeHost(e->err_h);
   if (e->prl_h) cudaFreeHost(e->prl_h);
-  cudaEvent_t evs[] = {e->ev_round, e->ev_cs, e->ev_cd, e->ev_dyn_done, e->ev_gat[0], e->ev_gat[1],
+  cudaEvent_t evs[] = {e->ev_round, e->ev_cd, e->ev_dyn_done, e->ev_gat[0], e->ev_gat[1],
                        e->ev_rel[0], e->ev_rel[1], e->t_s0, e->t_s1, e->t_d0};
   for (auto ev : evs)
     if (ev) cudaEventDestroy(ev);
@@ -525,7 +529,7 @@ int create_query_state(og_engine *e) {
   CK(cudaStreamCreateWithPriority(&e->s_main, cudaStreamNonBlocking, prio));
   CK(cudaStreamCreateWithPriority(&e->s_dyn, cudaStreamNonBlocking, prio));
   CK(cudaStreamCreateWithPriority(&e->s_gat, cudaStreamNonBlocking, prio));
-  cudaEvent_t *evs[] = {&e->ev_round, &e->ev_cs, &e->ev_cd, &e->ev_dyn_done, &e->ev_gat[0],
+  cudaEvent_t *evs[] = {&e->ev_round, &e->ev_cd, &e->ev_dyn_done, &e->ev_gat[0],
                         &e->ev_gat[1], &e->ev_rel[0], &e->ev_rel[1], &e->t_s0, &e->t_s1, &e->t_d0};
   for (auto ev : evs) CK(cudaEventCreate(ev));
   RC(dalloc(e, &e->value_d, V + 1));
@@ -552,15 +556,16 @@ int create_query_state(og_engine *e) {
     // epochs start at 1: zeroed slots are "empty"
     CK(cudaMemsetAsync(e->lb[r].slot, 0, sizeof(ulonglong2) * (e->lb_tiles + 1), e->s_main));
   }
-  RC(dalloc(e, &e->counts_d, 3));  // Counts[2] + u64 far key[2]
-  CK(cudaMemsetAsync(e->counts_d, 0, 3 * sizeof(Counts), e->s_main));
-  RC(dalloc(e, &e->err_d, 4));
+  RC(dalloc(e, &e->counts_d, 64));  // 1 KiB
+  CK(cudaMemsetAsync(e->counts_d, 0, kControlCounts * sizeof(Counts), e->s_main));
+  e->err_d = (uint32_t *)(e->counts_d + 3);
   e->active_d = e->err_d + 1;
+  e->sb_masks = (uint32_t *)(e->counts_d + 4);
   RC(dalloc(e, &e->sum64_d, 3ull * e->sms * 8 + 4));
-  CK(cudaMallocHost(&e->counts_h, 3 * sizeof(Counts)));
+  CK(cudaMallocHost(&e->counts_h, kControlCounts * sizeof(Counts)));
+  e->err_h = (uint32_t *)(e->counts_h + 3);
   RC(dalloc(e, (char **)&e->rounds_d, sizeof(RoundsState)));
   CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState)));
-  CK(cudaMallocHost(&e->err_h, 4 * sizeof(uint32_t)));
   CK(cudaMallocHost(&e->prl_h, sizeof(PrLoop)));
   if (P.chunk_edges && !(e->cfg.flags & OG_CFG_DIRECT)) {
     for (int b = 0; b < 2; b++) {
@@ -602,7 +607,6 @@ int create_query_state(og_engine *e) {
       e->sb_dist = (uint32_t *)e->arena;
       e->sb_pend = e->sb_dist + (V + 1) * e->sb_ks;
       e->sb_lmask = e->sb_pend + (V + 1);  // list_cap[0] + list_cap[1] <= V + 1 entries
-      RC(dalloc(e, &e->sb_masks, 4));
       RC(dalloc(e, &e->sb_io_d, 128));
       RC(dalloc(e, &e->sb_ck_d, 2 * kSbMaxSources));
       CK(cudaMallocHost(&e->sb_io_h, 128 * sizeof(uint32_t)));
@@ -811,13 +815,11 @@ uint32_t compact_tile_words(uint32_t words, uint32_t max_tiles) {
   return tw;
 }
 
-int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint32_t ve,
-                   cudaStream_t s, const SplitArgs &sp = SplitArgs()) {
-  if (ve <= vb) {  // empty region: no kernel writes its counts
-    CK(cudaMemsetAsync(e->counts_d + r, 0, sizeof(Counts), s));
-    return OG_OK;
-  }
+CompactArgs compact_args(og_engine *e, int r, const uint32_t *bits, const SplitArgs &sp) {
+  const uint32_t vb = r ? e->Vs : 0, ve = r ? e->V : e->Vs;
   CompactArgs a{};
+  a.counts = e->counts_d + r;
+  if (ve <= vb) return a;  // empty region
   a.bits = bits;
   a.v_begin = vb;
   a.v_end = ve;
@@ -829,7 +831,6 @@ int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint3
   a.list = e->list_d[r];
   a.pref = e->pref_d[r];
   a.tile_first = e->tile_d[r];
-  a.counts = e->counts_d + r;
   a.lb = e->lb[r];
   a.err = e->err_d;
   a.list_cap = e->list_cap[r];
@@ -841,9 +842,30 @@ int launch_compact(og_engine *e, int r, const uint32_t *bits, uint32_t vb, uint3
   a.far_key = (unsigned long long *)(e->counts_d + 2) + r;
   a.clear_bits = sp.clear_bits;
   a.epoch = e->epoch;
-  if (a.ntiles + 1 > e->lb_tiles) return fail(OG_E_STATE, "compaction scratch too small");
-  k_compact<<<a.ntiles, kThreads, 0, s>>>(a);
+  return a;
+}
+
+// Both regions in one launch.
+template <class Args, class Kernel>
+int launch_compact(og_engine *e, const CompactPair<Args> &p, Kernel kernel) {
+  const uint32_t n0 = p.r[0].ntiles, n1 = p.r[1].ntiles;
+  if (std::max(n0, n1) + 1 > e->lb_tiles) return fail(OG_E_STATE, "compaction scratch too small");
+  if (n0 + n1) {
+    kernel<<<n0 + n1, kThreads, 0, e->s_main>>>(p);
+    e->launches++;
+  } else {
+    CK(cudaMemsetAsync(e->counts_d, 0, 2 * sizeof(Counts), e->s_main));
+  }
+  return OG_OK;
+}
+
+// Waits for a compaction and what is enqueued before it; counts, error words
+// and multi-source masks come to the host in one copy.
+int compact_wait(og_engine *e) {
+  static_assert(sizeof(Counts) == sizeof(uint4), "one word per entry");
+  k_publish<<<1, 32, 0, e->s_main>>>((const uint4 *)e->counts_d, (uint4 *)e->counts_h, kControlCounts);
   e->launches++;
+  CK(cudaStreamSynchronize(e->s_main));
   return OG_OK;
 }
 
@@ -1136,15 +1158,10 @@ int compact_round(og_engine *e, const uint32_t *cur, og_stats &st, Timing &tm, u
     e->epoch = 1;
   }
   CK(cudaEventRecord(e->ev_round, e->s_main));
-  RC(launch_compact(e, 0, cur, 0, e->Vs, e->s_main, sp));
-  CK(cudaEventRecord(e->ev_cs, e->s_main));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-  RC(launch_compact(e, 1, cur, e->Vs, e->V, e->s_dyn, sp));
-  CK(cudaEventRecord(e->ev_cd, e->s_dyn));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_cs, 0));
-  CK(cudaMemcpyAsync(e->counts_h, e->counts_d, 3 * sizeof(Counts), cudaMemcpyDeviceToHost, e->s_dyn));
-  CK(cudaMemcpyAsync(e->err_h, e->err_d, 8, cudaMemcpyDeviceToHost, e->s_dyn));  // and active_d
-  CK(cudaStreamSynchronize(e->s_dyn));
+  const CompactPair<CompactArgs> p{{compact_args(e, 0, cur, sp), compact_args(e, 1, cur, sp)}};
+  RC(launch_compact(e, p, k_compact));
+  CK(cudaEventRecord(e->ev_cd, e->s_main));
+  RC(compact_wait(e));
   collect_timing(e, tm, &st);
   float ms;
   if (cudaEventElapsedTime(&ms, e->ev_round, e->ev_cd) == cudaSuccess) st.ms_compact += ms;
@@ -1282,7 +1299,6 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
     };
     RC((run_regions<K>(e, st, tm, sfn, dfn, pfn, gfn)));
     if constexpr (K::kFrag) e->frag->since += e->counts_h[1].total;
-    CK(cudaStreamWaitEvent(e->s_main, e->ev_cd, 0));
     CK(cudaMemsetAsync(cur, 0, 4 * e->nwords, e->s_main));
     std::swap(cur, next);
     ro.level++;
@@ -1456,7 +1472,6 @@ int run_batch(og_engine *e, const uint32_t *srcs, uint32_t n, uint32_t *out, uin
                                                                  e->hist_d, depth_d, V, level + 1);
     e->launches++;
     CK(cudaMemcpyAsync(e->hist_h, e->hist_d, 64 * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamWaitEvent(s, e->ev_cd, 0));
     CK(cudaMemsetAsync(cur_any, 0, 4 * e->nwords, s));
     CK(cudaMemsetAsync(cur, 0, 8 * (V + 1), s));
     CK(cudaStreamSynchronize(s));
@@ -1600,7 +1615,6 @@ int bb_step_impl(og_engine *e, uint64_t *pending, bool *done, og_stats &st, Timi
                                                                e->bb_io_d + 128);
   e->launches++;
   CK(cudaMemcpyAsync(e->hist_h, e->hist_d, 64 * 8, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamWaitEvent(s, e->ev_cd, 0));
   CK(cudaMemsetAsync(cur_any, 0, 4 * e->nwords, s));
   CK(cudaMemsetAsync(cur, 0, 8 * (V + 1), s));
   CK(cudaStreamSynchronize(s));
@@ -1879,15 +1893,13 @@ int run_batch_persist(og_engine *e, const uint32_t *srcs, uint32_t n, void *out,
 
 // ------------------------------------------------------------ multi-source SSSP
 
-// Launches k_compact_sb for region r over the active (scan_wait = false) or
+// k_compact_sb's arguments for region r over the active (scan_wait = false) or
 // waiting bitmap.
-int launch_compact_sb(og_engine *e, int r, uint32_t *bits, uint32_t vb, uint32_t ve, bool scan_wait,
-                      cudaStream_t s) {
-  if (ve <= vb) {
-    CK(cudaMemsetAsync(e->counts_d + r, 0, sizeof(Counts), s));
-    return OG_OK;
-  }
+SbCompactArgs compact_args_sb(og_engine *e, int r, uint32_t *bits, bool scan_wait) {
+  const uint32_t vb = r ? e->Vs : 0, ve = r ? e->V : e->Vs;
   SbCompactArgs a{};
+  a.counts = e->counts_d + r;
+  if (ve <= vb) return a;  // empty region
   a.bits = bits;
   a.wait = e->bm[2];
   a.v_begin = vb;
@@ -1901,7 +1913,6 @@ int launch_compact_sb(og_engine *e, int r, uint32_t *bits, uint32_t vb, uint32_t
   a.pref = e->pref_d[r];
   a.tile_first = e->tile_d[r];
   a.lmask = e->sb_lmask + (e->list_d[r] - e->list_d[0]);
-  a.counts = e->counts_d + r;
   a.lb = e->lb[r];
   a.err = e->err_d;
   a.list_cap = e->list_cap[r];
@@ -1914,10 +1925,7 @@ int launch_compact_sb(og_engine *e, int r, uint32_t *bits, uint32_t vb, uint32_t
   a.far_key = (unsigned long long *)(e->counts_d + 2) + r;
   a.masks = e->sb_masks;
   a.epoch = e->epoch;
-  if (a.ntiles + 1 > e->lb_tiles) return fail(OG_E_STATE, "compaction scratch too small");
-  k_compact_sb<<<a.ntiles, kThreads, 0, s>>>(a);
-  e->launches++;
-  return OG_OK;
+  return a;
 }
 
 // Clears the batch: no slot in use, no vertex active or waiting.
@@ -1998,21 +2006,16 @@ int sb_round(og_engine *e, og_stats &st, Timing &tm, uint32_t *pending, bool *do
   // waiting set is scanned again
   CK(cudaMemsetAsync(e->sb_masks, 0, adv ? 8 : 4, e->s_main));
   CK(cudaEventRecord(e->ev_round, e->s_main));
-  RC(launch_compact_sb(e, 0, bits, 0, e->Vs, adv, e->s_main));
-  CK(cudaEventRecord(e->ev_cs, e->s_main));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
-  RC(launch_compact_sb(e, 1, bits, e->Vs, e->V, adv, e->s_dyn));
-  CK(cudaEventRecord(e->ev_cd, e->s_dyn));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_cs, 0));
-  CK(cudaMemcpyAsync(e->counts_h, e->counts_d, 3 * sizeof(Counts), cudaMemcpyDeviceToHost, e->s_dyn));
-  CK(cudaMemcpyAsync(e->sb_io_h + 64, e->sb_masks, 8, cudaMemcpyDeviceToHost, e->s_dyn));
-  CK(cudaMemcpyAsync(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost, e->s_dyn));
-  CK(cudaStreamSynchronize(e->s_dyn));
+  const CompactPair<SbCompactArgs> p{{compact_args_sb(e, 0, bits, adv), compact_args_sb(e, 1, bits, adv)}};
+  RC(launch_compact(e, p, k_compact_sb));
+  CK(cudaEventRecord(e->ev_cd, e->s_main));
+  RC(compact_wait(e));
   collect_timing(e, tm, &st);
   float ms;
   if (cudaEventElapsedTime(&ms, e->ev_round, e->ev_cd) == cudaSuccess) st.ms_compact += ms;
   RC(check_device_error(e));
-  *pending = e->sb_io_h[64] | e->sb_io_h[65];
+  const uint32_t *masks = (const uint32_t *)(e->counts_h + 4);
+  *pending = masks[0] | masks[1];
   const uint32_t fm = std::min(far_of(e, 0), far_of(e, 1));
   e->sb_far_min = adv ? fm : std::min(e->sb_far_min, fm);
   const uint64_t n = (uint64_t)e->counts_h[0].n + e->counts_h[1].n;
@@ -2059,7 +2062,6 @@ int sb_round(og_engine *e, og_stats &st, Timing &tm, uint32_t *pending, bool *do
     return (int)OG_OK;
   };
   RC((run_regions<K>(e, st, tm, sfn, launch, pfn)));
-  CK(cudaStreamWaitEvent(e->s_main, e->ev_cd, 0));
   CK(cudaGetLastError());
   return OG_OK;
 }
@@ -2312,7 +2314,6 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
     const uint32_t *done = &e->prl_d->done;
     const LbsArgs a0 = lbs_args(e, 0, 0, c0.total, true, e->plan.static_edges);
     const LbsArgs a1 = lbs_args(e, 1, 0, c1.total, true, e->g->E);
-    CK(cudaStreamWaitEvent(s, e->ev_cd, 0));  // the dynamic region's list
     uint32_t launched = 0, batch = std::max<uint32_t>(1, e->pr_hint);
     while (launched < (uint32_t)max_iter) {
       batch = std::min<uint32_t>(batch, (uint32_t)max_iter - launched);
@@ -2723,7 +2724,6 @@ int run_cc_uf(og_engine *e, og_stats &st) {
       return (int)OG_OK;
     };
     RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
-    CK(cudaStreamWaitEvent(e->s_main, e->ev_cd, 0));
   }
   if (n) {  // nothing was linked since the last compression otherwise
     k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
@@ -3145,7 +3145,7 @@ void compact_launch(const uint32_t *bits, uint32_t v_begin, uint32_t v_end, cons
   a.far_key = nullptr;
   a.clear_bits = nullptr;
   a.epoch = 1;  // the caller's scratch is zeroed before every launch
-  k_compact<<<a.ntiles, kThreads, 0, s>>>(a);
+  k_compact<<<a.ntiles, kThreads, 0, s>>>(CompactPair<CompactArgs>{{a, CompactArgs{}}});
 }
 
 // Look-back scratch of `ntiles` tiles: a slot each, then the ticket.

@@ -136,8 +136,9 @@ struct SbSel {
   }
 };
 
-__global__ void __launch_bounds__(kThreads, 4) k_compact_sb(SbCompactArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) k_compact_sb(const __grid_constant__ CompactPair<SbCompactArgs> p) {
   __shared__ CompactShared sh;
+  const SbCompactArgs &a = compact_region(p);
   SbSel sel{a, 0xffffffffu, 0u, 0u};
   compact_tile(a, sel, sh);
 }
