@@ -406,9 +406,9 @@ def run_ours(args, rank, world, local):
     launches = sum(s["launches"] for s in stats)
     peaks = measured_peaks()
     # Kernel-level timing of the dominant kernel: the same queries again with
-    # the relax timer on, so that every relax launch of the device-driven
-    # rounds is bracketed by two stamp kernels reading the GPU's global timer
-    # (og_stats.ms_relax); the timed queries above run without them.  The
+    # the relax timer on, so that the relax phase of every device-driven round
+    # is timed with the GPU's global timer (og_stats.ms_relax); the timed
+    # queries above run without it.  The
     # host-driven loop is timed beside it with CUDA events around each round's
     # relax launch, for comparison: those intervals also hold any host delay
     # between the start event and the launch.
@@ -438,8 +438,8 @@ def run_ours(args, rank, world, local):
     # algorithmic bytes: per edge one packed record (plan edge_bits: 27 column +
     # 6 weight bits at scale 27) and the target distance (4 B); 20 B per vertex
     eb = plan["edge_bits"] / 8
-    kname = ("k_lbs_pair_dev<SrcP<true>,SrcP<true>,MinOp<true>> (device-driven rounds: static + dynamic "
-             "tiles of a round)" if args.direct else "k_gather<SrcP<true>,DstW<u8>> + staged relax")
+    kname = ("k_min_rounds<true> (relax phases: static + dynamic tiles of a round)" if args.direct
+             else "k_stage_round<SrcP<true>,DstW<u8>,SrcW<u8>,MinOp<true>>")
     link_gbs = link_dev / (relax_dev_ms / 1e3) / 1e9 if relax_dev_ms else 0.0
     static_gbs = (eb + 4) * static_dev / (relax_dev_ms / 1e3) / 1e9 if relax_dev_ms else 0.0
     host_link_gbs = dyn_bytes / (relax_ms / 1e3) / 1e9 if relax_ms else 0.0
@@ -448,12 +448,12 @@ def run_ours(args, rank, world, local):
     roof_link = {"bound": "host-link", "kernel": kname, "achieved": link_gbs, "peak": h2d, "unit": "GB/s",
                  "frac": link_gbs / h2d if h2d else None,
                  "traffic": link_dev / max(rounds_dev, 1) * SSSP_RELAX_LINK_TRAFFIC_RATIO,
-                 "traffic_note": "host-link bytes per relax launch: this query's algorithmic link bytes per round "
+                 "traffic_note": "host-link bytes per relax phase: this query's algorithmic link bytes per round "
                                  "x %.3f, the sysmem-sector / algorithmic ratio ncu measured for the same relax's "
                                  "largest dynamic launch on R-MAT 22 under a 256 MiB budget"
                                  % SSSP_RELAX_LINK_TRAFFIC_RATIO,
                  "peak_source": "highest of the link probes measured in this run (og_link_probe)", "link_probes": dict(LINK_PEAKS),
-                 "timing": "globaltimer stamps around every relax launch of %d device-driven queries "
+                 "timing": "globaltimer around every relax phase of %d device-driven queries "
                            "(the timed queries' sources, timer on)" % len(tstats)}
     roof_static = {"bound": "hbm", "kernel": kname + ", its HBM side", "achieved": static_gbs,
                    "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": static_gbs / peaks["hbm_gbs"],
@@ -871,8 +871,8 @@ def run_bfs_resident(args, rank, world, local):
     td_ex = sum(x["edges_static"] + x["edges_dynamic"] for x in tstats)
     td_fv = sum(x["frontier_sum"] for x in tstats)
     td_gbs = ((eb + 4) * td_ex + 20 * td_fv) / (td_ms / 1e3) / 1e9 if td_ms else 0.0
-    # the relax kernel alone: the same top-down queries with the engine's stamp
-    # timer around every relax launch (og_stats.ms_relax)
+    # the relax phases alone: the same top-down queries with the engine's timer
+    # around them (og_stats.ms_relax)
     eng.set_param(og.PARAM_RELAX_TIMER, 1)
     eng.bfs(src, out=False)
     rstats = []
@@ -902,15 +902,15 @@ def run_bfs_resident(args, rank, world, local):
                           "edges_examined_per_query": td_ex / args.steps,
                           "achieved_gbs": td_gbs, "frac": td_gbs / peaks["hbm_gbs"],
                           "graph_vs_l2": "packed records %.0f MB, L2 129 MB" % (g.E * eb / 1e6),
-                          "relax_kernel": {"kernel": "k_lbs_pair_dev<SrcP<false>,SrcP<false>,BfsOp>",
+                          "relax_kernel": {"kernel": "k_bfs_rounds, top-down relax phases",
                                            "ms_per_query": rx_ms / args.steps, "achieved_gbs": rx_gbs,
                                            "frac": rx_gbs / peaks["hbm_gbs"],
-                                           "timing": "globaltimer stamps around every relax launch"}},
+                                           "timing": "globaltimer around every relax phase"}},
         "direction": args.bfs_direction,
         "bit_exact_vs_runCPUBFS": exact, "levels": stats[0]["iterations"],
         "edges_examined_per_query": examined / args.steps,
-        "roofline": {"bound": "hbm", "kernel": "device-driven level loop (compaction, top-down k_lbs_pair_dev, "
-                                               "k_bfs_bottom_up, control): all kernels of a query",
+        "roofline": {"bound": "hbm", "kernel": "k_bfs_rounds and k_bfs_small (scan, top-down relax, "
+                                               "bottom-up): all kernels of a query",
                      "achieved": gbs,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
                      "traffic": None, "peak_source": peaks["source"]},
@@ -1079,7 +1079,7 @@ def run_cc_oom(args, rank, world, local):
         "e2e": {"value": args.steps / e2e_s, "unit": "runs/s", "h2d_bytes_per_step":
                 int(statistics.mean(x["link_bytes"] for x in stats)), "d2h_bytes_per_step": 4 * g.V},
         "roofline": {"bound": "host-link",
-                     "kernel": "k_uf_sample (one record per vertex, random 32-byte sectors over the link)"
+                     "kernel": "k_uf_init (two records per vertex, random 32-byte sectors over the link)"
                      if method == "union-find" else "k_lbs_pair<SrcP<false>,MinOp<false>> over host-mapped records",
                      "achieved": link_gbs, "peak": h2d, "unit": "GB/s", "frac": link_gbs / h2d if h2d else None,
                      "traffic": None, "peak_source": "highest of the link probes measured in this run (og_link_probe)", "link_probes": dict(LINK_PEAKS),
