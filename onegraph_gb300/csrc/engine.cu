@@ -1090,6 +1090,12 @@ int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynF
       return OG_OK;
     }
   }
+  // The dynamic region's work starts behind what the caller has enqueued on
+  // s_main since the counts came back (push PageRank clears its sums there).
+  if (cd.n) {
+    CK(cudaEventRecord(e->ev_round, e->s_main));
+    CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
+  }
   if (cs.n) {
     CK(cudaEventRecord(e->t_s0, e->s_main));
     RC(static_fn(lbs_args(e, 0, 0, cs.total, true, e->plan.static_edges)));
@@ -2194,8 +2200,6 @@ int launch_pr_fixup(og_engine *e, const uint32_t *done) {
 }
 
 int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
-  CK(cudaEventRecord(e->ev_round, e->s_main));
-  CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
   auto sfn = [&](const LbsArgs &a) {
     return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main)
                                : launch_pr_pull<false>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main);
