@@ -11,6 +11,7 @@
 //    previous buffer is relaxed and the static region is relaxed on the main
 //    stream (CalculateOpt.h:75-188, GraphMeta.h:471-557).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <type_traits>
 #include <chrono>
@@ -145,7 +146,7 @@ struct og_engine {
   uint32_t *ring_d = nullptr;  // staged rounds: ticket, then (kRingPad words on) the slot states
   uint32_t level_loop = 0;        // OG_LOOP_AUTO / OG_LOOP_HOST
   uint32_t relax_timer = 0;       // OG_PARAM_RELAX_TIMER
-  void *out = nullptr;            // the running query's result buffer, until its copy is enqueued
+  void *out = nullptr;            // the running query's result array, null once it is delivered
   uint32_t graph_n = 0;
   int graph_cfg = -1;
   int graph_dopt = -1;
@@ -565,7 +566,7 @@ int create_query_state(og_engine *e) {
   CK(cudaMallocHost(&e->counts_h, kControlCounts * sizeof(Counts)));
   e->err_h = (uint32_t *)(e->counts_h + 3);
   RC(dalloc(e, (char **)&e->rounds_d, sizeof(RoundsState)));
-  CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState)));
+  CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState) + 4 * kPostedResult));  // the state, then a small result
   CK(cudaMallocHost(&e->prl_h, sizeof(PrLoop)));
   if (P.chunk_edges && !(e->cfg.flags & OG_CFG_DIRECT)) {
     for (int b = 0; b < 2; b++) {
@@ -1327,8 +1328,26 @@ bool rounds_on_device(const og_engine *e) {
          rounds_fit(e->V, e->g->E);
 }
 
-// BFS, SSSP or label-propagation CC as one kernel; the result is copied to the
-// caller's buffer behind it, so that the host waits once.
+// Waits for the rounds kernel's state (rounds_post): it is in page-locked memory
+// before the kernel has quite ended, so that the copy of the result can be
+// enqueued meanwhile.  Returns as well when the stream is idle or failed, which
+// is asked for rarely: the call takes the CUDA driver's locks.
+int rounds_wait(og_engine *e) {
+  const volatile uint32_t *posted = &e->rounds_h->posted;
+  for (uint32_t i = 1; !*posted; i++) {
+    if (i % 65536) continue;
+    const cudaError_t q = cudaStreamQuery(e->s_main);
+    if (q == cudaErrorNotReady) continue;
+    CK(q);
+    break;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return OG_OK;
+}
+
+// BFS, SSSP or label-propagation CC as one kernel.  The caller's array is written
+// once, after the error word has been read: small results come with the state
+// (RoundsArgs::result), larger ones by a copy.
 int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   cudaStream_t s = e->s_main;
   RoundsArgs a{};
@@ -1348,6 +1367,8 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
     a.tile_cap[r] = e->tile_cap[r];
   }
   a.st = e->rounds_d;
+  a.post = e->rounds_h;
+  if (e->out && a.V <= kPostedResult) a.result = (uint32_t *)(e->rounds_h + 1);
   a.src = src;
   a.delta = algo == OG_ALGO_SSSP ? e->sssp_delta : 0;
   a.split = a.delta ? 1u : 0u;
@@ -1379,20 +1400,23 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
     CK(cudaMemsetAsync(e->rounds_d, 0, sizeof(RoundsState), s));
   }
   for (uint64_t pass = 0;; pass++) {
+    h.posted = 0;
     if (bfs) {
       k_bfs_small<<<1, kSmallThreads, sizeof(SmallShared), s>>>(a, u0, u1);
       e->launches++;
     }
     CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, 0, s));
     e->launches++;
-    CK(cudaMemcpyAsync(&h, e->rounds_d, sizeof h, cudaMemcpyDeviceToHost, s));
-    // the result goes out behind the first pair, which ends most queries
-    if (e->out) CK(cudaMemcpyAsync(e->out, e->value_d, 4ull * e->V, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    RC(rounds_wait(e));
+    if (!h.posted) {  // the kernel ended without its last stores: a barrier gave up
+      CK(cudaMemcpyAsync(&h, e->rounds_d, sizeof h, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      if (!h.err) return fail(OG_E_STATE, "the rounds kernel ended early");
+      break;
+    }
     if (!bfs || h.done || h.err) break;
     if (pass > a.V) return fail(OG_E_STATE, "BFS did not end");
   }
-  e->out = nullptr;
   if (h.err & kErrBarrier) return fail(OG_E_TIMEOUT, "grid barrier wait gave up");
   *e->err_h = h.err;
   RC(check_device_error(e));
@@ -1405,6 +1429,10 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   st.link_bytes += (h.edges_dynamic * e->bpe + 7) / 8;
   st.chunks += (uint32_t)h.iterations;
   e->last_algo = algo;
+  if (e->out && !a.result) return OG_OK;  // fetched by query_common
+  CK(cudaStreamSynchronize(s));
+  if (e->out) memcpy(e->out, a.result, 4ull * a.V);
+  e->out = nullptr;
   return OG_OK;
 }
 
@@ -2460,10 +2488,12 @@ int query_common(og_engine *e, int algo, og_stats *st_out, void *out,
     e->bb_session = false;
     const double t0 = now_ms();
     e->out = out;
-    RC(body(e, st, ctx));
-    st.launches = e->launches;
-    if (e->out) RC(fetch(e, out));  // unless the body has copied it
+    const int rc = body(e, st, ctx);
+    const bool left = e->out != nullptr;  // the body has not delivered the result
     e->out = nullptr;
+    RC(rc);
+    st.launches = e->launches;
+    if (left) RC(fetch(e, out));
     st.ms_total = now_ms() - t0;
     if (st_out) *st_out = st;
     (void)algo;

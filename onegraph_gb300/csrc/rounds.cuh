@@ -21,6 +21,7 @@
 // CTAs wrote in an earlier phase is read with plain loads: the barrier's
 // acquire orders them (and drops stale L1 lines).
 #pragma once
+#include <cstddef>
 #include <type_traits>
 
 #include "batch_persist.cuh"
@@ -48,7 +49,7 @@ struct alignas(128) RoundSlot {
 struct RoundsState {
   unsigned long long bar;  // grid barrier: arrivals so far (polled: on a line of its own)
   alignas(128) uint32_t err;
-  uint32_t pad0;
+  uint32_t posted;  // in the host's copy: the rest of it is there (rounds_post)
   // results for the host
   unsigned long long iterations, frontier_sum, edges_static, edges_dynamic;
   unsigned long long ns_total, ns_relax;
@@ -70,8 +71,33 @@ struct RoundsArgs {
   uint32_t *tile[2];
   uint64_t list_cap[2], tile_cap[2];
   RoundsState *st;
+  RoundsState *post;  // the host's copy, page-locked
+  uint32_t *result;   // when not null: page-locked, takes the values of a query that has ended
   uint32_t src, delta, split, dopt, timer;
 };
+
+// Results of up to this many vertices are stored to page-locked memory by the
+// kernel that ends the query and copied to the caller's array by the host: a
+// copy-engine transfer takes 5-11 us to start, a pageable target as long again.
+constexpr uint32_t kPostedResult = 1u << 14;
+
+// All CTAs, after the last value has been written.
+__device__ __forceinline__ void rounds_result(const RoundsArgs &a) {
+  if (!a.result) return;
+  for (uint32_t v = blockIdx.x * kThreads + threadIdx.x; v < a.V; v += gridDim.x * kThreads)
+    a.result[v] = __ldcg(a.value + v);
+}
+
+// One thread, as the last thing a launch does: the state for the host.
+__device__ __forceinline__ void rounds_post(const RoundsArgs &a) {
+  constexpr size_t n = (offsetof(RoundsState, slot) - offsetof(RoundsState, err)) / 16;
+  const uint4 *s = reinterpret_cast<const uint4 *>(&a.st->err);
+  uint4 *d = reinterpret_cast<uint4 *>(&a.post->err);
+#pragma unroll
+  for (size_t i = 0; i < n; i++) d[i] = __ldcg(s + i);  // posted among them: 0 on the device
+  __threadfence_system();
+  *const_cast<volatile uint32_t *>(&a.post->posted) = 1u;
+}
 
 __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long *p) {
   return cuda::atomic_ref<const unsigned long long, cuda::thread_scope_device>(*p).load(cuda::memory_order_relaxed);
@@ -497,9 +523,11 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
       merge = true;
     }
   }
+  rounds_result(a);
   if (lead) {
     st->ns_relax = nsr;
     st->ns_total = globaltimer_ns() - t0;
+    rounds_post(a);
   }
 }
 
@@ -537,7 +565,7 @@ __global__ void __launch_bounds__(kThreads) k_bfs_init(const __grid_constant__ R
     RoundsState *st = a.st;
     for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
     st->bar = 0;
-    st->err = 0;
+    st->err = st->posted = 0;
     st->iterations = st->frontier_sum = st->edges_static = st->edges_dynamic = 0;
     st->ns_total = st->ns_relax = 0;
     st->unexplored = a.E;
@@ -752,9 +780,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
   } sh;
   __shared__ RelaxShared<SrcP<false>> rs;
   RoundsState *st = a.st;
-  if (st->done) return;  // set before this launch: every CTA reads the same
   unsigned long long target = 0, t0 = 0;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  if (st->done) {  // set before this launch: every CTA reads the same
+    rounds_result(a);
+    if (lead) rounds_post(a);
+    return;
+  }
   if (lead) t0 = globaltimer_ns();
   relax_setup(a, rs, s0, s1);
   bool bottom = st->bottom, counted = st->counted, done = false;
@@ -827,6 +859,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
     level++;
     par ^= 1u;
   }
+  if (done) rounds_result(a);
   if (lead) {
     st->done = done;
     st->small = !done;
@@ -836,6 +869,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
     st->bottom = 0;
     st->unexplored = unexplored;
     st->ns_total += globaltimer_ns() - t0;
+    rounds_post(a);
   }
 }
 

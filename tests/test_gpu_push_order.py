@@ -34,7 +34,8 @@ def test_push_sums_start_from_zero(mode, V, E):
     kw = MODES[mode]
     flags = og.CFG_PR | (og.CFG_DIRECT if "direct" in kw else 0) | (og.CFG_NO_STATIC if "no_static" in kw else 0)
     p = t.plan(budget=1 << 40, flags=flags)
-    edges = E // 2 * 8 if "direct" in kw else 2 * 2048 * p["stage_edge_bytes"] + 4096  # staged: two buffers of a tile
+    # direct: two fifths of the records; staged: two buffers of a tile and a little
+    edges = E * 2 // 5 * p["edge_bits"] // 8 if "direct" in kw else 2 * 2048 * p["stage_edge_bytes"] + 4096
     e = og.Engine(t, budget=p["vertex_bytes"] + p["fixed_bytes"] + edges, pagerank=True, **kw)
     assert e.plan["dynamic_edges"] > 0
     for _ in range(3):
