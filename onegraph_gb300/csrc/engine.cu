@@ -2192,6 +2192,7 @@ PrArgs pr_args(const og_engine *e, int r, const uint32_t *done) {
   q.base = r ? e->plan.static_edges : 0;
   q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
   q.done = done;
+  q.link = (uint32_t)r;
   return q;
 }
 

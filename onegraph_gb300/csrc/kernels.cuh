@@ -1515,6 +1515,7 @@ struct PrArgs {
   uint64_t base, nwords;
   // iterations launched ahead: when not null, nothing is done once *done is set
   const uint32_t *done;
+  uint32_t link;  // the records are read over the host link
 };
 
 // Pull sum sum[v] = sum over in-edges (u -> v) of contrib[u]
@@ -1531,22 +1532,29 @@ struct PrArgs {
 // position does not depend on the list, so the tile's words are fetched 16
 // bytes a lane before anything else and the gather starts while the flags
 // are still being built.  Other lists read each record through its vertex's
-// cursor.  Measured on 8.4 M vertices and 131 M edges: 1.09 ms an iteration with
+// cursor.  Over the host link a warp's lanes read consecutive positions and hand
+// the columns to their owners through shared memory: with each lane on its own
+// eight records a warp asks for every sector several times (direct delta PageRank of
+// 4.2 M vertices, two fifths resident: 21.1 ms so, 12.5 now); from HBM the detour
+// costs more than it gives (all resident: 7.0 ms without, 8.0 with).  Measured on 8.4 M vertices and 131 M edges: 1.09 ms an iteration with
 // positions strided over the threads and staged twice through shared memory,
 // 0.53 ms in this form (247 G edges/s; 65 M edges: L1 81 % busy, L2 65 %).
-constexpr uint32_t kPrFlagBytes = kTile;
+constexpr uint32_t pr_flag_bytes(bool dense) { return dense ? kTile : 2 * kTile; }
 constexpr uint32_t pr_smem_bytes(bool dense, uint32_t bpe) {
-  // flags, then (by phase) the tile's words / the cursors, and the sums
+  // flags (cursor form: later each position's vertex), then by phase the
+  // tile's words / the cursors, the columns, and the sums
   const uint32_t words = (kTile * bpe / 32 + 10) * 4, tot = (kTile + 1) * 4, cur = (kTile + 1) * 8;
-  return kPrFlagBytes + (dense ? (words > tot ? words : tot) : cur) + 16;
+  return pr_flag_bytes(dense) + (dense ? (words > tot ? words : tot) : cur) + 16;
 }
 
 template <bool kDense, class Src>
 __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const PrArgs &p, uint64_t k) {
   extern __shared__ __align__(16) unsigned char pr_smem[];
   unsigned char *flag = pr_smem;
-  uint32_t *words = reinterpret_cast<uint32_t *>(pr_smem + kPrFlagBytes);
-  unsigned long long *cur = reinterpret_cast<unsigned long long *>(words);  // !kDense
+  uint32_t *words = reinterpret_cast<uint32_t *>(pr_smem + pr_flag_bytes(kDense));
+  // !kDense
+  unsigned long long *cur = reinterpret_cast<unsigned long long *>(words);
+  uint16_t *map = reinterpret_cast<uint16_t *>(pr_smem);
   float *tot = reinterpret_cast<float *>(words);  // once the records are in registers
   __shared__ uint32_t s_bad, s_edge;
   __shared__ float s_wv[kThreads / 32];
@@ -1634,6 +1642,11 @@ __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const 
   uint32_t heads = 0;
 #pragma unroll
   for (int i = 0; i < 4; i++) heads |= ((fw.x >> (8 * i)) & 1u) << i | ((fw.y >> (8 * i)) & 1u) << (4 + i);
+  // whether a vertex ends with this thread's last position; the cursor form reads it before the map takes the
+  // flags' place, the other one where it is needed (a register more costs it 2 %)
+  auto ends_here = [&]() { return x0 + kItems >= tlen || flag[x0 + kItems]; };
+  bool last = false;
+  if constexpr (!kDense) last = ends_here();
   const uint32_t lane = tid & 31, warp = tid >> 5;
   uint32_t u[kItems];
   if constexpr (kDense) {
@@ -1655,13 +1668,39 @@ __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const 
     __syncthreads();
     uint32_t l = ic - c;
     for (uint32_t w = 0; w < warp; w++) l += s_wc[w];
+    if (!p.link) {  // uniform
 #pragma unroll
-    for (int i = 0; i < (int)kItems; i++) {
-      u[i] = 0xffffffffu;
-      l += (heads >> i) & 1u;
-      if (x0 + i < tlen) u[i] = src.at(cur[l], x0 + i);
+      for (int i = 0; i < (int)kItems; i++) {
+        l += (heads >> i) & 1u;
+        u[i] = x0 + i < tlen ? src.at(cur[l], x0 + i) : 0xffffffffu;
+      }
+      __syncthreads();  // s_wc is written again below
+    } else {
+      uint32_t m[kItems / 2];
+#pragma unroll
+      for (int i = 0; i < (int)kItems; i += 2) {
+        l += (heads >> i) & 1u;
+        m[i / 2] = l;
+        l += (heads >> (i + 1)) & 1u;
+        m[i / 2] |= l << 16;
+      }
+      *reinterpret_cast<uint4 *>(map + x0) = make_uint4(m[0], m[1], m[2], m[3]);  // every flag has been read
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < (int)kItems; i++) {
+        const uint32_t x = i * kThreads + tid;
+        u[i] = x < tlen ? src.at(cur[map[x]], x) : 0xffffffffu;
+      }
+      __syncthreads();  // the cursors have been read: the columns take their place
+#pragma unroll
+      for (int i = 0; i < (int)kItems; i++) words[i * kThreads + tid] = u[i];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < (int)kItems; i += 4) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(words + x0 + i);
+        u[i] = q.x, u[i + 1] = q.y, u[i + 2] = q.z, u[i + 3] = q.w;
+      }
     }
-    __syncthreads();  // s_wc is written again below
   }
   float c[kItems];
 #pragma unroll
@@ -1717,7 +1756,7 @@ __device__ __forceinline__ void pr_tile(const LbsArgs &a, const Src &src, const 
     }
     run += c[i];
   }
-  if (x0 < tlen && (x0 + kItems >= tlen || flag[x0 + kItems])) tot[l] = run;
+  if (x0 < tlen && (kDense ? ends_here() : last)) tot[l] = run;
   __syncthreads();
   for (uint32_t j = tid; j < nl; j += kThreads) {
     const uint32_t i = i0 + j;
