@@ -565,7 +565,7 @@ int create_query_state(og_engine *e) {
   RC(dalloc(e, &e->sum64_d, 3ull * e->sms * 8 + 4));
   CK(cudaMallocHost(&e->counts_h, kControlCounts * sizeof(Counts)));
   e->err_h = (uint32_t *)(e->counts_h + 3);
-  RC(dalloc(e, (char **)&e->rounds_d, sizeof(RoundsState)));
+  RC(dalloc(e, (char **)&e->rounds_d, kJumps * sizeof(RoundsState)));
   CK(cudaMallocHost(&e->rounds_h, sizeof(RoundsState) + 4 * kPostedResult));  // the state, then a small result
   CK(cudaMallocHost(&e->prl_h, sizeof(PrLoop)));
   if (P.chunk_edges && !(e->cfg.flags & OG_CFG_DIRECT)) {
@@ -893,7 +893,7 @@ int check_device_error(og_engine *e) {
   const uint32_t err = *e->err_h;
   if (!err) return OG_OK;
   if (err & kErrLookback) return fail(OG_E_TIMEOUT, "frontier compaction look-back wait gave up");
-  if (err & kErrBarrier) return fail(OG_E_TIMEOUT, "staged round: a slot wait gave up");
+  if (err & kErrBarrier) return fail(OG_E_TIMEOUT, "a wait between thread blocks gave up");
   return fail(OG_E_DEVICE, "kernel reported an out-of-range index (flags 0x%x)", err);
 }
 
@@ -2690,6 +2690,18 @@ int run_cc_uf(og_engine *e, og_stats &st) {
   cudaStream_t s = e->s_main;
   const int g = grid_for(V, e->sms);
   uint32_t *par = e->value_d;
+  uint32_t jumps = 0;
+  auto compress = [&]() -> int {  // every vertex right under its root
+    int occ = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_uf_jump, kThreads, 0));
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, occ) * e->sms, V / 1024 + 1);
+    uint32_t v = V, *p = par;
+    RoundsState *state = e->rounds_d + jumps++;  // cleared by k_uf_init
+    void *args[4] = {&p, &v, &state, &e->err_d};
+    CK(cudaLaunchCooperativeKernel((const void *)k_uf_jump, dim3(grid), dim3(kThreads), args, 0, s));
+    e->launches++;
+    return OG_OK;
+  };
   unsigned long long *reads = e->sum64_d;  // [0] host records, [1] static records
   uint32_t *roots_d = (uint32_t *)(e->sum64_d + 2);
   constexpr uint32_t kRoots = 1024;
@@ -2699,11 +2711,11 @@ int run_cc_uf(og_engine *e, og_stats &st) {
   CK(cudaEventRecord(t0, s));
   uint2 *pend = (uint2 *)e->pref_d[0];  // V + 2 entries of 8 bytes, not in use before the compaction
   k_uf_init<EKU::PSrc><<<g, kThreads, 0, s>>>(e->off_d, V, e->plan.static_edges, EKU::stat(e), EKU::host(e), par, pend,
-                                              reads, e->err_d);
-  k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
+                                              reads, (uint32_t *)e->rounds_d, kJumps * sizeof(RoundsState) / 4, e->err_d);
+  RC(compress());
   k_uf_link<<<g, kThreads, 0, s>>>(pend, V, par, e->err_d);
-  k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
-  e->launches += 4;
+  RC(compress());
+  e->launches += 2;
   st.iterations += 2;
   k_uf_roots<<<(kRoots + kThreads - 1) / kThreads, kThreads, 0, s>>>(par, V, kRoots, roots_d);
   e->launches++;
@@ -2760,12 +2772,7 @@ int run_cc_uf(og_engine *e, og_stats &st) {
     };
     RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
   }
-  if (n) {  // nothing was linked since the last compression otherwise
-    k_uf_compress<<<g, kThreads, 0, s>>>(par, V, e->err_d);
-    e->launches++;
-  }
-  k_uf_flatten<<<g, kThreads, 0, s>>>(par, V, e->err_d);
-  e->launches++;
+  if (n) RC(compress());  // nothing was linked since the last compression otherwise
   CK(cudaStreamSynchronize(s));
   collect_timing(e, tm, &st);
   CK(cudaMemcpy(e->err_h, e->err_d, 4, cudaMemcpyDeviceToHost));

@@ -2295,7 +2295,9 @@ __device__ __forceinline__ void uf_link(uint32_t *par, uint32_t a, uint32_t b, u
 template <class PS>
 __global__ void __launch_bounds__(kThreads) k_uf_init(const uint64_t *off, uint32_t V, uint64_t static_edges, PS stat,
                                                       PS host, uint32_t *par, uint2 *pend, unsigned long long *reads,
-                                                      uint32_t *err) {
+                                                      uint32_t *states, uint32_t nstate, uint32_t *err) {
+  if (blockIdx.x == 0)  // the barrier states of the compressions to come
+    for (uint32_t i = threadIdx.x; i < nstate; i += kThreads) states[i] = 0u;
   const uint32_t cmask = stat.bc >= 32 ? 0xffffffffu : (1u << stat.bc) - 1u;
   uint32_t nh = 0, ns = 0;  // records read from the host copy / the static region
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
@@ -2378,33 +2380,6 @@ __global__ void __launch_bounds__(kThreads) k_uf_link(const uint2 *pend, uint32_
         __syncwarp();
       }
     }
-  }
-}
-
-// parent[v] = root of v for every vertex, up to the walks that halve a path
-// through v at the same moment: such a walk may put an ancestor it read
-// earlier back after v's own store.  Long chains become short ones.
-__global__ void __launch_bounds__(kThreads) k_uf_compress(uint32_t *par, uint32_t V, uint32_t *err) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
-    __stcg(par + v, uf_find(par, (uint32_t)v, V, err));
-}
-
-// The labels, after k_uf_compress: walks that store nothing but their own
-// vertex's root, so every vertex ends with it.
-__global__ void __launch_bounds__(kThreads) k_uf_flatten(uint32_t *par, uint32_t V, uint32_t *err) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t p0 = __ldca(par + v);
-    uint32_t x = p0;
-    for (uint32_t steps = 0;; steps++) {
-      const uint32_t p = __ldca(par + x);
-      if (p == x) break;
-      if (p > x || steps > V) {
-        atomicOr(err, kErrVertex);
-        break;
-      }
-      x = p;
-    }
-    if (x != p0) __stcg(par + v, x);
   }
 }
 

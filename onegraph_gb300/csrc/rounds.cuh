@@ -873,4 +873,64 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
   }
 }
 
+// ------------------------------------------------------------- union-find CC
+
+// parent[v] = root of v for every vertex, by pointer jumping between grid
+// barriers: a pass takes each vertex up to kJumpHops parents up, from where the
+// pass before has taken them, until one leaves no vertex below its root.  A
+// thread stores its own vertices only, and the barrier drops the parents that
+// L1 holds, so chains shrink by the number of hops with every pass.  Bound by
+// latency, a round trip per hop.  A kernel of whole walks per vertex kept each
+// wave of threads waiting for its longest chain where first neighbours form
+// chains: union-find CC of a 5000 x 4000 grid numbered by rows 2.72 ms with it,
+// 0.87 now (4 hops 0.94, two walks a thread 0.88); R-MAT of 2^23 vertices, whose
+// chains are shorter than a pass, 0.45 either way.
+constexpr uint32_t kJumps = 3;  // compressions of a run
+constexpr uint32_t kJumpHops = 8;
+constexpr int kJumpWalks = 4;  // vertices a thread has in flight
+__global__ void __launch_bounds__(kThreads) k_uf_jump(uint32_t *par, uint32_t V, RoundsState *st, uint32_t *err) {
+  unsigned long long target = 0;
+  const uint64_t first = blockIdx.x * (uint64_t)kThreads + threadIdx.x, stride = (uint64_t)gridDim.x * kThreads;
+  for (uint32_t pass = 0;; pass++) {
+    uint32_t open = 0;
+    for (uint64_t v = first; v < V; v += kJumpWalks * stride) {
+      uint32_t x[kJumpWalks], p[kJumpWalks], todo = 0;
+#pragma unroll
+      for (int j = 0; j < kJumpWalks; j++) {
+        const bool on = v + j * stride < V;
+        x[j] = p[j] = on ? (uint32_t)(v + j * stride) : 0u;
+        todo |= (on ? 1u : 0u) << j;
+      }
+      const uint32_t mine = todo;
+      uint32_t own[kJumpWalks];
+#pragma unroll
+      for (uint32_t h = 0; h <= kJumpHops; h++) {
+        if (!todo) break;
+#pragma unroll
+        for (int j = 0; j < kJumpWalks; j++)
+          if ((todo >> j) & 1u) p[j] = __ldca(par + x[j]);
+#pragma unroll
+        for (int j = 0; j < kJumpWalks; j++) {
+          if (h == 0) own[j] = p[j];
+          if (p[j] > x[j]) atomicOr(err, kErrVertex);
+          if (p[j] >= x[j]) todo &= ~(1u << j);  // x is a root
+          else x[j] = p[j];
+        }
+      }
+      open |= todo;
+#pragma unroll
+      for (int j = 0; j < kJumpWalks; j++)
+        if (((mine >> j) & 1u) && x[j] != own[j]) __stcg(par + v + j * stride, x[j]);
+    }
+    uint32_t *flag = &st->slot[pass & 3u].near;
+    if (__syncthreads_or(open != 0u) && threadIdx.x == 0) *flag = 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->slot[(pass + 2) & 3u].near = 0u;  // last read before the barrier before
+    if (!rounds_sync(st, target) || pass > 64) {
+      if (threadIdx.x == 0) atomicOr(err, kErrBarrier);
+      return;
+    }
+    if (!__ldcg(flag)) return;
+  }
+}
+
 }  // namespace og
