@@ -438,7 +438,8 @@ def run_ours(args, rank, world, local):
     # algorithmic bytes: per edge one packed record (plan edge_bits: 27 column +
     # 6 weight bits at scale 27) and the target distance (4 B); 20 B per vertex
     eb = plan["edge_bits"] / 8
-    kname = ("k_min_rounds<true> (relax phases: static + dynamic tiles of a round)" if args.direct
+    kname = ("k_lbs_pair<SrcP<true>,SrcP<true>,MinOp<true>> (large rounds) and k_min_rounds<true> (relax phases of "
+             "the others: static + dynamic tiles of a round)" if args.direct
              else "k_stage_round<SrcP<true>,DstW<u8>,SrcW<u8>,MinOp<true>>")
     link_gbs = link_dev / (relax_dev_ms / 1e3) / 1e9 if relax_dev_ms else 0.0
     static_gbs = (eb + 4) * static_dev / (relax_dev_ms / 1e3) / 1e9 if relax_dev_ms else 0.0

@@ -473,7 +473,8 @@ int og_engine_clone(og_engine *parent, og_engine **out);
 /* OG_PARAM_LEVEL_LOOP: OG_LOOP_AUTO (default) runs the levels / rounds of
  *   og_bfs, og_sssp and label-propagation og_cc on the device, in one
  *   cooperative kernel that takes every per-round decision itself (BFS: with
- *   a one-CTA kernel for small frontiers beside it), in direct mode or on a
+ *   a one-CTA kernel for small frontiers beside it; rounds of very many edges
+ *   are relaxed by a launch of their own in between), in direct mode or on a
  *   fully resident graph of fewer than 2^28 vertices and 2^36 edges; other
  *   engines keep the host loop.  OG_LOOP_HOST waits for each round's
  *   counts on the host.  Results are identical. */
@@ -482,7 +483,8 @@ int og_engine_clone(og_engine *parent, og_engine **out);
 #define OG_LOOP_HOST 1
 /* OG_PARAM_RELAX_TIMER: 1 sums the time of the (top-down) relax phases of the
  *   device-driven rounds, read from the GPU's global timer after the grid
- *   barriers around each (og_stats.ms_relax); 0 (default) does not read it.
+ *   barriers around each (og_stats.ms_relax), or with events where the phase
+ *   is a launch of its own; 0 (default) reads neither.
  *   Levels of small BFS frontiers, expanded by one CTA, count as a whole. */
 #define OG_PARAM_RELAX_TIMER 5
 /* OG_PARAM_SSSP_BATCH_DELTA: near/far width of og_sssp_batch, shared by its

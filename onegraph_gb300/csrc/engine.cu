@@ -1345,6 +1345,44 @@ int rounds_wait(og_engine *e) {
   return OG_OK;
 }
 
+// Tiles above which a round is relaxed by a launch of its own (hands_over), and
+// vertices from which a bottom-up level is expanded by one.  A handover costs a
+// wait and two launches, about 25 us.  In the rounds kernel / handed over, ms:
+// resident rounds, label propagation on R-MAT 20 (16 thousand tiles a round) 0.82 /
+// 0.50, 22 3.27 / 1.69, 24 13.6 / 6.8, at 4096 tiles about even; SSSP over
+// the link, R-MAT 24 12.3 / 12.3, 26 54.1 / 47.5, 27 117 / 94.7; top-down BFS over
+// the link, 24 8.73 / 8.96, 27 75.0 / 77.1: never handed over.  Bottom-up levels of
+// BFS over the link, R-MAT 22 0.54 / 0.60, 23 0.92 / 0.92, 24 2.04 / 1.94, 27 14.2 /
+// 12.6; resident 24 1.15 / 1.01.
+constexpr uint64_t kHandHbm = 4096, kHandLink = 32768;
+constexpr uint32_t kHandBottomVertices = 1u << 24;
+
+// The relax of a round that the rounds kernel has handed over: its lists are in
+// place, `op` acts on them as the kernel's would.
+template <class Src, class Op>
+int relax_handed(og_engine *e, const RoundsState &h, Src s0, Src s1, Op op) {
+  LbsArgs a[2];
+  uint64_t n[2];
+  for (int r = 0; r < 2; r++) {
+    Counts &c = e->counts_h[r];
+    c.n = (uint32_t)(h.hx[r] >> kAppendShift);
+    c.total = h.hx[r] & ((1ull << kAppendShift) - 1);
+    a[r] = lbs_args(e, r, 0, c.total, true, r ? e->g->E : e->plan.static_edges);
+    a[r].err = &e->rounds_d->err;
+    n[r] = lbs_grid(0, c.total);
+  }
+  op.err = &e->rounds_d->err;
+  if (n[0] && n[1])
+    k_lbs_pair<Src, Src, Op><<<(unsigned)(n[0] + n[1]), kThreads, 0, e->s_main>>>(a[0], s0, a[1], s1, op, n[0],
+                                                                                 n[0] + n[1]);
+  else if (n[0])
+    k_lbs<Src, Op><<<(unsigned)n[0], kThreads, 0, e->s_main>>>(a[0], s0, op);
+  else
+    k_lbs<Src, Op><<<(unsigned)n[1], kThreads, 0, e->s_main>>>(a[1], s1, op);
+  e->launches++;
+  return OG_OK;
+}
+
 // BFS, SSSP or label-propagation CC as one kernel.  The caller's array is written
 // once, after the error word has been read: small results come with the state
 // (RoundsArgs::result), larger ones by a copy.
@@ -1374,6 +1412,9 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   a.split = a.delta ? 1u : 0u;
   a.dopt = algo == OG_ALGO_BFS && e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1;
   a.timer = e->relax_timer;
+  a.hand_hbm = kHandHbm;
+  a.hand_link = algo == OG_ALGO_BFS ? ~0ull : kHandLink;
+  a.hand_bottom = a.V >= kHandBottomVertices;
   SrcP<false> u0 = EKU::stat(e), u1 = EKU::host(e);
   SrcP<true> w0{e->spk_d, e->bpe, e->bc, e->wmin}, w1{e->hpk_d, e->bpe, e->bc, e->wmin};
   const bool bfs = algo == OG_ALGO_BFS;
@@ -1399,9 +1440,28 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   } else {
     CK(cudaMemsetAsync(e->rounds_d, 0, sizeof(RoundsState), s));
   }
+  float ms_handed = 0, ms_handed_relax = 0;
+  h.hand = 0;
   for (uint64_t pass = 0;; pass++) {
     h.posted = 0;
-    if (bfs) {
+    const uint32_t handed = h.hand;
+    if (handed) {
+      CK(cudaEventRecord(e->t_d0, s));
+      if (handed == kHandBottomUp) {
+        k_bfs_bottom_up<EKU::PSrc><<<grid_for(a.V, e->sms), kThreads, 0, s>>>(
+            e->off_d, a.V, a.Vs, u0, u1, a.bm[h.par], a.bm[2], a.bm[h.par ^ 1], e->value_d, h.level + 1,
+            e->rounds_d->hbu, &e->rounds_d->err);
+        e->launches++;
+      } else if (bfs) {  // the state is already that of the next level
+        RC(relax_handed(e, h, u0, u1, BfsOp{a.bm[2], a.bm[h.par], e->value_d, nullptr, a.V, h.level}));
+      } else if (algo == OG_ALGO_SSSP) {
+        RC(relax_handed(e, h, w0, w1, MinOp<true>{e->value_d, a.bm[h.par], nullptr, a.V}));
+      } else {
+        RC(relax_handed(e, h, u0, u1, MinOp<false>{e->value_d, a.bm[h.par], nullptr, a.V}));
+      }
+      CK(cudaEventRecord(e->ev_dyn_done, s));
+      CK(cudaMemsetAsync(&e->rounds_d->bar, 0, sizeof e->rounds_d->bar, s));
+    } else if (bfs) {
       k_bfs_small<<<1, kSmallThreads, sizeof(SmallShared), s>>>(a, u0, u1);
       e->launches++;
     }
@@ -1414,14 +1474,20 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
       if (!h.err) return fail(OG_E_STATE, "the rounds kernel ended early");
       break;
     }
-    if (!bfs || h.done || h.err) break;
-    if (pass > a.V) return fail(OG_E_STATE, "BFS did not end");
+    if (handed) {
+      float ms = 0;
+      CK(cudaEventElapsedTime(&ms, e->t_d0, e->ev_dyn_done));
+      ms_handed += ms;
+      if (handed == kHandRelax && a.timer) ms_handed_relax += ms;
+    }
+    if (h.done || h.err) break;
+    if (pass > 2ull * a.V + 64) return fail(OG_E_STATE, "the rounds did not end");
   }
   if (h.err & kErrBarrier) return fail(OG_E_TIMEOUT, "grid barrier wait gave up");
   *e->err_h = h.err;
   RC(check_device_error(e));
-  st.ms_dynamic += h.ns_total / 1e6;
-  st.ms_relax += h.ns_relax / 1e6;
+  st.ms_dynamic += h.ns_total / 1e6 + ms_handed;
+  st.ms_relax += h.ns_relax / 1e6 + ms_handed_relax;
   st.iterations += (uint32_t)h.iterations;
   st.frontier_sum += h.frontier_sum;
   st.edges_static += h.edges_static;

@@ -912,6 +912,12 @@ struct HasCommit : std::false_type {};
 template <class T>
 struct HasCommit<T, std::void_t<decltype(&T::commit)>> : std::true_type {};
 
+// Positions of a tile that a thread has in flight.
+template <class Op>
+struct OpGroup {
+  static constexpr int value = kItems;
+};
+
 // Runs `body(lo, hi, j0)` over positions [plo, phi) of tile k: once, or in parts
 // of kThreads positions when the tile holds more than kLocal vertices.  In
 // the body, position x belongs to table entry map[x] - j0, and src.at(cb[entry],
@@ -1022,40 +1028,49 @@ __device__ __forceinline__ void lbs_tile(const LbsArgs &a, const Src &src, const
   const uint32_t phi = min((uint32_t)min((uint64_t)kTile, a.pos_end - pos0), plo + kTile / parts);
   if (plo >= phi) return;  // uniform
   lbs_run<Op::kNeedVal>(a, src, op, sh, k, plo, phi, [&](uint32_t lo, uint32_t hi, uint32_t j0) {
-    // All eight loads are issued before the first relax, so each thread keeps
-    // eight edge reads in flight (the host-link gather is latency bound).
-    const uint32_t x0 = lo + threadIdx.x;
-    typename Src::Item ev[kItems];
-    uint32_t lv[kItems];
+    constexpr int G = OpGroup<Op>::value;
+    // Positions x0, x0 + kThreads, ...: G of them.  All their loads are issued
+    // before the first relax, so each thread keeps G edge reads in flight (the
+    // host-link gather is latency bound).
+    auto group = [&](uint32_t x0) {
+      typename Src::Item ev[G];
+      uint32_t lv[G];
 #pragma unroll
-    for (int it = 0; it < (int)kItems; it++) {
-      const uint32_t x = it * kThreads + x0;
-      lv[it] = 0;
-      if (x < hi) {
-        const uint32_t l = sh.map[x] - j0;
-        lv[it] = l;
-        ev[it] = src.at(sh.cb[l], x);
+      for (int it = 0; it < G; it++) {
+        const uint32_t x = it * kThreads + x0;
+        lv[it] = 0;
+        if (x < hi) {
+          const uint32_t l = sh.map[x] - j0;
+          lv[it] = l;
+          ev[it] = src.at(sh.cb[l], x);
+        }
       }
-    }
-    if constexpr (HasCommit<Op>::value)
-      if (!op.commit()) return;
-    // Probe phase: every target's current state is read before the first
-    // atomic, so the eight random reads of a thread overlap (in program order
-    // the compiler may not lift a load above an earlier atomic).  A probe is
-    // only a filter: relax() acts through atomics, so a stale probe costs an
-    // extra atomic, never a wrong result.
-    typename Op::Probe pr[kItems];
+      if constexpr (HasCommit<Op>::value)
+        if (!op.commit()) return;
+      // Probe phase: every target's current state is read before the first
+      // atomic, so the random reads of a thread overlap (in program order
+      // the compiler may not lift a load above an earlier atomic).  A probe is
+      // only a filter: relax() acts through atomics, so a stale probe costs an
+      // extra atomic, never a wrong result.
+      typename Op::Probe pr[G];
 #pragma unroll
-    for (int it = 0; it < (int)kItems; it++)
-      if (it * kThreads + x0 < hi) {
-        if constexpr (HasProbeVal<Op>::value) pr[it] = op.probe_v(ev[it], sh.val[lv[it]]);
-        else pr[it] = op.probe(ev[it]);
+      for (int it = 0; it < G; it++)
+        if (it * kThreads + x0 < hi) {
+          if constexpr (HasProbeVal<Op>::value) pr[it] = op.probe_v(ev[it], sh.val[lv[it]]);
+          else pr[it] = op.probe(ev[it]);
+        }
+#pragma unroll
+      for (int it = 0; it < G; it++) {
+        if (it * kThreads + x0 < hi)
+          op.relax(ev[it], Op::kNeedVal ? sh.val[lv[it]] : typename Op::Val{},
+                   pos0 + it * kThreads + x0, pr[it]);
       }
-#pragma unroll
-    for (int it = 0; it < (int)kItems; it++) {
-      if (it * kThreads + x0 < hi)
-        op.relax(ev[it], Op::kNeedVal ? sh.val[lv[it]] : typename Op::Val{},
-                 pos0 + it * kThreads + x0, pr[it]);
+    };
+    if constexpr (G == kItems) {
+      group(lo + threadIdx.x);
+    } else {
+#pragma unroll 1
+      for (uint32_t x = lo; x < hi; x += G * kThreads) group(x + threadIdx.x);
     }
   });
 }

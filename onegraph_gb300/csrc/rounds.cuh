@@ -12,6 +12,8 @@
 //          per region; a 64-bit atomic reserves list entries and edge positions
 //          together, so the order of the appends does not matter
 //   relax  edge-balanced tiles of both lists, interleaved (lbs_tile)
+// Rounds of very many tiles are handed over: the kernel ends after the scan, the
+// host launches the relax on its own and then this kernel again (kHandRelax).
 // Small BFS frontiers are expanded by a kernel of one CTA out of shared memory,
 // level after level.
 //
@@ -57,6 +59,10 @@ struct RoundsState {
   unsigned long long unexplored, fn;
   uint32_t level, par, bottom, counted, done;
   uint32_t small, n0, n;  // the frontier is listed: n0 static vertices, n in all
+  // round handed over to a launch of its own (kHand*), and what it needs
+  uint32_t hand, thr, far_min, pad0;
+  unsigned long long hx[2];   // list reservations of the two regions
+  unsigned long long hbu[4];  // bottom-up counts, taken by that launch
   RoundSlot slot[4];
 };
 
@@ -74,7 +80,20 @@ struct RoundsArgs {
   RoundsState *post;  // the host's copy, page-locked
   uint32_t *result;   // when not null: page-locked, takes the values of a query that has ended
   uint32_t src, delta, split, dopt, timer;
+  uint64_t hand_hbm, hand_link;  // rounds of more tiles are handed over (hands_over)
+  uint32_t hand_bottom;          // bottom-up levels are
 };
+
+// A round of many tiles is faster as a launch of one CTA per tile: the tables of
+// a CTA's next tile are then built while its neighbours' reads are under way,
+// where a CTA of this kernel waits for all its warps between two tiles, with
+// fewer CTAs on the SM.  The state is kept in RoundsState meanwhile.  The line
+// between the limits is where the link takes as long as HBM: 42 G edges/s
+// against 160 (top-down BFS, R-MAT 24).
+constexpr uint32_t kHandRelax = 1, kHandBottomUp = 2;
+__device__ __forceinline__ bool hands_over(const RoundsArgs &a, uint64_t n0, uint64_t n1) {
+  return n0 + n1 > (4 * n1 > n0 ? a.hand_link : a.hand_hbm);
+}
 
 // Results of up to this many vertices are stored to page-locked memory by the
 // kernel that ends the query and copied to the caller's array by the host: a
@@ -103,18 +122,18 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
   return cuda::atomic_ref<const unsigned long long, cuda::thread_scope_device>(*p).load(cuda::memory_order_relaxed);
 }
 
-// Grid barrier over one counter of arrivals: `target` grows by the grid size
-// with every barrier.  The polls are relaxed and one acquire fence follows
+// Grid barrier over one counter of arrivals: `target`, which thread 0 keeps, grows by
+// the grid size with every barrier.  The polls are relaxed and one acquire fence follows
 // them: an acquiring poll drops the SM's whole L1 each time, under the CTAs
 // that still work (a round's relax, resident SSSP of 0.3 M vertices: 13-15 us
 // on average so, 9 us now).  A wait longer than kSpinLimit polls sets kErrBarrier and returns
 // false instead of hanging.
 __device__ __forceinline__ bool rounds_sync(RoundsState *st, unsigned long long &target) {
   __shared__ int s_ok;
-  target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
+    target += gridDim.x;
     __threadfence();
     atomicAdd(&st->bar, 1ull);
     uint32_t spins = 0;
@@ -273,8 +292,9 @@ __device__ __forceinline__ uint32_t scan_group(const RoundsArgs &a, ScanWarp &sh
 // it, and with `merge` the waiting set is scanned too.  A warp owns its
 // group's words, so no bitmap update needs an atomic.  Small graphs get small
 // groups, so that the frontier is spread over all warps.
-// Not inlined, as the other phases besides the relax: the tile loop then
-// keeps its registers (inlined, 300-460 B a thread were spilled).
+// Not inlined, as the other phases: inlined, 300-460 B a thread were spilled.  What
+// spills now is a few words around the calls (24-28 B a thread in k_min_rounds, 160
+// in k_bfs_rounds) and in the scans (up to 76 B), not in the loops over tiles.
 template <bool kSplit, bool kZeroCur>
 __device__ __noinline__ void scan_frontier(const RoundsArgs &a, ScanShared &shared, uint32_t *cur, uint32_t *next,
                                            uint32_t *waiting, bool merge, uint32_t thr, RoundSlot *slot) {
@@ -317,6 +337,10 @@ __device__ __noinline__ void scan_frontier(const RoundsArgs &a, ScanShared &shar
   }
 }
 
+__device__ __forceinline__ uint64_t list_tiles(unsigned long long app) {
+  return ((app & ((1ull << kAppendShift) - 1)) + kTile - 1) / kTile;
+}
+
 __device__ __forceinline__ void slot_clear(RoundSlot *s) {
   s->app[0] = s->app[1] = 0;
   s->tile_next = 0;
@@ -325,15 +349,18 @@ __device__ __forceinline__ void slot_clear(RoundSlot *s) {
   s->bu[0] = s->bu[1] = s->bu[2] = s->bu[3] = 0;
 }
 
-// Arguments of a region's tiles live in shared memory and one tile body serves
-// both regions: kept in registers across the tile loop they cost 98 registers
-// per thread (2 CTAs per SM).
-template <class Src>
+// What a CTA's threads have in common lives in shared memory, and one tile body
+// serves both regions: the regions' arguments kept in registers across the tile
+// loop cost 98 registers per thread (2 CTAs per SM), and the op, the barrier's
+// target and the timers as many spills.
+template <class Src, class Op>
 struct RelaxShared {
   LbsArgs a[2];
   Src s[2];
   PairTile pt[2];
   uint32_t b[2];
+  Op op;
+  unsigned long long target;
 };
 
 // Relax of both regions' lists.  A CTA's first tile is its index in the grid
@@ -345,7 +372,7 @@ struct RelaxShared {
 // (resident SSSP of 0.3 M vertices: 1.05 -> 0.87 ms with parts).  The next ticket (and its region
 // split, by thread 0) is fetched while the current tile runs.
 template <class Src, class Op>
-__device__ __noinline__ Op relax_lists(RelaxShared<Src> &rs, LbsSh<Op> &sh, Op op, RoundSlot *slot) {
+__device__ __noinline__ void relax_lists(RelaxShared<Src, Op> &rs, LbsSh<Op> &sh, RoundSlot *slot) {
   __builtin_assume(__isShared(&rs));  // shared, not generic, accesses
   __builtin_assume(__isShared(&sh));
   if (threadIdx.x == 0) {
@@ -375,14 +402,14 @@ __device__ __noinline__ Op relax_lists(RelaxShared<Src> &rs, LbsSh<Op> &sh, Op o
       rs.b[k ^ 1] = nb;
       if (nb < n) rs.pt[k ^ 1] = pair_split(nb / parts, n0, n0 + n1);
     }
-    lbs_tile(rs.a[pt.r], rs.s[pt.r], op, sh, pt.t, b % parts, parts);
+    lbs_tile(rs.a[pt.r], rs.s[pt.r], rs.op, sh, pt.t, b % parts, parts);
     __syncthreads();  // the tile tables are rebuilt and the next ticket is read after this
   }
-  return op;
 }
 
-template <class Src>
-__device__ __forceinline__ void relax_setup(const RoundsArgs &a, RelaxShared<Src> &rs, const Src &s0, const Src &s1) {
+template <class Src, class Op>
+__device__ __forceinline__ void relax_setup(const RoundsArgs &a, RelaxShared<Src, Op> &rs, const Src &s0,
+                                            const Src &s1) {
   if (threadIdx.x == 0) {
     for (int r = 0; r < 2; r++) {
       LbsArgs &l = rs.a[r];
@@ -397,13 +424,14 @@ __device__ __forceinline__ void relax_setup(const RoundsArgs &a, RelaxShared<Src
     }
     rs.s[0] = s0;
     rs.s[1] = s1;
+    rs.target = 0;
   }
 }
 
 // ------------------------------------------------------------ SSSP and CC
 
-// MinOp that also notes, per thread, whether it lowered a value below the
-// threshold and the smallest value at or above it that it wrote: the next
+// MinOp, in shared memory, that also notes whether the CTA lowered a value below
+// the threshold and the smallest value at or above it that it wrote: the next
 // round then needs no scan to learn that nothing near is left.
 template <bool kWeighted>
 struct MinRoundOp : MinOp<kWeighted> {
@@ -420,9 +448,19 @@ struct MinRoundOp : MinOp<kWeighted> {
     if (cand >= p) return;
     atomicMin(this->value + v, cand);
     atomicOr(this->next + (v >> 5), 1u << (v & 31));
+    if constexpr (!kWeighted) return;  // no threshold
     if (cand < thr) near = 1u;
-    else far_cand = min(far_cand, cand);
+    else if (cand < far_cand) atomicMin(&far_cand, cand);  // seldom: the smallest so far is read first
   }
+};
+
+// Eight records at a time do not fit: the tile loop spills 160 B a thread for
+// weighted ones (64 registers, four CTAs per SM) and 64 B for columns, 68 B and
+// none with four.  Resident SSSP of 0.3 M vertices 874 us with eight, 856 with four;
+// label propagation over the link, R-MAT 20, 1.02 ms and 0.98.
+template <bool kWeighted>
+struct OpGroup<MinRoundOp<kWeighted>> {
+  static constexpr int value = 4;
 };
 
 // SSSP from a.src (kWeighted; a.split: near/far with width a.delta) or label
@@ -442,39 +480,40 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
     LbsSh<Op> lbs;
     ScanShared scan;
   } sh;
-  __shared__ RelaxShared<SrcP<kWeighted>> rs;
+  __shared__ RelaxShared<SrcP<kWeighted>, Op> rs;
   RoundsState *st = a.st;
-  unsigned long long target = 0, t0 = 0;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-  if (lead) t0 = globaltimer_ns();
+  if (lead) st->ns_total -= globaltimer_ns();
   // initial values and frontier (SSSP/oneGraph/GraphMeta.h:376-381,
   // CC/onegraph/GraphMeta.h:341-345); the host cleared st
+  const bool resume = st->hand != 0;  // behind the relax of a round handed over
   const uint64_t gid = blockIdx.x * (uint64_t)kThreads + threadIdx.x, gsz = (uint64_t)gridDim.x * kThreads;
-  for (uint64_t v = gid; v < a.V; v += gsz) a.value[v] = kWeighted ? (v == a.src ? 1u : 0xffffffffu) : (uint32_t)v;
-  for (uint64_t w = gid; w < a.nwords; w += gsz) {
-    const uint64_t b = w * 32;
-    uint32_t x = 0;
-    if (!kWeighted) x = b + 32 <= a.V ? 0xffffffffu : (b >= a.V ? 0u : (1u << (a.V - b)) - 1u);
-    else if (w == a.src >> 5) x = 1u << (a.src & 31);
-    a.bm[0][w] = x;
-    a.bm[1][w] = 0u;
-    if (a.split) a.bm[2][w] = 0u;
+  if (!resume) {
+    for (uint64_t v = gid; v < a.V; v += gsz) a.value[v] = kWeighted ? (v == a.src ? 1u : 0xffffffffu) : (uint32_t)v;
+    for (uint64_t w = gid; w < a.nwords; w += gsz) {
+      const uint64_t b = w * 32;
+      uint32_t x = 0;
+      if (!kWeighted) x = b + 32 <= a.V ? 0xffffffffu : (b >= a.V ? 0u : (1u << (a.V - b)) - 1u);
+      else if (w == a.src >> 5) x = 1u << (a.src & 31);
+      a.bm[0][w] = x;
+      a.bm[1][w] = 0u;
+      if (a.split) a.bm[2][w] = 0u;
+    }
   }
   relax_setup(a, rs, s0, s1);
   if (lead)
     for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
-  if (!rounds_sync(st, target)) return;
-
-  uint32_t par = 0, far_min = 0xffffffffu;
   uint64_t t = 1ull + a.delta;
-  uint32_t thr = !a.split || t > 0xffffffffull ? 0xffffffffu : (uint32_t)t;
-  bool merge = false;
-  unsigned long long nsr = 0;
+  uint32_t par = resume ? st->par : 0u, far_min = resume ? st->far_min : 0xffffffffu;
+  uint32_t thr = resume ? st->thr : !a.split || t > 0xffffffffull ? 0xffffffffu : (uint32_t)t;
+  if (!rounds_sync(st, rs.target)) return;
+
+  bool merge = false, hand = false;
   for (uint32_t seq = 0;; seq++) {
     RoundSlot *slot = st->slot + (seq & 3u);
     if (a.split) scan_frontier<true, true>(a, sh.scan, a.bm[par], nullptr, a.bm[2], merge, thr, slot);
     else scan_frontier<false, true>(a, sh.scan, a.bm[par], nullptr, nullptr, false, 0u, slot);
-    if (!rounds_sync(st, target)) return;
+    if (!rounds_sync(st, rs.target)) return;
     if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
     const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
     const uint64_t n = (x0 >> kAppendShift) + (x1 >> kAppendShift);
@@ -492,27 +531,36 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
       st->edges_static += x0 & ((1ull << kAppendShift) - 1);
       st->edges_dynamic += x1 & ((1ull << kAppendShift) - 1);
     }
-    Op op;
-    op.value = a.value;
-    op.next = a.bm[par ^ 1];
-    op.err = &st->err;
-    op.V = a.V;
-    op.thr = thr;
-    op.near = 0;
-    op.far_cand = 0xffffffffu;
-    unsigned long long tr = 0;
-    if (lead && a.timer) tr = globaltimer_ns();
-    op = relax_lists(rs, sh.lbs, op, slot);
-    if (a.split) {
-      const int near = __syncthreads_or(op.near);
-      const uint32_t fc = block_min_u32(op.far_cand);
-      if (threadIdx.x == 0) {
-        if (near) slot->near = 1u;
-        if (fc != 0xffffffffu) atomicMin(&slot->far_cand, fc);
+    if (hands_over(a, list_tiles(x0), list_tiles(x1))) {
+      // the launch that relaxes them does not note what it lowers: the next
+      // scan is one at the present threshold
+      if (lead) {
+        st->hx[0] = x0;
+        st->hx[1] = x1;
+        st->par = par ^ 1u;
+        st->thr = thr;
+        st->far_min = far_min;
       }
+      hand = true;
+      break;
     }
-    if (!rounds_sync(st, target)) return;
-    if (lead && a.timer) nsr += globaltimer_ns() - tr;
+    if (threadIdx.x == 0) {
+      rs.op.value = a.value;
+      rs.op.next = a.bm[par ^ 1];
+      rs.op.err = &st->err;
+      rs.op.V = a.V;
+      rs.op.thr = thr;
+      rs.op.near = 0;
+      rs.op.far_cand = 0xffffffffu;
+    }
+    if (lead && a.timer) st->ns_relax -= globaltimer_ns();
+    relax_lists(rs, sh.lbs, slot);  // has a barrier before the first tile and after each
+    if (a.split && threadIdx.x == 0) {
+      if (rs.op.near) slot->near = 1u;
+      if (rs.op.far_cand != 0xffffffffu) atomicMin(&slot->far_cand, rs.op.far_cand);
+    }
+    if (!rounds_sync(st, rs.target)) return;
+    if (lead && a.timer) st->ns_relax += globaltimer_ns();
     par ^= 1u;
     merge = false;
     if (a.split && !slot->near) {
@@ -523,10 +571,11 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
       merge = true;
     }
   }
-  rounds_result(a);
+  if (!hand) rounds_result(a);
   if (lead) {
-    st->ns_relax = nsr;
-    st->ns_total = globaltimer_ns() - t0;
+    st->hand = hand ? kHandRelax : 0u;
+    st->done = !hand;
+    st->ns_total += globaltimer_ns();
     rounds_post(a);
   }
 }
@@ -563,9 +612,8 @@ __global__ void __launch_bounds__(kThreads) k_bfs_init(const __grid_constant__ R
   }
   if (gid == 0) {
     RoundsState *st = a.st;
-    for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
     st->bar = 0;
-    st->err = st->posted = 0;
+    st->err = st->posted = st->hand = 0;
     st->iterations = st->frontier_sum = st->edges_static = st->edges_dynamic = 0;
     st->ns_total = st->ns_relax = 0;
     st->unexplored = a.E;
@@ -610,10 +658,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_bfs_small(const __grid_consta
     if (tid == 0) {
       sm.cnt[0] = n;
       sm.nz = sm.es = 0;
-      // the last k_bfs_rounds launch, if any, has ended: the next one's
-      // barriers and counters start afresh
-      st->bar = 0;
-      for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
+      st->bar = 0;  // the last k_bfs_rounds launch, if any, has ended: the next one's barriers start afresh
     }
   }
   __syncthreads();
@@ -778,27 +823,48 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
     LbsSh<BfsOp> lbs;
     ScanShared scan;
   } sh;
-  __shared__ RelaxShared<SrcP<false>> rs;
+  __shared__ RelaxShared<SrcP<false>, BfsOp> rs;
   RoundsState *st = a.st;
-  unsigned long long target = 0, t0 = 0;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   if (st->done) {  // set before this launch: every CTA reads the same
     rounds_result(a);
     if (lead) rounds_post(a);
     return;
   }
-  if (lead) t0 = globaltimer_ns();
+  if (lead) st->ns_total -= globaltimer_ns();
   relax_setup(a, rs, s0, s1);
   bool bottom = st->bottom, counted = st->counted, done = false;
-  uint32_t level = st->level, par = st->par, streak = 0;
+  uint32_t level = st->level, par = st->par, streak = 0, hand = 0;
   uint64_t unexplored = st->unexplored, fn = st->fn;
-  if (!rounds_sync(st, target)) return;  // every CTA has read the state that is rewritten at the end
-  for (uint32_t seq = 0;; seq++) {
+  // After a bottom-up level: accounting and the direction of the next one; true
+  // when it reached nothing.
+  auto counted_bottom = [&](const unsigned long long *bu) {
+    const uint64_t nn = bu[0];
+    if (lead) {
+      st->iterations++;
+      st->frontier_sum += fn;
+      st->edges_dynamic += bu[2];
+      st->edges_static += bu[3];
+    }
+    unexplored -= min(unexplored, (uint64_t)bu[1]);
+    if (nn == 0) return true;
+    bottom = !(nn < a.V / kBfsBeta && nn < fn);  // small and shrinking: top-down again
+    fn = nn;
+    counted = true;
+    level++;
+    par ^= 1u;
+    return false;
+  };
+  if (st->hand == kHandBottomUp) done = counted_bottom(st->hbu);
+  if (lead)
+    for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
+  if (!rounds_sync(st, rs.target)) return;  // every CTA has read the state that is rewritten at the end
+  for (uint32_t seq = 0; !done; seq++) {
     uint32_t *cur = a.bm[par], *next = a.bm[par ^ 1];
     RoundSlot *slot = st->slot + (seq & 3u);
     if (!bottom) {
       scan_frontier<false, false>(a, sh.scan, cur, next, nullptr, false, 0u, slot);
-      if (!rounds_sync(st, target)) return;
+      if (!rounds_sync(st, rs.target)) return;
       if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
       const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
       const uint64_t n0 = x0 >> kAppendShift, n = n0 + (x1 >> kAppendShift);
@@ -827,48 +893,49 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
           st->edges_static += m0;
           st->edges_dynamic += mf - m0;
         }
-        BfsOp op{a.bm[2], next, a.value, &st->err, a.V, level + 1};
-        unsigned long long tr = 0;
-        if (lead && a.timer) tr = globaltimer_ns();
-        relax_lists(rs, sh.lbs, op, slot);
-        if (!rounds_sync(st, target)) return;
-        if (lead && a.timer) st->ns_relax += globaltimer_ns() - tr;
+        if (hands_over(a, list_tiles(x0), list_tiles(x1))) {
+          if (lead) {
+            st->hx[0] = x0;
+            st->hx[1] = x1;
+          }
+          hand = kHandRelax;
+          level++;
+          par ^= 1u;
+          break;
+        }
+        if (threadIdx.x == 0) rs.op = BfsOp{a.bm[2], next, a.value, &st->err, a.V, level + 1};
+        if (lead && a.timer) st->ns_relax -= globaltimer_ns();
+        relax_lists(rs, sh.lbs, slot);
+        if (!rounds_sync(st, rs.target)) return;
+        if (lead && a.timer) st->ns_relax += globaltimer_ns();
+        level++;
+        par ^= 1u;
+        continue;
       }
     }
-    if (bottom) {
-      streak = 0;
-      bfs_bottom_up_level(a, s0, s1, cur, next, level + 1, slot);
-      if (!rounds_sync(st, target)) return;
-      if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
-      const uint64_t nn = slot->bu[0];
-      if (lead) {
-        st->iterations++;
-        st->frontier_sum += fn;
-        st->edges_dynamic += slot->bu[2];
-        st->edges_static += slot->bu[3];
-      }
-      unexplored -= min(unexplored, (uint64_t)slot->bu[1]);
-      if (nn == 0) {
-        done = true;
-        break;
-      }
-      bottom = !(nn < a.V / kBfsBeta && nn < fn);  // small and shrinking: top-down again
-      fn = nn;
-      counted = true;
+    streak = 0;
+    if (a.hand_bottom) {
+      hand = kHandBottomUp;
+      break;
     }
-    level++;
-    par ^= 1u;
+    bfs_bottom_up_level(a, s0, s1, cur, next, level + 1, slot);
+    if (!rounds_sync(st, rs.target)) return;
+    if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
+    done = counted_bottom(slot->bu);
   }
   if (done) rounds_result(a);
   if (lead) {
     st->done = done;
-    st->small = !done;
+    st->small = !done && !hand;
+    st->hand = hand;
     st->level = level;
     st->par = par;
     st->counted = counted;
-    st->bottom = 0;
+    st->bottom = hand == kHandBottomUp;
+    st->fn = fn;
+    st->hbu[0] = st->hbu[1] = st->hbu[2] = st->hbu[3] = 0;
     st->unexplored = unexplored;
-    st->ns_total += globaltimer_ns() - t0;
+    st->ns_total += globaltimer_ns();
     rounds_post(a);
   }
 }

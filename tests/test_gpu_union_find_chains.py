@@ -45,8 +45,8 @@ def path(n, step=1):
 
 
 CASES = {
-    "rows": lambda: grid(701, 499), "columns": lambda: grid(13, 40_003), "wide": lambda: grid(1_200_000, 2),
-    "permuted": lambda: grid(701, 499, 3), "path": lambda: path(2_000_003), "backwards": lambda: path(65_537, -1),
+    "rows": lambda: grid(701, 499), "columns": lambda: grid(13, 40_003), "wide": lambda: grid(350_000, 2),
+    "permuted": lambda: grid(701, 499, 3), "path": lambda: path(600_003), "backwards": lambda: path(65_537, -1),
     "comb": lambda: comb(50_000, 300),
 }
 
