@@ -475,8 +475,8 @@ int og_engine_clone(og_engine *parent, og_engine **out);
  *   cooperative kernel that takes every per-round decision itself (BFS: with
  *   a one-CTA kernel for small frontiers beside it; rounds of very many edges
  *   are relaxed by a launch of their own in between), in direct mode or on a
- *   fully resident graph of fewer than 2^28 vertices and 2^36 edges; other
- *   engines keep the host loop.  OG_LOOP_HOST waits for each round's
+ *   fully resident graph whose vertex and edge counts together take at most
+ *   64 bits; other engines keep the host loop.  OG_LOOP_HOST waits for each round's
  *   counts on the host.  Results are identical. */
 #define OG_PARAM_LEVEL_LOOP 4
 #define OG_LOOP_AUTO 0

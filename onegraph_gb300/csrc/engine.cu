@@ -1365,8 +1365,8 @@ int relax_handed(og_engine *e, const RoundsState &h, Src s0, Src s1, Op op) {
   uint64_t n[2];
   for (int r = 0; r < 2; r++) {
     Counts &c = e->counts_h[r];
-    c.n = (uint32_t)(h.hx[r] >> kAppendShift);
-    c.total = h.hx[r] & ((1ull << kAppendShift) - 1);
+    c.n = (uint32_t)(h.hx[r] >> append_shift(e->g->E));
+    c.total = append_edges(h.hx[r], append_shift(e->g->E));
     a[r] = lbs_args(e, r, 0, c.total, true, r ? e->g->E : e->plan.static_edges);
     a[r].err = &e->rounds_d->err;
     n[r] = lbs_grid(0, c.total);
@@ -1412,6 +1412,7 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   a.split = a.delta ? 1u : 0u;
   a.dopt = algo == OG_ALGO_BFS && e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1;
   a.timer = e->relax_timer;
+  a.shift = append_shift(a.E);
   a.hand_hbm = kHandHbm;
   a.hand_link = algo == OG_ALGO_BFS ? ~0ull : kHandLink;
   a.hand_bottom = a.V >= kHandBottomVertices;

@@ -32,9 +32,18 @@
 namespace og {
 
 // A list reservation packs both of its counters into 64 bits: vertices above,
-// edge positions below.  Larger graphs take the host-driven loop.
-constexpr uint32_t kAppendShift = 36;
-inline bool rounds_fit(uint64_t V, uint64_t E) { return V < (1ull << 28) && E < (1ull << kAppendShift); }
+// edge positions below, as many bits as the graph's edge count takes.  Graphs
+// whose two counts do not fit take the host-driven loop (2^28 vertices go with
+// up to 2^35 edges, 240 GB of records).
+inline uint32_t append_shift(uint64_t E) {
+  uint32_t b = 1;
+  while (E >> b) b++;
+  return b;
+}
+inline bool rounds_fit(uint64_t V, uint64_t E) { return append_shift(V) + append_shift(E) <= 64; }
+__host__ __device__ __forceinline__ uint64_t append_edges(unsigned long long app, uint32_t shift) {
+  return app & ((1ull << shift) - 1);
+}
 
 // Counters of one scan and the relax after it.  Four of them are used in turn:
 // after the barrier that ends scan s, CTA 0 clears the one of scan s + 2, whose
@@ -80,6 +89,7 @@ struct RoundsArgs {
   RoundsState *post;  // the host's copy, page-locked
   uint32_t *result;   // when not null: page-locked, takes the values of a query that has ended
   uint32_t src, delta, split, dopt, timer;
+  uint32_t shift;  // of the vertex counter in a list reservation
   uint64_t hand_hbm, hand_link;  // rounds of more tiles are handed over (hands_over)
   uint32_t hand_bottom;          // bottom-up levels are
 };
@@ -246,11 +256,11 @@ __device__ __forceinline__ uint32_t scan_group(const RoundsArgs &a, ScanWarp &sh
     const uint32_t tn = __shfl_sync(0xffffffffu, ic, 31);
     if (tn == 0) continue;
     unsigned long long base = 0;
-    if (lane == 31) base = atomicAdd(app, ((unsigned long long)tn << kAppendShift) | is);
+    if (lane == 31) base = atomicAdd(app, ((unsigned long long)tn << a.shift) | is);
     base = __shfl_sync(0xffffffffu, base, 31);
     const uint64_t te = __shfl_sync(0xffffffffu, is, 31);
-    uint32_t pos = (uint32_t)(base >> kAppendShift);
-    uint64_t ep = base & ((1ull << kAppendShift) - 1);
+    uint32_t pos = (uint32_t)(base >> a.shift);
+    uint64_t ep = append_edges(base, a.shift);
     uint32_t *list = a.list[r], *tile = a.tile[r];
     uint64_t *pref = a.pref[r];
     if ((uint64_t)pos + tn > a.list_cap[r] || (ep + te + kTile - 1) / kTile > a.tile_cap[r]) {
@@ -337,8 +347,8 @@ __device__ __noinline__ void scan_frontier(const RoundsArgs &a, ScanShared &shar
   }
 }
 
-__device__ __forceinline__ uint64_t list_tiles(unsigned long long app) {
-  return ((app & ((1ull << kAppendShift) - 1)) + kTile - 1) / kTile;
+__device__ __forceinline__ uint64_t list_tiles(unsigned long long app, uint32_t shift) {
+  return (append_edges(app, shift) + kTile - 1) / kTile;
 }
 
 __device__ __forceinline__ void slot_clear(RoundSlot *s) {
@@ -361,6 +371,7 @@ struct RelaxShared {
   uint32_t b[2];
   Op op;
   unsigned long long target;
+  uint32_t shift;
 };
 
 // Relax of both regions' lists.  A CTA's first tile is its index in the grid
@@ -379,8 +390,8 @@ __device__ __noinline__ void relax_lists(RelaxShared<Src, Op> &rs, LbsSh<Op> &sh
     for (int r = 0; r < 2; r++) {
       const unsigned long long x = slot->app[r];
       LbsArgs &l = rs.a[r];
-      l.n = (uint32_t)(x >> kAppendShift);
-      l.total = l.pos_end = x & ((1ull << kAppendShift) - 1);
+      l.n = (uint32_t)(x >> rs.shift);
+      l.total = l.pos_end = append_edges(x, rs.shift);
     }
   }
   __syncthreads();
@@ -425,6 +436,7 @@ __device__ __forceinline__ void relax_setup(const RoundsArgs &a, RelaxShared<Src
     rs.s[0] = s0;
     rs.s[1] = s1;
     rs.target = 0;
+    rs.shift = a.shift;
   }
 }
 
@@ -516,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
     if (!rounds_sync(st, rs.target)) return;
     if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
     const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
-    const uint64_t n = (x0 >> kAppendShift) + (x1 >> kAppendShift);
+    const uint64_t n = (x0 >> a.shift) + (x1 >> a.shift);
     if (a.split) far_min = merge ? slot->far_min : min(far_min, slot->far_min);
     if (n == 0) {
       if (!a.split || far_min == 0xffffffffu) break;
@@ -528,10 +540,10 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
     if (lead) {
       st->iterations++;
       st->frontier_sum += n;
-      st->edges_static += x0 & ((1ull << kAppendShift) - 1);
-      st->edges_dynamic += x1 & ((1ull << kAppendShift) - 1);
+      st->edges_static += append_edges(x0, a.shift);
+      st->edges_dynamic += append_edges(x1, a.shift);
     }
-    if (hands_over(a, list_tiles(x0), list_tiles(x1))) {
+    if (hands_over(a, list_tiles(x0, a.shift), list_tiles(x1, a.shift))) {
       // the launch that relaxes them does not note what it lowers: the next
       // scan is one at the present threshold
       if (lead) {
@@ -867,8 +879,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
       if (!rounds_sync(st, rs.target)) return;
       if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
       const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
-      const uint64_t n0 = x0 >> kAppendShift, n = n0 + (x1 >> kAppendShift);
-      const uint64_t m0 = x0 & ((1ull << kAppendShift) - 1), mf = m0 + (x1 & ((1ull << kAppendShift) - 1));
+      const uint64_t n0 = x0 >> a.shift, n = n0 + (x1 >> a.shift);
+      const uint64_t m0 = append_edges(x0, a.shift), mf = m0 + append_edges(x1, a.shift);
       if (n == 0) {
         done = true;
         break;
@@ -893,7 +905,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
           st->edges_static += m0;
           st->edges_dynamic += mf - m0;
         }
-        if (hands_over(a, list_tiles(x0), list_tiles(x1))) {
+        if (hands_over(a, list_tiles(x0, a.shift), list_tiles(x1, a.shift))) {
           if (lead) {
             st->hx[0] = x0;
             st->hx[1] = x1;
