@@ -64,8 +64,11 @@ int og_k_gather(const uint32_t *list, const uint64_t *pref, const uint32_t *tile
  * one-CTA launch, on a signal that is never given.  which = 0: the
  * compaction look-back of a tile whose predecessor never publishes;
  * which = 1: the persistent kernel's grid barrier expecting one CTA more than
- * the launch has.  The wait gives up after spin_limit polls (the engine uses
- * 2^24), sets its error bit and lets the kernel end, so this returns
+ * the launch has; which = 2: the same of the device-driven rounds' barrier;
+ * which = 3: a staged round (two CTAs) whose ring slots nobody hands over, which
+ * gives up after 5000 polls whatever spin_limit is.  The
+ * wait gives up after spin_limit polls (the engine uses 2^24, and more on large
+ * graphs for the barriers of whole queries), sets its error bit and lets the kernel end, so this returns
  * OG_E_TIMEOUT and the CUDA context stays usable.  No reference counterpart. */
 int og_k_wait_check(int which, uint32_t spin_limit);
 

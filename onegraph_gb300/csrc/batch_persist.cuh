@@ -64,6 +64,7 @@ struct PersistArgs {
   uint32_t *defer;            // bottom-up vertices handed to the pull pass (bitmap, zero between levels)
   uint32_t Vs;                // first dynamic vertex
   uint32_t dopt;              // bottom-up sources allowed (the graph is symmetric)
+  uint32_t spin_limit;        // of a grid barrier (wait_limit)
   __device__ __forceinline__ unsigned long long *act_slot(uint32_t level) const {
     return stat + 4 + (level & 1u);
   }
@@ -75,11 +76,11 @@ struct PersistArgs {
 constexpr uint64_t kBatchAlpha = 14, kBatchBeta = 24;
 
 // Grid-wide barrier of a cooperative launch: the last of `expected` CTAs to
-// arrive (default: the whole grid) releases the others by bumping the
+// arrive (0: the whole grid) releases the others by bumping the
 // generation word.  A wait longer than spin_limit polls sets kErrBarrier and
 // returns false instead of hanging.
-__device__ __forceinline__ bool grid_barrier(unsigned int *bar, uint32_t *err, uint32_t expected = 0,
-                                             uint32_t spin_limit = kSpinLimit) {
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, uint32_t *err, uint32_t expected,
+                                             uint32_t spin_limit) {
   __shared__ int s_ok;
   if (expected == 0) expected = gridDim.x;
   __syncthreads();
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(BLOCK, (ITEMS <= 4 ? 1024 : 512) / BLOCK) k_ba
     uint32_t exc;
     uint64_t exe, dyn_td;
     count_list<BLOCK>(a, sh, cur_any, wb, we, 0, a.dopt ? cur : nullptr, td, exc, exe, dyn_td);
-    if (!grid_barrier(a.bar, a.err)) return;
+    if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
     // ---- 2. grand totals, then the bottom-up and the top-down sources
     grid_totals<BLOCK>(a, sh);
     const uint64_t total_n = sh.red_tn, total_e = sh.red_te;
@@ -728,12 +729,12 @@ __global__ void __launch_bounds__(BLOCK, (ITEMS <= 4 ? 1024 : 512) / BLOCK) k_ba
     }
     if (bu) {
       bottom_up_scan<BLOCK>(a, bu, cur, next, next_any);
-      if (!grid_barrier(a.bar, a.err)) return;
+      if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
       // the deferred vertices' remaining records, edge-balanced (the pull
       // pass counts the records it reads)
       uint64_t dyn;
       count_list<BLOCK>(a, sh, a.defer, wb, we, kBuLaneRecords, nullptr, 0, exc, exe, dyn);
-      if (!grid_barrier(a.bar, a.err)) return;
+      if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
       grid_totals<BLOCK>(a, sh);
       const uint64_t dn = sh.red_tn, de = sh.red_te;
       if (dn) {
@@ -743,10 +744,10 @@ __global__ void __launch_bounds__(BLOCK, (ITEMS <= 4 ? 1024 : 512) / BLOCK) k_ba
         }
         write_list<TILE>(a, a.defer, wb, we, kBuLaneRecords, nullptr, 0, sh.red_n + exc, sh.red_e + exe, dn,
                          de);
-        if (!grid_barrier(a.bar, a.err)) return;
+        if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
         expand_tiles<BLOCK, ITEMS, true>(a, sh, dn, de, kBuLaneRecords, bu, cur, next, next_any);
         // the list buffers are rebuilt for the top-down sources below
-        if (!grid_barrier(a.bar, a.err)) return;
+        if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
       }
     }
     if (total_n) {
@@ -757,10 +758,10 @@ __global__ void __launch_bounds__(BLOCK, (ITEMS <= 4 ? 1024 : 512) / BLOCK) k_ba
         break;
       }
       write_list<TILE>(a, cur_any, wb, we, 0, a.dopt ? cur : nullptr, td, td_pos, td_ep, total_n, total_e);
-      if (!grid_barrier(a.bar, a.err)) return;
+      if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
       expand_tiles<BLOCK, ITEMS, false>(a, sh, total_n, total_e, 0, td, cur, next, next_any);
     }
-    if (!grid_barrier(a.bar, a.err)) return;
+    if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
     // ---- 4. settle the deferred vertices; per-source counts of the newly
     //         reached vertices (and, for top-down sources, their degree
     //         sums), depths, and clearing of the consumed frontier
@@ -778,7 +779,7 @@ __global__ void __launch_bounds__(BLOCK, (ITEMS <= 4 ? 1024 : 512) / BLOCK) k_ba
       atomicAdd(a.smf_slot(level + 1) + threadIdx.x, sh.msum[threadIdx.x]);
     if (threadIdx.x == 0 && sh.act) atomicOr(a.act_slot(level + 1), sh.act);
     // the next level reads the counts and masks written above by other CTAs
-    if (!grid_barrier(a.bar, a.err)) return;
+    if (!grid_barrier(a.bar, a.err, 0, a.spin_limit)) return;
     unsigned long long *tm = cur;
     cur = next;
     next = tm;

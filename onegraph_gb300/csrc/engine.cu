@@ -1413,6 +1413,7 @@ int run_rounds(og_engine *e, int algo, uint32_t src, og_stats &st) {
   a.dopt = algo == OG_ALGO_BFS && e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1;
   a.timer = e->relax_timer;
   a.shift = append_shift(a.E);
+  a.spin_limit = wait_limit(a.E);
   a.hand_hbm = kHandHbm;
   a.hand_link = algo == OG_ALGO_BFS ? ~0ull : kHandLink;
   a.hand_bottom = a.V >= kHandBottomVertices;
@@ -1840,6 +1841,7 @@ int enqueue_persist(og_engine *e, uint32_t n, int ci, uint32_t *depth_d, uint8_t
   a.defer = e->bm[2];
   a.Vs = e->Vs;
   a.dopt = batch_dopt(e);
+  a.spin_limit = wait_limit(e->g->E);
   RC(launch_persist(e, ci, a, s));
   CK(cudaMemcpyAsync(e->hist_h, e->hist_d, 8ull * kMaxBatchLevels * 64, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(e->pmisc_h, e->bar_d, 64, cudaMemcpyDeviceToHost, s));
@@ -2764,7 +2766,8 @@ int run_cc_uf(og_engine *e, og_stats &st) {
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(1, occ) * e->sms, V / 1024 + 1);
     uint32_t v = V, *p = par;
     RoundsState *state = e->rounds_d + jumps++;  // cleared by k_uf_init
-    void *args[4] = {&p, &v, &state, &e->err_d};
+    uint32_t limit = wait_limit(V);
+    void *args[5] = {&p, &v, &state, &limit, &e->err_d};
     CK(cudaLaunchCooperativeKernel((const void *)k_uf_jump, dim3(grid), dim3(kThreads), args, 0, s));
     e->launches++;
     return OG_OK;

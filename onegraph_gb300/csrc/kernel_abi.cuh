@@ -17,6 +17,7 @@
 #include "batch_persist.cuh"
 #include "kernels.cuh"
 #include "og_internal.hpp"
+#include "rounds.cuh"
 
 namespace kabi {
 
@@ -81,10 +82,54 @@ __global__ void k_wait_check(int which, uint32_t spin_limit, uint32_t *scratch, 
     uint64_t pe;
     int bad;
     lookback_prefix(lb, 1, 1, 0, 0, err, pn, pe, bad, spin_limit);
-  } else {
+  } else if (which == 1) {
     // a barrier expecting one CTA more than the launch holds
     grid_barrier((unsigned int *)scratch, err, gridDim.x + 1, spin_limit);
+  } else {
+    RoundsState *st = (RoundsState *)scratch;
+    unsigned long long target = 1;  // one arrival more than there are CTAs
+    if (rounds_sync(st, target, spin_limit)) return;
+    if (threadIdx.x == 0) atomicOr(err, st->err);
   }
+}
+
+// A staged round of one tile (vertex 0 with one edge to itself) on a ring whose
+// slots no step will ever find in the state it waits for: the gather and the
+// relax both give up, and neither writes.
+constexpr uint32_t kCheckPolls = 5000;
+int stage_wait_check(char *scratch, uint32_t *err) {
+  struct Host {
+    uint32_t list[4], tile[4], words[4], value[4], next[4], ticket[4], state[4];
+    uint64_t pref[2], off[2];
+    uint32_t stage[2];
+  } h;
+  memset(&h, 0, sizeof h);
+  h.pref[1] = h.off[1] = 1;
+  h.state[0] = h.state[1] = 77;
+  h.value[0] = 5;
+  h.stage[0] = h.stage[1] = 0xdeadbeefu;
+  CK(cudaMemcpy(scratch, &h, sizeof h, cudaMemcpyHostToDevice));
+  Host *d = (Host *)scratch;
+  LbsArgs a;
+  a.list = d->list;
+  a.pref = d->pref;
+  a.tile_first = d->tile;
+  a.n = 1;
+  a.total = a.pos_end = 1;
+  a.pos_begin = 0;
+  a.off = d->off;
+  a.stage_base = 0;
+  a.edge_bound = 1;
+  a.err = err;
+  const StageRingT<kCheckPolls> ring{d->state, d->ticket, 2, 1};
+  const SrcP<false> rec{d->words, 1, 1, 0};
+  k_stage_round<<<2, kThreads>>>(a, rec, DstU{d->stage}, DstU{d->stage + 1}, SrcU{d->stage}, SrcU{d->stage + 1}, 1,
+                                 MinOp<false>{d->value, d->next, err, 1}, ring);
+  CK(cudaGetLastError());
+  CK(cudaMemcpy(&h, scratch, sizeof h, cudaMemcpyDeviceToHost));
+  if (h.stage[0] != 0xdeadbeefu || h.stage[1] != 0xdeadbeefu || h.value[0] != 5 || h.next[0] || h.state[0] != 77)
+    return fail(OG_E_STATE, "a staged step that gave up has written");
+  return OG_OK;
 }
 
 // Streams `words` 16-byte words of page-locked host memory through the SMs
@@ -182,20 +227,28 @@ extern "C" int og_k_gather(const uint32_t *list, const uint64_t *pref, const uin
 
 extern "C" int og_k_wait_check(int which, uint32_t spin_limit) {
   clear_error();
-  if (which != 0 && which != 1) return fail(OG_E_ARG, "og_k_wait_check: which = %d", which);
+  if (which < 0 || which > 3) return fail(OG_E_ARG, "og_k_wait_check: which = %d", which);
   cudaGetLastError();
   ErrWord w;
   uint32_t *scratch = nullptr;
   CK(cudaMalloc(&w.d, 4));
-  if (cudaMalloc(&scratch, 256) != cudaSuccess) return fail(OG_E_CUDA, "og_k_wait_check: cudaMalloc");
+  constexpr size_t kScratch = 4096;
+  static_assert(sizeof(RoundsState) <= kScratch, "scratch of the checks");
+  if (cudaMalloc(&scratch, kScratch) != cudaSuccess) return fail(OG_E_CUDA, "og_k_wait_check: cudaMalloc");
   struct Free {
     uint32_t *p;
     ~Free() { cudaFree(p); }
   } free_scratch{scratch};
   CK(cudaMemset(w.d, 0, 4));
-  CK(cudaMemset(scratch, 0, 256));
-  k_wait_check<<<1, which == 0 ? 32 : kThreads>>>(which, spin_limit, scratch, w.d);
-  return finish(nullptr, w, which == 0 ? "compaction look-back" : "grid barrier");
+  CK(cudaMemset(scratch, 0, kScratch));
+  if (which == 3) {
+    const int rc = stage_wait_check((char *)scratch, w.d);
+    if (rc != OG_OK) return rc;
+  } else {
+    k_wait_check<<<1, which == 0 ? 32 : kThreads>>>(which, spin_limit, scratch, w.d);
+  }
+  const char *const what[] = {"compaction look-back", "grid barrier", "rounds barrier", "staged round"};
+  return finish(nullptr, w, what[which]);
 }
 
 extern "C" int og_link_probe(const void *host, uint64_t bytes, int mode, int reps, double *gbs) {

@@ -38,7 +38,14 @@ constexpr uint32_t kErrEdgeIndex = 2u;   // edge index outside the array
 constexpr uint32_t kErrVertex = 4u;      // column >= V
 constexpr uint32_t kErrTileMap = 8u;     // LBS tile map inconsistent
 
+// Polls after which a wait within a launch gives up: 2^24 (several seconds) for
+// waits on work of fixed size; between the phases of a whole query, which may
+// read every edge, a poll more for every 64 edges (a phase that gets through 0.2 G
+// edges a second still ends in time).
 constexpr uint32_t kSpinLimit = 1u << 24;
+inline uint32_t wait_limit(uint64_t E) {
+  return (uint32_t)((kSpinLimit + E / 64) < (1ull << 31) ? kSpinLimit + E / 64 : 1ull << 31);
+}
 constexpr uint32_t kErrBarrier = 16u;  // a bounded wait within a launch gave up
 
 // Nanosecond global timer (the same clock on every SM).
@@ -1133,17 +1140,22 @@ __global__ void __launch_bounds__(kThreads, 5) k_lbs_pair(LbsArgs a0, Src0 s0, L
 // tickets was slower (4.19 to 3.41 ms).
 constexpr uint32_t kRingSlots = 2048;  // most slots in use: 4 M positions, more than are ever in flight
 constexpr uint32_t kRingPad = 32;      // words before them: the ticket's cache line
-struct StageRing {
+// kLimit: polls of a wait for a slot (a constant: read from the arguments it cost
+// delta PageRank of 777777 vertices 3.10 ms instead of 3.02).
+template <uint32_t kLimit>
+struct StageRingT {
   uint32_t *state, *ticket;  // zeroed before the launch
   uint32_t slots, half;      // half: slots of buffer 0
 };
+using StageRing = StageRingT<kSpinLimit>;
 struct StageStep {
   uint64_t tile, base;  // base: position minus buffer entry (mod 2^64)
   uint32_t slot, want;  // want: the state this step waits for; odd: relax
   uint32_t buf, ready;
 };
 // This CTA's step, from the next ticket.
-__device__ __forceinline__ void stage_take(const StageRing &g, uint64_t ntiles, StageStep &step) {
+template <class Ring>
+__device__ __forceinline__ void stage_take(const Ring &g, uint64_t ntiles, StageStep &step) {
   if (threadIdx.x == 0) {
     const uint64_t i = atomicAdd(g.ticket, 1u), lead = min((uint64_t)(g.slots / 2), ntiles);
     const uint64_t j = i - lead, pairs = ntiles - lead;  // j: valid for i >= lead
@@ -1172,9 +1184,10 @@ __device__ __forceinline__ void stage_take(const StageRing &g, uint64_t ntiles, 
 // wait sets kErrBarrier, which ends the waits of the others).  The polls are
 // relaxed and one fence follows: it also drops lines of the slot's earlier
 // use from L1.
-__device__ __forceinline__ void stage_wait(const StageRing &g, StageStep &x, uint32_t *err) {
+template <uint32_t kLimit>
+__device__ __forceinline__ void stage_wait(const StageRingT<kLimit> &g, StageStep &x, uint32_t *err) {
   for (uint32_t spins = 0; ld_relaxed(g.state + x.slot) != x.want;) {
-    if (++spins > kSpinLimit || ((spins & 255u) == 0 && (ld_relaxed(err) & kErrBarrier))) {
+    if (++spins > kLimit || ((spins & 255u) == 0 && (ld_relaxed(err) & kErrBarrier))) {
       atomicOr(err, kErrBarrier);
       return;
     }
@@ -1184,12 +1197,14 @@ __device__ __forceinline__ void stage_wait(const StageRing &g, StageStep &x, uin
   x.ready = 1;
 }
 // All threads: waits for the slot; false: gave up.
-__device__ __forceinline__ bool stage_ready(const StageRing &g, StageStep &x, uint32_t *err) {
+template <class Ring>
+__device__ __forceinline__ bool stage_ready(const Ring &g, StageStep &x, uint32_t *err) {
   if (threadIdx.x == 0 && !x.ready) stage_wait(g, x, err);
   __syncthreads();
   return x.ready != 0;
 }
-__device__ __forceinline__ void stage_post(const StageRing &g, StageStep &x, uint32_t *err) {
+template <class Ring>
+__device__ __forceinline__ void stage_post(const Ring &g, StageStep &x, uint32_t *err) {
   __syncthreads();
   if (threadIdx.x != 0) return;
   if (!x.ready) stage_wait(g, x, err);  // a gather that stopped before its stores
@@ -1199,13 +1214,13 @@ __device__ __forceinline__ void stage_post(const StageRing &g, StageStep &x, uin
 // The gather of a staged round as an edge op: position pos goes to entry
 // pos - base of a staging buffer.  The slot is waited for after the link reads
 // have been issued, so a step holds it for its stores alone.
-template <class Dst>
+template <class Dst, class Ring>
 struct GatherOp {
   using Val = uint32_t;
   static constexpr bool kNeedVal = false;
   Dst stage;
   uint64_t base;
-  const StageRing *ring;
+  const Ring *ring;
   StageStep *step;  // shared memory
   uint32_t *err;
   __device__ __forceinline__ bool commit() const { return stage_ready(*ring, *step, err); }
@@ -1221,12 +1236,12 @@ struct GatherOp {
   }
 };
 
-template <class PSrc, class Dst, class Src, class Op>
+template <class PSrc, class Dst, class Src, class Op, class Ring>
 __global__ void __launch_bounds__(kThreads, 5) k_stage_round(const __grid_constant__ LbsArgs a, PSrc ps, Dst d0, Dst d1,
                                                              Src s0, Src s1, uint64_t cap, Op op,
-                                                             const __grid_constant__ StageRing ring) {
+                                                             const __grid_constant__ Ring ring) {
   __shared__ union {
-    LbsSh<GatherOp<Dst>> gather;
+    LbsSh<GatherOp<Dst, Ring>> gather;
     LbsSh<Op> relax;
   } sh;
   __shared__ StageStep x;
@@ -1239,7 +1254,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_stage_round(const __grid_consta
     r.edge_bound = cap;
     lbs_tile(r, x.buf ? s1 : s0, op, sh.relax, x.tile);
   } else {
-    lbs_tile(a, ps, GatherOp<Dst>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh.gather, x.tile);
+    lbs_tile(a, ps, GatherOp<Dst, Ring>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh.gather, x.tile);
   }
   stage_post(ring, x, a.err);
 }
@@ -1801,7 +1816,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_stage_round_pr(const __grid_con
                                                                 Dst d1, Src s0, Src s1, uint64_t cap,
                                                                 const __grid_constant__ PrArgs p,
                                                                 const __grid_constant__ StageRing ring) {
-  __shared__ LbsSh<GatherOp<Dst>> sh;
+  __shared__ LbsSh<GatherOp<Dst, StageRing>> sh;
   __shared__ StageStep x;
   stage_take(ring, (a.total + kTile - 1) / kTile, x);
   if (x.want & 1u) {
@@ -1813,7 +1828,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_stage_round_pr(const __grid_con
     q.nwords = cap;
     pr_tile<true>(r, x.buf ? s1 : s0, q, x.tile);
   } else {
-    lbs_tile(a, ps, GatherOp<Dst>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh, x.tile);
+    lbs_tile(a, ps, GatherOp<Dst, StageRing>{x.buf ? d1 : d0, x.base, &ring, &x, a.err}, sh, x.tile);
   }
   stage_post(ring, x, a.err);
 }

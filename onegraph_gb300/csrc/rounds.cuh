@@ -90,6 +90,7 @@ struct RoundsArgs {
   uint32_t *result;   // when not null: page-locked, takes the values of a query that has ended
   uint32_t src, delta, split, dopt, timer;
   uint32_t shift;  // of the vertex counter in a list reservation
+  uint32_t spin_limit;
   uint64_t hand_hbm, hand_link;  // rounds of more tiles are handed over (hands_over)
   uint32_t hand_bottom;          // bottom-up levels are
 };
@@ -136,9 +137,9 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
 // the grid size with every barrier.  The polls are relaxed and one acquire fence follows
 // them: an acquiring poll drops the SM's whole L1 each time, under the CTAs
 // that still work (a round's relax, resident SSSP of 0.3 M vertices: 13-15 us
-// on average so, 9 us now).  A wait longer than kSpinLimit polls sets kErrBarrier and returns
-// false instead of hanging.
-__device__ __forceinline__ bool rounds_sync(RoundsState *st, unsigned long long &target) {
+// on average so, 9 us now).  A wait longer than `limit` polls (wait_limit) sets
+// kErrBarrier and returns false instead of hanging.
+__device__ __forceinline__ bool rounds_sync(RoundsState *st, unsigned long long &target, uint32_t limit) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -148,7 +149,7 @@ __device__ __forceinline__ bool rounds_sync(RoundsState *st, unsigned long long 
     atomicAdd(&st->bar, 1ull);
     uint32_t spins = 0;
     while (ld_relaxed64(&st->bar) < target) {
-      if (++spins > kSpinLimit) {
+      if (++spins > limit) {
         atomicOr(&st->err, kErrBarrier);
         ok = 0;
         break;
@@ -518,14 +519,14 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
   uint64_t t = 1ull + a.delta;
   uint32_t par = resume ? st->par : 0u, far_min = resume ? st->far_min : 0xffffffffu;
   uint32_t thr = resume ? st->thr : !a.split || t > 0xffffffffull ? 0xffffffffu : (uint32_t)t;
-  if (!rounds_sync(st, rs.target)) return;
+  if (!rounds_sync(st, rs.target, a.spin_limit)) return;
 
   bool merge = false, hand = false;
   for (uint32_t seq = 0;; seq++) {
     RoundSlot *slot = st->slot + (seq & 3u);
     if (a.split) scan_frontier<true, true>(a, sh.scan, a.bm[par], nullptr, a.bm[2], merge, thr, slot);
     else scan_frontier<false, true>(a, sh.scan, a.bm[par], nullptr, nullptr, false, 0u, slot);
-    if (!rounds_sync(st, rs.target)) return;
+    if (!rounds_sync(st, rs.target, a.spin_limit)) return;
     if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
     const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
     const uint64_t n = (x0 >> a.shift) + (x1 >> a.shift);
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(cons
       if (rs.op.near) slot->near = 1u;
       if (rs.op.far_cand != 0xffffffffu) atomicMin(&slot->far_cand, rs.op.far_cand);
     }
-    if (!rounds_sync(st, rs.target)) return;
+    if (!rounds_sync(st, rs.target, a.spin_limit)) return;
     if (lead && a.timer) st->ns_relax += globaltimer_ns();
     par ^= 1u;
     merge = false;
@@ -870,13 +871,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
   if (st->hand == kHandBottomUp) done = counted_bottom(st->hbu);
   if (lead)
     for (int i = 0; i < 4; i++) slot_clear(st->slot + i);
-  if (!rounds_sync(st, rs.target)) return;  // every CTA has read the state that is rewritten at the end
+  if (!rounds_sync(st, rs.target, a.spin_limit)) return;  // every CTA has read the state that is rewritten at the end
   for (uint32_t seq = 0; !done; seq++) {
     uint32_t *cur = a.bm[par], *next = a.bm[par ^ 1];
     RoundSlot *slot = st->slot + (seq & 3u);
     if (!bottom) {
       scan_frontier<false, false>(a, sh.scan, cur, next, nullptr, false, 0u, slot);
-      if (!rounds_sync(st, rs.target)) return;
+      if (!rounds_sync(st, rs.target, a.spin_limit)) return;
       if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
       const unsigned long long x0 = slot->app[0], x1 = slot->app[1];
       const uint64_t n0 = x0 >> a.shift, n = n0 + (x1 >> a.shift);
@@ -918,7 +919,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
         if (threadIdx.x == 0) rs.op = BfsOp{a.bm[2], next, a.value, &st->err, a.V, level + 1};
         if (lead && a.timer) st->ns_relax -= globaltimer_ns();
         relax_lists(rs, sh.lbs, slot);
-        if (!rounds_sync(st, rs.target)) return;
+        if (!rounds_sync(st, rs.target, a.spin_limit)) return;
         if (lead && a.timer) st->ns_relax += globaltimer_ns();
         level++;
         par ^= 1u;
@@ -931,7 +932,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
       break;
     }
     bfs_bottom_up_level(a, s0, s1, cur, next, level + 1, slot);
-    if (!rounds_sync(st, rs.target)) return;
+    if (!rounds_sync(st, rs.target, a.spin_limit)) return;
     if (lead) slot_clear(st->slot + ((seq + 2) & 3u));
     done = counted_bottom(slot->bu);
   }
@@ -967,7 +968,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_bfs_rounds(const __grid_constan
 constexpr uint32_t kJumps = 3;  // compressions of a run
 constexpr uint32_t kJumpHops = 8;
 constexpr int kJumpWalks = 4;  // vertices a thread has in flight
-__global__ void __launch_bounds__(kThreads) k_uf_jump(uint32_t *par, uint32_t V, RoundsState *st, uint32_t *err) {
+__global__ void __launch_bounds__(kThreads) k_uf_jump(uint32_t *par, uint32_t V, RoundsState *st, uint32_t spin_limit,
+                                                    uint32_t *err) {
   unsigned long long target = 0;
   const uint64_t first = blockIdx.x * (uint64_t)kThreads + threadIdx.x, stride = (uint64_t)gridDim.x * kThreads;
   for (uint32_t pass = 0;; pass++) {
@@ -1004,7 +1006,7 @@ __global__ void __launch_bounds__(kThreads) k_uf_jump(uint32_t *par, uint32_t V,
     uint32_t *flag = &st->slot[pass & 3u].near;
     if (__syncthreads_or(open != 0u) && threadIdx.x == 0) *flag = 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) st->slot[(pass + 2) & 3u].near = 0u;  // last read before the barrier before
-    if (!rounds_sync(st, target) || pass > 64) {
+    if (!rounds_sync(st, target, spin_limit) || pass > 64) {
       if (threadIdx.x == 0) atomicOr(err, kErrBarrier);
       return;
     }
