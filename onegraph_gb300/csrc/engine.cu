@@ -122,7 +122,11 @@ struct og_engine {
   uint32_t *outdeg_d = nullptr, *carry_idx_d = nullptr;
   double *part_d = nullptr;
   PrLoop *prl_d = nullptr, *prl_h = nullptr;  // L1 iterations: state and its page-locked mirror
-  uint32_t pr_hint = 8;  // iterations the last run took (launched before its first check)
+  // iterations the last run of this damping and tolerance took (launched before
+  // the first check)
+  uint32_t pr_hint = 8;
+  float pr_hint_damping = 0;
+  double pr_hint_tol = -1;
   uint32_t part_n = 0;
   uint64_t pr_tiles = 0;
 
@@ -2416,6 +2420,11 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
     const uint32_t *done = &e->prl_d->done;
     const LbsArgs a0 = lbs_args(e, 0, 0, c0.total, true, e->plan.static_edges);
     const LbsArgs a1 = lbs_args(e, 1, 0, c1.total, true, e->g->E);
+    if (damping != e->pr_hint_damping || tol != e->pr_hint_tol) {
+      e->pr_hint = 8;
+      e->pr_hint_damping = damping;
+      e->pr_hint_tol = tol;
+    }
     uint32_t launched = 0, batch = std::max<uint32_t>(1, e->pr_hint);
     while (launched < (uint32_t)max_iter) {
       batch = std::min<uint32_t>(batch, (uint32_t)max_iter - launched);
