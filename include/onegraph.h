@@ -253,7 +253,10 @@ typedef struct og_stats {
   uint64_t link_bytes;       /* bytes read over the host link               */
   double ms_total;           /* host wall time of the query                 */
   double ms_static;          /* device time of static relax kernels         */
-  double ms_dynamic;         /* device time of dynamic gather+relax         */
+  double ms_dynamic;         /* device time of dynamic gather+relax (og_pr_l1
+                                in direct mode: of every iteration's pull, by
+                                the GPU's timer, launch to launch; all
+                                resident: in ms_static)                     */
   double ms_compact;         /* device time of frontier compaction          */
   double residual;           /* PR: last L1 delta; otherwise 0              */
   uint64_t launches;         /* kernels launched for the query              */

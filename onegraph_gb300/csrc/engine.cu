@@ -2266,6 +2266,7 @@ PrArgs pr_args(const og_engine *e, int r, const uint32_t *done) {
   q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
   q.done = done;
   q.link = (uint32_t)r;
+  if (done) q.t = e->prl_d->t;
   return q;
 }
 
@@ -2428,10 +2429,9 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
     uint32_t launched = 0, batch = std::max<uint32_t>(1, e->pr_hint);
     while (launched < (uint32_t)max_iter) {
       batch = std::min<uint32_t>(batch, (uint32_t)max_iter - launched);
-      const uint32_t before = launched ? e->prl_h->iters : 0;
+      k_pr_begin<<<1, 1, 0, s>>>(e->prl_d, launched == 0);
+      e->launches++;
       for (uint32_t i = 0; i < batch; i++, launched++) {
-        // the pulls of a run are alike: the first of a batch is timed
-        if (i == 0) CK(cudaEventRecord(e->t_d0, s));
         if (c0.n && c1.n) {
           RC(launch_pr_pull_pair(e, a0, EKU::stat(e), a1, EKU::host(e), done, s));
         } else if (c0.n || c1.n) {
@@ -2440,17 +2440,14 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
                   ? launch_pr_pull<true>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)
                   : launch_pr_pull<false>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)));
         }
-        if (i == 0) CK(cudaEventRecord(e->ev_dyn_done, s));
         RC(launch_pr_fixup(e, done));
         RC(launch_pr_update(e, teleport, damping, tol, done));
       }
       RC(pr_check(e, st));
-      float ms = 0;
-      if (cudaEventElapsedTime(&ms, e->t_d0, e->ev_dyn_done) == cudaSuccess)
-        (c1.n ? st.ms_dynamic : st.ms_static) += ms * (e->prl_h->iters - before);
       if (e->prl_h->done) break;
       batch = 4;
     }
+    (c1.n ? st.ms_dynamic : st.ms_static) += e->prl_h->t[1] / 1e6;
     const uint64_t its = e->prl_h->iters;
     e->pr_hint = (uint32_t)its;
     st.iterations += (uint32_t)its;

@@ -1546,6 +1546,10 @@ struct PrArgs {
   // iterations launched ahead: when not null, nothing is done once *done is set
   const uint32_t *done;
   uint32_t link;  // the records are read over the host link
+  // when not null: t[0] is when the iteration before ended; k_pr_fixup, right
+  // behind the pull, adds the time since to t[1] (ns of the GPU's global timer;
+  // a stamp in the pull itself cost 4 us of its 590)
+  unsigned long long *t;
 };
 
 // Pull sum sum[v] = sum over in-edges (u -> v) of contrib[u]
@@ -1856,6 +1860,7 @@ struct PrFixup {
 __global__ void k_pr_fixup(PrFixup f0, uint64_t n0, PrFixup f1, uint64_t n1) {
   const uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (x >= n0 + n1 || (f0.p.done && *f0.p.done)) return;
+  if (f0.p.t && x == 0) f0.p.t[1] += globaltimer_ns() - f0.p.t[0];
   const bool r0 = x < n0;
   const uint64_t k = r0 ? x : x - n0;
   const PrFixup &f = r0 ? f0 : f1;
@@ -1908,6 +1913,7 @@ struct PrLoop {
   double residual;  // of the last iteration
   uint32_t done;    // it was below the tolerance
   uint32_t iters;
+  unsigned long long t[2];  // PrArgs::t
 };
 
 // Normalised update p' = teleport + damping*sum for every vertex, with the L1
@@ -1975,6 +1981,12 @@ __global__ void __launch_bounds__(kThreads) k_pr_update_l1(uint64_t V, float *ra
   if (threadIdx.x == 0) part[blockIdx.x] = s_d[0];
 }
 
+// Begins iterations: clears the state (first), or goes on with it after a wait.
+__global__ void k_pr_begin(PrLoop *loop, int first) {
+  if (first) *loop = PrLoop{};
+  loop->t[0] = globaltimer_ns();
+}
+
 // Sum of the partials, and the end of the iteration.
 __global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double tol) {
   __shared__ double s_d[kThreads];
@@ -1991,6 +2003,7 @@ __global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double
     loop->residual = s_d[0];
     loop->iters++;
     if (s_d[0] < tol) loop->done = 1;
+    loop->t[0] = globaltimer_ns();
   }
 }
 

@@ -39,3 +39,29 @@ def test_launches_follow_the_tolerance():
         assert e.stats["launches"] <= PER_ITERATION * n + 8
     np.testing.assert_array_equal(e.pr_l1(0.85, 1e-9, 500), tight)
     e.close()
+
+
+@pytest.mark.parametrize("mode", ["resident", "direct"])
+@pytest.mark.parametrize("V,E", [(2000, 30_000), (200_000, 3_000_000)])
+def test_pull_times_are_those_of_every_iteration(mode, V, E):
+    """The first pull of an engine finds cold caches and code; times a number of
+    iterations it would exceed the query's own time."""
+    g = graph(V, E, 1)
+    kw = {}
+    if mode == "direct":
+        kw = dict(budget=budget_for(g, E // 8, og.CFG_DIRECT), advisek=0.5, direct=True)
+    per = []
+    for _ in range(6):
+        e = og.Engine(g, **kw)
+        assert (e.plan["dynamic_edges"] > 0) == (mode == "direct")
+        for its in (7, 100, 1):
+            e.pr_l1(0.85, 0.0, its)
+            st = e.stats
+            pull = st["ms_dynamic"] + st["ms_static"]
+            assert st["iterations"] == its and 0 < pull <= st["ms_total"], (its, st)
+            assert (st["ms_dynamic"] == 0) == (mode == "resident") and (st["ms_static"] == 0) == (mode == "direct")
+            if its == 100:
+                per.append((pull / its, st["ms_total"] / its))
+        e.close()
+    # the pulls are most of an iteration on a graph of 15 edges a vertex, and never more than it
+    assert V < 100_000 or all(p > 0.3 * t for p, t in per), per
