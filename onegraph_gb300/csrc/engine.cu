@@ -1753,11 +1753,20 @@ struct PersistCfg {
 constexpr PersistCfg kPersistConfigs[] = {{256, 8}, {128, 8}, {256, 4}, {512, 4}, {128, 16}};
 constexpr int kNumPersistConfigs = 5;
 
+// Bottom-up levels need the graph's reverse edges: only a symmetric graph has
+// them in its own records.
+uint32_t batch_dopt(const og_engine *e) {
+  return e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1 ? 1u : 0u;
+}
+
 // Configuration of an engine that has not been tuned.  512 x 4 keeps 32 warps
 // on an SM where 256 x 8 keeps 16 (128 registers); on small graphs the latter's
 // fewer CTAs make cheaper barriers.  64 sources, ms (512 x 4 / 256 x 8): 259 M
-// edges 4.27 / 5.41, 31 M edges 0.85 / 0.92, 3.2 M edges 0.46 / 0.43.
-int persist_default(const og_engine *e) { return e->g->E >= (8u << 20) ? 3 : 0; }
+// edges 4.27 / 5.41, 31 M edges 0.85 / 0.92, 7.6 M 0.55 / 0.56, 3.7 M 0.49 / 0.48,
+// 1.8 M 0.45 / 0.43.  Without bottom-up levels the pushes of every edge are
+// most of the work, and the line lies lower: 8.0 M edges 0.64 / 0.79, 3.9 M 0.48 / 0.54,
+// 1.0 M 0.35 / 0.37 (one source: 0.35 / 0.39, 0.28 / 0.30, 0.23 / 0.24).
+int persist_default(const og_engine *e) { return e->g->E >= (batch_dopt(e) ? 8u << 20 : 1u << 20) ? 3 : 0; }
 
 template <int B, int I>
 int launch_persist_cfg(og_engine *e, const PersistArgs &a, cudaStream_t s) {
@@ -1789,12 +1798,6 @@ int launch_persist(og_engine *e, int ci, const PersistArgs &a, cudaStream_t s) {
     case 3: return launch_persist_cfg<512, 4>(e, a, s);
     default: return launch_persist_cfg<128, 16>(e, a, s);
   }
-}
-
-// Bottom-up levels need the graph's reverse edges: only a symmetric graph has
-// them in its own records.
-uint32_t batch_dopt(const og_engine *e) {
-  return e->bfs_direction == OG_BFS_AUTO && e->g->symmetric == 1 ? 1u : 0u;
 }
 
 // Enqueues one whole batch on s_main: clear state, upload the sources from the
