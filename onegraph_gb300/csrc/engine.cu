@@ -1070,6 +1070,11 @@ void collect_timing(og_engine *e, Timing &t, og_stats *st) {
 struct NoPair {};
 struct NoStage {};
 
+// Whether the caller of run_regions has put work on s_main since the counts came
+// back (push PageRank clears its sums there, the L1 pull updates the ranks): the
+// dynamic region's own stream then waits for it, 2 us a round.
+enum class MainStream { kIdle, kBusy };
+
 // One round's region work given the compaction counts (already on the host).
 // `static_fn(a)` / `dyn_fn(a, src, stream)` launch the per-region kernel;
 // `pair_fn(a0, src0, a1, src1, stream)`, when given, launches both regions
@@ -1077,8 +1082,9 @@ struct NoStage {};
 // static tiles then overlap the link-bound dynamic ones instead of taking the
 // SMs first.  Its time is counted as dynamic-region time.
 // `stage_fn(a)`, when given, launches a staged round of the dynamic list a.
+// `main`: see MainStream.
 template <class K, class StaticFn, class DynFn, class PairFn = NoPair, class StageFn = NoStage>
-int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynFn dyn_fn,
+int run_regions(og_engine *e, og_stats &st, Timing &tm, MainStream main, StaticFn static_fn, DynFn dyn_fn,
                 PairFn pair_fn = PairFn(), StageFn stage_fn = StageFn()) {
   const Counts cs = e->counts_h[0], cd = e->counts_h[1];
   if constexpr (!std::is_same<PairFn, NoPair>::value) {
@@ -1095,9 +1101,7 @@ int run_regions(og_engine *e, og_stats &st, Timing &tm, StaticFn static_fn, DynF
       return OG_OK;
     }
   }
-  // The dynamic region's work starts behind what the caller has enqueued on
-  // s_main since the counts came back (push PageRank clears its sums there).
-  if (cd.n) {
+  if (cd.n && main == MainStream::kBusy) {
     CK(cudaEventRecord(e->ev_round, e->s_main));
     CK(cudaStreamWaitEvent(e->s_dyn, e->ev_round, 0));
   }
@@ -1308,7 +1312,7 @@ int run_frontier(og_engine *e, int algo, uint32_t src, og_stats &st) {
       if constexpr (K::kFrag) return (int)OG_OK;  // direct mode only
       else return launch_stage_round<K>(e, ro, a, next, e->s_dyn);
     };
-    RC((run_regions<K>(e, st, tm, sfn, dfn, pfn, gfn)));
+    RC((run_regions<K>(e, st, tm, MainStream::kIdle, sfn, dfn, pfn, gfn)));
     if constexpr (K::kFrag) e->frag->since += e->counts_h[1].total;
     CK(cudaMemsetAsync(cur, 0, 4 * e->nwords, e->s_main));
     std::swap(cur, next);
@@ -1572,7 +1576,7 @@ int run_batch(og_engine *e, const uint32_t *srcs, uint32_t n, uint32_t *out, uin
       e->launches++;
       return (int)OG_OK;
     };
-    RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
+    RC((run_regions<EKU>(e, st, tm, MainStream::kIdle, sfn, launch, pfn)));
     CK(cudaMemsetAsync(e->hist_d, 0, 64 * 8, s));
     k_batch_level<<<grid_for(e->nwords, e->sms), kThreads, 0, s>>>(next_any, next, e->nwords, n,
                                                                  e->hist_d, depth_d, V, level + 1);
@@ -1713,7 +1717,7 @@ int bb_step_impl(og_engine *e, uint64_t *pending, bool *done, og_stats &st, Timi
     e->launches++;
     return (int)OG_OK;
   };
-  RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
+  RC((run_regions<EKU>(e, st, tm, MainStream::kIdle, sfn, launch, pfn)));
   CK(cudaMemsetAsync(e->hist_d, 0, 64 * 8, s));
   const uint32_t depth = e->bb_level + 1;  // of the vertices this level reaches, for a source joined at begin
   k_batch_level<<<grid_for(e->nwords, e->sms), kThreads, 0, s>>>(next_any, next, e->nwords, 64, e->hist_d,
@@ -2171,7 +2175,7 @@ int sb_round(og_engine *e, og_stats &st, Timing &tm, uint32_t *pending, bool *do
     e->launches++;
     return (int)OG_OK;
   };
-  RC((run_regions<K>(e, st, tm, sfn, launch, pfn)));
+  RC((run_regions<K>(e, st, tm, MainStream::kIdle, sfn, launch, pfn)));
   CK(cudaGetLastError());
   return OG_OK;
 }
@@ -2305,7 +2309,7 @@ int launch_pr_fixup(og_engine *e, const uint32_t *done) {
   return OG_OK;
 }
 
-int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
+int pr_sums(og_engine *e, og_stats &st, Timing &tm, MainStream main) {
   auto sfn = [&](const LbsArgs &a) {
     return pr_contiguous(e, 0) ? launch_pr_pull<true>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main)
                                : launch_pr_pull<false>(e, a, EKU::stat(e), pr_args(e, 0, nullptr), e->s_main);
@@ -2329,7 +2333,7 @@ int pr_sums(og_engine *e, og_stats &st, Timing &tm) {
   auto pfn = [&](const LbsArgs &a0, auto s0, const LbsArgs &a1, auto s1, cudaStream_t ps) {
     return launch_pr_pull_pair(e, a0, s0, a1, s1, nullptr, ps);
   };
-  RC((run_regions<EKU>(e, st, tm, sfn, dfn, pfn, gfn)));
+  RC((run_regions<EKU>(e, st, tm, main, sfn, dfn, pfn, gfn)));
   return launch_pr_fixup(e, nullptr);
 }
 
@@ -2355,7 +2359,7 @@ int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
     st.iterations++;
     st.frontier_sum += n;
     st.static_vertices += e->counts_h[0].n;
-    RC(pr_sums(e, st, tm));
+    RC(pr_sums(e, st, tm, MainStream::kIdle));  // the compaction was waited for
     CK(cudaMemsetAsync(e->active_d, 0, 4, s));
     k_pr_update_delta<<<grid_for(e->nwords, e->sms), kThreads, 0, s>>>(
         cur, next, e->nwords, (float *)e->value_d, e->contrib_d, e->sum_d, e->outdeg_d, thresh,
@@ -2467,7 +2471,7 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
     st.iterations++;
     st.frontier_sum += n;
     st.static_vertices += e->counts_h[0].n;
-    RC(pr_sums(e, st, tm));
+    RC(pr_sums(e, st, tm, MainStream::kBusy));
     RC(launch_pr_update(e, teleport, damping, tol, nullptr));
     RC(pr_check(e, st));
     collect_timing(e, tm, &st);
@@ -2518,7 +2522,7 @@ int run_pr_l1_push(og_engine *e, float damping, double tol, int max_iter, og_sta
     st.frontier_sum += n;
     st.static_vertices += e->counts_h[0].n;
     CK(cudaMemsetAsync(e->sum_d, 0, 4 * V, s));
-    RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
+    RC((run_regions<EKU>(e, st, tm, MainStream::kBusy, sfn, launch, pfn)));
     RC(launch_pr_update(e, teleport, damping, tol, nullptr));
     RC(pr_check(e, st));
     collect_timing(e, tm, &st);
@@ -2849,7 +2853,7 @@ int run_cc_uf(og_engine *e, og_stats &st) {
       e->launches++;
       return (int)OG_OK;
     };
-    RC((run_regions<EKU>(e, st, tm, sfn, launch, pfn)));
+    RC((run_regions<EKU>(e, st, tm, MainStream::kIdle, sfn, launch, pfn)));
   }
   if (n) RC(compress());  // nothing was linked since the last compression otherwise
   CK(cudaStreamSynchronize(s));
