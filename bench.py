@@ -764,13 +764,13 @@ def run_pr_precision(args, rank, world, local):
     peaks = measured_peaks()
     kms = st["ms_dynamic"] / iters
     hbm_gbs = (24 * g.V + 8 * g.E) / (kms / 1e3) / 1e9 if kms else 0.0
-    roof_hbm = {"bound": "hbm", "kernel": "k_pr_pull_pair<true> (the pulls of every iteration of the run)",
+    roof_hbm = {"bound": "hbm", "kernel": "k_pr_pull_pair<true> (the mean of every eighth iteration's pull)",
                 "achieved": hbm_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": hbm_gbs / peaks["hbm_gbs"], "traffic": None, "peak_source": peaks["source"],
                 "bytes_per_launch": 24 * g.V + 8 * g.E, "kernel_ms_per_iter": kms,
                 "note": "algorithmic bytes V (16 + 4 + 4) + 8 E per iteration over the pull launches' time"}
     link_gbs = st["link_bytes"] / (st["ms_dynamic"] / 1e3) / 1e9 if st["ms_dynamic"] else 0.0
-    roof = {"bound": "host-link", "kernel": "k_pr_pull_pair<true> (the pulls of every iteration of the run)",
+    roof = {"bound": "host-link", "kernel": "k_pr_pull_pair<true> (the mean of every eighth iteration's pull)",
             "achieved": link_gbs, "peak": h2d, "unit": "GB/s", "frac": link_gbs / h2d if h2d else None,
             "traffic": st["link_bytes"] / iters * PR_PULL_LINK_TRAFFIC_RATIO,
             "traffic_note": "host-link bytes per launch: algorithmic bytes x %.3f, the sysmem-sector / "

@@ -254,8 +254,9 @@ typedef struct og_stats {
   double ms_total;           /* host wall time of the query                 */
   double ms_static;          /* device time of static relax kernels         */
   double ms_dynamic;         /* device time of dynamic gather+relax (og_pr_l1
-                                in direct mode: of every iteration's pull, by
-                                the GPU's timer, launch to launch; all
+                                in direct mode: the mean of every eighth
+                                iteration's pull by the GPU's timer, launch
+                                to launch, times the iterations; all
                                 resident: in ms_static)                     */
   double ms_compact;         /* device time of frontier compaction          */
   double residual;           /* PR: last L1 delta; otherwise 0              */

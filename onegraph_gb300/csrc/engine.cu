@@ -2273,7 +2273,6 @@ PrArgs pr_args(const og_engine *e, int r, const uint32_t *done) {
   q.nwords = r ? e->g->packed_words : e->g->packed_words_for(e->plan.static_edges);
   q.done = done;
   q.link = (uint32_t)r;
-  if (done) q.t = e->prl_d->t;
   return q;
 }
 
@@ -2292,12 +2291,13 @@ int launch_pr_pull_pair(og_engine *e, const LbsArgs &a0, SrcP<false> s0, const L
   return OG_OK;
 }
 
-int launch_pr_fixup(og_engine *e, const uint32_t *done) {
+int launch_pr_fixup(og_engine *e, const uint32_t *done, bool timed = false) {
   PrFixup f[2];
   uint64_t nt[2];
   for (int r = 0; r < 2; r++) {
     const Counts c = e->counts_h[r];
     f[r] = PrFixup{e->list_d[r], e->pref_d[r], c.n, pr_args(e, r, done)};
+    f[r].p.t = timed ? e->prl_d->t : nullptr;
     nt[r] = c.n ? (c.total + kTile - 1) / kTile : 0;
   }
   if (nt[0] + nt[1]) {
@@ -2382,10 +2382,10 @@ int run_pr_delta(og_engine *e, float thresh, int max_rounds, og_stats &st) {
 }
 
 // The update of every rank and the end of the iteration (k_pr_finish).
-int launch_pr_update(og_engine *e, float teleport, float damping, double tol, const uint32_t *done) {
+int launch_pr_update(og_engine *e, float teleport, float damping, double tol, const uint32_t *done, bool stamp = false) {
   k_pr_update_l1<<<e->part_n, kThreads, 0, e->s_main>>>(e->V, (float *)e->value_d, e->contrib_d, e->sum_d,
                                                         e->outdeg_d, teleport, damping, e->part_d, done);
-  k_pr_finish<<<1, kThreads, 0, e->s_main>>>(e->part_d, e->part_n, e->prl_d, tol);
+  k_pr_finish<<<1, kThreads, 0, e->s_main>>>(e->part_d, e->part_n, e->prl_d, tol, stamp);
   e->launches += 2;
   return OG_OK;
 }
@@ -2436,8 +2436,10 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
     uint32_t launched = 0, batch = std::max<uint32_t>(1, e->pr_hint);
     while (launched < (uint32_t)max_iter) {
       batch = std::min<uint32_t>(batch, (uint32_t)max_iter - launched);
-      k_pr_begin<<<1, 1, 0, s>>>(e->prl_d, launched == 0);
-      e->launches++;
+      if (launched % kPrTimed == 0) {  // behind a wait: the first one is timed
+        k_pr_begin<<<1, 1, 0, s>>>(e->prl_d, launched == 0);
+        e->launches++;
+      }
       for (uint32_t i = 0; i < batch; i++, launched++) {
         if (c0.n && c1.n) {
           RC(launch_pr_pull_pair(e, a0, EKU::stat(e), a1, EKU::host(e), done, s));
@@ -2447,15 +2449,15 @@ int run_pr_l1(og_engine *e, float damping, double tol, int max_iter, og_stats &s
                   ? launch_pr_pull<true>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)
                   : launch_pr_pull<false>(e, r ? a1 : a0, r ? EKU::host(e) : EKU::stat(e), pr_args(e, r, done), s)));
         }
-        RC(launch_pr_fixup(e, done));
-        RC(launch_pr_update(e, teleport, damping, tol, done));
+        RC(launch_pr_fixup(e, done, launched % kPrTimed == 0));
+        RC(launch_pr_update(e, teleport, damping, tol, done, i + 1 < batch && (launched + 1) % kPrTimed == 0));
       }
       RC(pr_check(e, st));
       if (e->prl_h->done) break;
       batch = 4;
     }
-    (c1.n ? st.ms_dynamic : st.ms_static) += e->prl_h->t[1] / 1e6;
     const uint64_t its = e->prl_h->iters;
+    if (e->prl_h->t[2]) (c1.n ? st.ms_dynamic : st.ms_static) += e->prl_h->t[1] / 1e6 * its / e->prl_h->t[2];
     e->pr_hint = (uint32_t)its;
     st.iterations += (uint32_t)its;
     st.frontier_sum += n * its;

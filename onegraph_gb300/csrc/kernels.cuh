@@ -1546,9 +1546,11 @@ struct PrArgs {
   // iterations launched ahead: when not null, nothing is done once *done is set
   const uint32_t *done;
   uint32_t link;  // the records are read over the host link
-  // when not null: t[0] is when the iteration before ended; k_pr_fixup, right
-  // behind the pull, adds the time since to t[1] (ns of the GPU's global timer;
-  // a stamp in the pull itself cost 4 us of its 590)
+  // when not null, this iteration is timed: t[0] is when the one before ended;
+  // k_pr_fixup, right behind the pull, adds the time since to t[1] (ns of the
+  // GPU's global timer) and one to t[2].  Every kPrTimed-th iteration is: the
+  // timer is slow to read (3 % of the iterations of a graph of 0.1 M vertices
+  // when all were; a stamp in the pull itself cost 4 us of 590)
   unsigned long long *t;
 };
 
@@ -1860,7 +1862,10 @@ struct PrFixup {
 __global__ void k_pr_fixup(PrFixup f0, uint64_t n0, PrFixup f1, uint64_t n1) {
   const uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (x >= n0 + n1 || (f0.p.done && *f0.p.done)) return;
-  if (f0.p.t && x == 0) f0.p.t[1] += globaltimer_ns() - f0.p.t[0];
+  if (f0.p.t && x == 0) {
+    f0.p.t[1] += globaltimer_ns() - f0.p.t[0];
+    f0.p.t[2]++;
+  }
   const bool r0 = x < n0;
   const uint64_t k = r0 ? x : x - n0;
   const PrFixup &f = r0 ? f0 : f1;
@@ -1913,8 +1918,9 @@ struct PrLoop {
   double residual;  // of the last iteration
   uint32_t done;    // it was below the tolerance
   uint32_t iters;
-  unsigned long long t[2];  // PrArgs::t
+  unsigned long long t[3];  // PrArgs::t
 };
+constexpr uint32_t kPrTimed = 8;
 
 // Normalised update p' = teleport + damping*sum for every vertex, with the L1
 // delta accumulated in FP64: per-thread, then a fixed-shape block tree, one
@@ -1988,7 +1994,7 @@ __global__ void k_pr_begin(PrLoop *loop, int first) {
 }
 
 // Sum of the partials, and the end of the iteration.
-__global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double tol) {
+__global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double tol, int stamp) {
   __shared__ double s_d[kThreads];
   if (loop->done) return;
   double acc = 0.0;
@@ -2003,7 +2009,7 @@ __global__ void k_pr_finish(const double *part, uint32_t n, PrLoop *loop, double
     loop->residual = s_d[0];
     loop->iters++;
     if (s_d[0] < tol) loop->done = 1;
-    loop->t[0] = globaltimer_ns();
+    if (stamp) loop->t[0] = globaltimer_ns();  // the next iteration is timed
   }
 }
 

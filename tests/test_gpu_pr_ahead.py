@@ -43,7 +43,7 @@ def test_launches_follow_the_tolerance():
 
 @pytest.mark.parametrize("mode", ["resident", "direct"])
 @pytest.mark.parametrize("V,E", [(2000, 30_000), (200_000, 3_000_000)])
-def test_pull_times_are_those_of_every_iteration(mode, V, E):
+def test_pull_times_are_measured(mode, V, E):
     """The first pull of an engine finds cold caches and code; times a number of
     iterations it would exceed the query's own time."""
     g = graph(V, E, 1)
