@@ -1125,11 +1125,11 @@ SERVING_ADVISEK = 1.0
 ALGO_BFS, ALGO_SSSP, ALGO_PR = 0, 1, 3  # og_algo values (the reference arm loads no engine)
 # host-link sectors read by one PageRank pull launch over its algorithmic link
 # bytes, measured with ncu on R-MAT 22 directed under a 256 MiB budget:
-# 2,025,677 sectors of 32 B for 64.2 MB of records per iteration
-PR_PULL_LINK_TRAFFIC_RATIO = 1.010
-# the same for the single-source SSSP relax's largest dynamic launch on R-MAT
-# 22 weighted, 256 MiB: 96.6 MB of sysmem sectors for 94.8 MB of records
-SSSP_RELAX_LINK_TRAFFIC_RATIO = 1.019
+# 2,018,745 sectors of 32 B for 64.16 MB of records per iteration
+PR_PULL_LINK_TRAFFIC_RATIO = 1.007
+# the same for a round of every edge by k_lbs_pair on R-MAT 22 weighted, 256 MiB:
+# 288.1 MB of sysmem sectors for 284.0 MB of records
+SSSP_RELAX_LINK_TRAFFIC_RATIO = 1.014
 
 
 def serving_requests(degrees, n, rate, seed=4):
