@@ -455,7 +455,7 @@ def run_ours(args, rank, world, local):
                                  "largest dynamic launch on R-MAT 22 under a 256 MiB budget"
                                  % SSSP_RELAX_LINK_TRAFFIC_RATIO,
                  "peak_source": "highest of the link probes measured in this run (og_link_probe)", "link_probes": dict(LINK_PEAKS),
-                 "timing": "globaltimer around every relax phase of %d device-driven queries "
+                 "timing": "globaltimer or CUDA events around every relax phase of %d device-driven queries "
                            "(the timed queries' sources, timer on)" % len(tstats)}
     roof_static = {"bound": "hbm", "kernel": kname + ", its HBM side", "achieved": static_gbs,
                    "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": static_gbs / peaks["hbm_gbs"],
@@ -904,15 +904,15 @@ def run_bfs_resident(args, rank, world, local):
                           "edges_examined_per_query": td_ex / args.steps,
                           "achieved_gbs": td_gbs, "frac": td_gbs / peaks["hbm_gbs"],
                           "graph_vs_l2": "packed records %.0f MB, L2 129 MB" % (g.E * eb / 1e6),
-                          "relax_kernel": {"kernel": "k_bfs_rounds, top-down relax phases",
+                          "relax_kernel": {"kernel": "k_lbs<SrcP<false>,BfsOp> (large levels), k_bfs_rounds (relax phases of the others)",
                                            "ms_per_query": rx_ms / args.steps, "achieved_gbs": rx_gbs,
                                            "frac": rx_gbs / peaks["hbm_gbs"],
-                                           "timing": "globaltimer around every relax phase"}},
+                                           "timing": "globaltimer or CUDA events around every relax phase"}},
         "direction": args.bfs_direction,
         "bit_exact_vs_runCPUBFS": exact, "levels": stats[0]["iterations"],
         "edges_examined_per_query": examined / args.steps,
-        "roofline": {"bound": "hbm", "kernel": "k_bfs_rounds and k_bfs_small (scan, top-down relax, "
-                                               "bottom-up): all kernels of a query",
+        "roofline": {"bound": "hbm", "kernel": "k_bfs_rounds, k_bfs_small, k_lbs and k_bfs_bottom_up: all kernels "
+                                               "of a query",
                      "achieved": gbs,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
                      "traffic": None, "peak_source": peaks["source"]},

@@ -109,7 +109,6 @@ struct og_engine {
   uint64_t list_cap[2] = {0, 0}, tile_cap[2] = {0, 0};
   Lookback lb[2]{};
   uint32_t lb_tiles = 0;
-  // counts of the two regions followed by their two far keys (u64), one D2H
   // What the host reads after a compaction, in one copy: Counts[2], u64 far
   // key[2], 4 error words (err_d, active_d), 4 mask words (sb_masks).
   Counts *counts_d = nullptr, *counts_h = nullptr;

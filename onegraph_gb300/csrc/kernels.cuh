@@ -2300,9 +2300,7 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bottom_up(const uint64_t *off,
 
 // Parents are read through L1.  The giant component's root is read by every
 // walk, and from the L2 those reads of one line run one after another (linking
-// 8.4 M vertices: 0.95 ms so, 0.27 ms through L1; a compression 125 and 33 us);
-// a stale
-// parent is an older ancestor, so a walk only ends too early, at a vertex that
+// 8.4 M vertices: 0.95 ms so, 0.27 ms through L1); a stale parent is an older ancestor, so a walk only ends too early, at a vertex that
 // is no root any more, and the compare-and-swap on it returns the newer one.
 __device__ __forceinline__ uint32_t uf_find(uint32_t *par, uint32_t x, uint32_t V, uint32_t *err) {
   for (uint32_t steps = 0; steps <= V; steps++) {

@@ -381,8 +381,9 @@ struct RelaxShared {
 // CTAs that got cheap tiles take more.  When there are fewer tiles than CTAs,
 // each is split into up to eight parts of 256 positions: one SM takes 12 us
 // over a full tile's 4096 atomics, and a round of three tiles used three SMs
-// (resident SSSP of 0.3 M vertices: 1.05 -> 0.87 ms with parts).  The next ticket (and its region
-// split, by thread 0) is fetched while the current tile runs.
+// (resident SSSP of 0.3 M vertices: 1.12 ms with whole tiles, 0.86 with parts).
+// The next ticket (and its region split, by thread 0) is fetched while the
+// current tile runs.
 template <class Src, class Op>
 __device__ __noinline__ void relax_lists(RelaxShared<Src, Op> &rs, LbsSh<Op> &sh, RoundSlot *slot) {
   __builtin_assume(__isShared(&rs));  // shared, not generic, accesses
@@ -480,10 +481,11 @@ struct OpGroup<MinRoundOp<kWeighted>> {
 // propagation.  A round whose relax lowered nothing below the threshold is
 // followed by one scan of frontier and waiting set together at the advanced
 // threshold (the host loop scans the frontier, then the waiting set).
-// CTAs per SM, measured: three for label propagation and BFS (85 registers,
-// 23 M directed edges 641 us against 748 at four; resident BFS of 2^20 vertices
-// 173 against 182), four for SSSP, whose host-link rounds want more reads in
-// flight (2^24 vertices 12.5 ms against 12.9 at three and 12.7 at five).
+// CTAs per SM, measured: three for label propagation and BFS (80 registers,
+// 23 M directed edges 529 us against 534-566 at four; resident BFS of 2^20 vertices
+// 175 against 183), four for SSSP, whose host-link rounds want more reads in
+// flight (2^24 vertices 12.66 ms against 12.74 at three and 12.71 at five; resident
+// queries of 0.3 M vertices would rather have three: 0.78 ms against 0.86 and 0.94).
 template <bool kWeighted>
 __global__ void __launch_bounds__(kThreads, kWeighted ? 4 : 3) k_min_rounds(const __grid_constant__ RoundsArgs a,
                                                                            const __grid_constant__ SrcP<kWeighted> s0,
