@@ -109,7 +109,9 @@ __device__ __forceinline__ bool hands_over(const RoundsArgs &a, uint64_t n0, uin
 // Results of up to this many vertices are stored to page-locked memory by the
 // kernel that ends the query and copied to the caller's array by the host: a
 // copy-engine transfer takes 5-11 us to start, a pageable target as long again.
-constexpr uint32_t kPostedResult = 1u << 14;
+// BFS, stored / copied: 17 thousand vertices 88.4 / 91.2 us, 28 thousand 75.3 / 76.3,
+// 40 thousand 80.2 / 78.4, 0.1 M 117 / 103.
+constexpr uint32_t kPostedResult = 1u << 15;
 
 // All CTAs, after the last value has been written.
 __device__ __forceinline__ void rounds_result(const RoundsArgs &a) {

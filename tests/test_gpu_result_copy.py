@@ -86,3 +86,30 @@ def test_no_partial_result_between_passes():
     assert not seen
     np.testing.assert_array_equal(oracle.normalise_bfs(out, V), want)
     e.close()
+
+
+@pytest.mark.parametrize("V", [8, 32_767, 32_768, 32_769])
+@pytest.mark.parametrize("direct", [False, True])
+def test_both_ways_of_delivery(V, direct):
+    """Results of up to 32768 vertices are stored by the kernel, larger ones are
+    copied: page-locked, pageable, and left on the device."""
+    g = graph(V, og.WEIGHTED)
+    off, pairs = np.array(g.offsets), np.array(g.edges)
+    col = pairs[:, 0].copy()
+    kw = dict(budget=budget_for(g, max(g.E // 4, 2048), og.CFG_DIRECT), advisek=0.1, direct=True) if direct else {}
+    e = og.Engine(g, **kw)
+    e.set_param(og.PARAM_CC_METHOD, og.CC_LABEL_PROPAGATION)
+    want = {"bfs": oracle.normalise_bfs(oracle.bfs(off, col, 1)[0], V), "sssp": oracle.sssp_dijkstra(off, pairs, 1),
+            "cc": oracle.cc(off, col)[0]}
+    calls = {"bfs": (lambda o: e.bfs(1, o), og.ALGO_BFS), "sssp": (lambda o: e.sssp(1, o), og.ALGO_SSSP),
+             "cc": (lambda o: e.cc(o), og.ALGO_CC)}
+    for name, (call, algo) in calls.items():
+        for out in (np.full(V, SENTINEL, np.uint32), og.pinned_empty(V, np.uint32)):
+            got = call(out)
+            assert got is out
+            np.testing.assert_array_equal(oracle.normalise_bfs(got, V) if name == "bfs" else got, want[name])
+            np.testing.assert_array_equal(e.fetch(algo), got)
+        assert call(False) is None
+        got = e.fetch(algo)
+        np.testing.assert_array_equal(oracle.normalise_bfs(got, V) if name == "bfs" else got, want[name])
+    e.close()
